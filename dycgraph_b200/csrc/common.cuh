@@ -38,7 +38,10 @@ constexpr uint32_t ALGO_SSSP = 0, ALGO_BFS = 1, ALGO_CC = 2, ALGO_PR = 3;
 constexpr uint32_t WEIGHT_HASH128 = 0, WEIGHT_STORED = 1;
 
 // Rows longer than HEAVY are split into TILE-slot tiles processed by whole CTAs.
-constexpr uint32_t HEAVY = 1024;
+// A warp walks a row 128 slots at a time (4 per lane in flight), so HEAVY bounds
+// a wave's longest chain at two such steps of ~2 us (host-link latency); at 1024
+// the longest row of a wave held its barrier for eight.
+constexpr uint32_t HEAVY = 256;
 constexpr uint32_t TILE = 4096;
 constexpr int BLOCK = 256;
 
@@ -114,23 +117,19 @@ struct Adj {
   uint32_t *tbits;       // HBM deletion bitmap, one bit per arena slot
 };
 
-constexpr uint32_t BAR_GROUPS = 16;
-
-// Per-launch control block in device memory: barrier, queues, counters.
-struct Ctl {
-  uint32_t bar_count;
-  uint32_t bar_gen;
+// Per-launch control block in device memory: barrier, queues, counters. The
+// counters the grid barrier publishes sit in two 16-byte words, so its last
+// arriver reads them with two independent loads.
+struct alignas(128) Ctl {
+  uint32_t pub[4];       // barrier publication (frontier.cuh): generation, count, tiles, vmin
+  uint32_t bar_count;    // blocks that have arrived at the current barrier
+  uint32_t pad0[27];     // the polled line apart from the counters' atomics
+  uint32_t q_count[3];   // wave queue lengths (q0/q1 alternate)
+  uint32_t n_aff;        // affected list length (follows q_count: selector 3)
+  uint32_t tile_count;
+  uint32_t vmin;         // ordered closure: minimum frontier value of the next wave
   uint32_t err;
   uint32_t err_info;
-  uint32_t n_aff;        // affected list length
-  uint32_t q_count[3];   // wave queue lengths (q0/q1 alternate; q2: the ordered bucket)
-  uint32_t tile_count;
-  uint32_t vmin;         // ordered closure: minimum frontier value of the wave
-  // snapshots taken by the last block to arrive at a barrier
-  uint32_t snap_aff;
-  uint32_t snap_q[3];
-  uint32_t snap_tiles;
-  uint32_t snap_vmin;
   uint32_t wave_tag;     // running wave tag (never reused)
   uint32_t waves;        // waves run in this launch
   uint32_t pad[2];       // PageRank: carried frontier (queue parity, length)
@@ -144,12 +143,10 @@ struct Ctl {
   u64 a_head, a_tail;
   uint32_t a_pend, a_pool, a_tiles, a_pad;
   u64 stat[20];
-  u64 tphase[8];         // batched repair: global timer at phase boundaries (ns)
-  // grid-barrier arrival groups, one 128-byte line each (frontier.cuh)
-  uint32_t bar_sub[BAR_GROUPS * 32];
+  u64 tphase[8];         // repair: global timer at phase boundaries (ns)
 };
 // read back to the host once per snapshot (dycgraph_b200/engine.py CTL_BYTES)
-static_assert(sizeof(Ctl) == 2904, "Ctl layout changed: update CTL_BYTES in engine.py");
+static_assert(sizeof(Ctl) == 1024, "Ctl layout changed: update CTL_BYTES in engine.py");
 
 enum StatIdx {
   ST_LINK_BYTES = 0,

@@ -283,7 +283,6 @@ void Engine::finish_load() {
   // range-ordered regions of ceil(n / 64) entries each
   q0_ = (uint32_t *)dmalloc((n + 64ull) * 4);
   q1_ = (uint32_t *)dmalloc((n + 64ull) * 4);
-  q2_ = opt_.ordered_delta ? (uint32_t *)dmalloc((n + 1ull) * 4) : nullptr;
   CK(cudaMemsetAsync(mark_, 0, (n + 1ull) * 4, st_));
   CK(cudaMemsetAsync(wtag_, 0, (n + 1ull) * 4, st_));
   CK(cudaMemsetAsync(touch_, 0, (n + 1ull) * 4, st_));
@@ -572,7 +571,6 @@ void Engine::init() {
     L.phases = PH_CLOSE;
     L.max_waves = (uint32_t)std::min<u64>(4ull * n_ + 1024, 0x7FFFFFFFull);
     L.delta = opt_.ordered_delta;
-    L.q2 = q2_;
     L.timeout_ns = timeout;
     L.algo = opt_.algo;
     L.stored = stored_;
@@ -889,7 +887,6 @@ void Engine::enqueue_snapshot(const dycg_edge_dev *d_dels, size_t nd, const dycg
     L.phases = (nd ? PH_DELETE : 0) | (na ? PH_INSERT : 0) | PH_CLOSE;
     L.max_waves = (uint32_t)std::min<u64>(4ull * n_ + 1024, 0x7FFFFFFFull);
     L.delta = opt_.ordered_delta;
-    L.q2 = q2_;
     L.timeout_ns = timeout;
     L.algo = opt_.algo;
     L.stored = stored_;
@@ -1209,7 +1206,6 @@ void Engine::init_queries(u64 timeout) {
     L.phases = PH_CLOSE;
     L.max_waves = (uint32_t)std::min<u64>(4ull * n_ + 1024, 0x7FFFFFFFull);
     L.delta = opt_.ordered_delta;
-    L.q2 = q2_;
     L.tag_dev = seq_ + 1;
     L.timeout_ns = timeout;
     L.algo = opt_.algo;
@@ -1263,7 +1259,6 @@ void Engine::repair_queries(uint32_t nd, uint32_t na, u64 timeout) {
     L.phases = phases;
     L.max_waves = (uint32_t)std::min<u64>(4ull * n_ + 1024, 0x7FFFFFFFull);
     L.delta = opt_.ordered_delta;
-    L.q2 = q2_;
     L.tag_dev = seq_ + 1;
     L.timeout_ns = timeout;
     L.algo = opt_.algo;

@@ -30,7 +30,6 @@ struct RepairLaunch {
   uint32_t n_add;
   uint32_t n, source, epoch, tag_base, phases, max_waves;
   uint32_t delta;  // ordered closure bucket width (0: unordered)
-  uint32_t *q2;
   uint32_t *tag_dev;  // optional device wave-tag counter (replaces tag_base)
   u64 timeout_ns;
   uint32_t algo;

@@ -87,50 +87,9 @@ __device__ __forceinline__ uint32_t mweight(uint32_t u, uint32_t v, uint32_t w) 
 // that turns out to be a no-op; across phases the grid barrier orders them.
 __device__ __forceinline__ u64 ldk(const u64 *p) { return __ldcg(p); }
 
-// Lower *addr to cand given a recent read `seen`; true when the value
-// decreased (strict CAS form where zero weights are possible, atomicMin with
-// parent tie-break otherwise).
-template <bool STRICT>
-__device__ __forceinline__ bool lower_from(u64 *addr, u64 cand, u64 seen) {
-  if (cand >= seen) return false;
-  if (STRICT) {
-    u64 old = seen;
-    while (key_value(cand) < key_value(old)) {
-      const u64 prev = atomicCAS(addr, old, cand);
-      if (prev == old) return true;
-      old = prev;
-    }
-    return false;
-  }
-  return key_value(atomicMin(addr, cand)) > key_value(cand);
-}
-
 template <bool STRICT>
 __device__ __forceinline__ bool lower_key(u64 *addr, u64 cand) {
   return lower_from<STRICT>(addr, cand, ldk(addr));
-}
-
-// lower_from split in two so that a lane can issue several independent
-// first attempts before it looks at any result: first_lower issues the first
-// atomic (false: cand cannot lower `seen`, nothing issued) and leaves its
-// result in got; lowered finishes the attempt (the strict form retries from
-// the value it lost to, exactly as lower_from's loop does).
-template <bool STRICT>
-__device__ __forceinline__ bool first_lower(u64 *addr, u64 cand, u64 seen, u64 &got) {
-  if (cand >= seen) return false;
-  if (STRICT) {
-    if (key_value(cand) >= key_value(seen)) return false;
-    got = atomicCAS(addr, seen, cand);
-  } else {
-    got = atomicMin(addr, cand);
-  }
-  return true;
-}
-template <bool STRICT>
-__device__ __forceinline__ bool lowered(u64 *addr, u64 cand, u64 seen, u64 got) {
-  if (!STRICT) return key_value(got) > key_value(cand);
-  if (got == seen) return true;
-  return lower_from<true>(addr, cand, got);
 }
 
 // Append y to the wave queue of parity par once per wave (tag). With range
@@ -412,14 +371,15 @@ __device__ __forceinline__ void staged_pairs(uint32_t v, const uint32_t (&m)[NB]
 // Expand items[0..cnt): prep(v, m) fills v's masks (false: skip). Rows whose
 // work exceeds P.heavy are cut into P.tile-slot tiles (x = row, y/z = slot
 // range, w = mapping) that whole CTAs process after a grid barrier; their
-// masks travel through cmask. Ends with a barrier that applies reset_flags.
-// Returns false when the launch has failed.
+// masks travel through cmask. Ends with a barrier that applies reset_flags and
+// publishes counter sel.
 constexpr uint32_t NO_QUEUE = 0xFFFFFFFFu;
 
 template <int NB, bool WITH_W, class Prep, class Ph>
-__device__ bool multi_expand(const MultiParams &P, const Adj &A, const uint32_t *items,
+__device__ Snap multi_expand(const MultiParams &P, const Adj &A, const uint32_t *items,
                              uint32_t cnt, Prep &prep, Ph &ph, u64 *s, uint2 *stage, Acc &acc,
-                             uint32_t qpar, uint32_t reset_flags, uint32_t qratio) {
+                             uint32_t &gen, uint32_t qpar, uint32_t sel, uint32_t reset_flags,
+                             uint32_t qratio) {
   Ctl *ctl = P.ctl;
   const uint32_t lane = lane_id();
   // a range-ordered wave queue (qpar: its parity) is read range by range:
@@ -501,9 +461,11 @@ __device__ bool multi_expand(const MultiParams &P, const Adj &A, const uint32_t 
     }
     expand_vertex<NB, WITH_W>(A, v, m, 0, len, 32, ql, ph, s, acc);
   }
-  if (!grid_sync(ctl, reset_flags | SYNC_RESET_GRAB, P.timeout_ns)) return false;
-  const uint32_t nt = min(*(volatile uint32_t *)&ctl->snap_tiles, P.tiles.cap);
-  if (nt == 0) return true;
+  const Snap sn = grid_sync(ctl, gen,
+                            reset_flags | SYNC_RESET_GRAB | (ranged ? SYNC_RESET_RANGES : 0u), sel,
+                            P.timeout_ns);
+  if (!sn.ok || sn.tiles == 0) return sn;
+  const uint32_t nt = min(sn.tiles, P.tiles.cap);
   const uint32_t wib = threadIdx.x >> 5;
   __shared__ uint32_t s_tile;
   uint32_t t = blockIdx.x;
@@ -535,7 +497,7 @@ __device__ bool multi_expand(const MultiParams &P, const Adj &A, const uint32_t 
       staged_pairs<NB>(tl.x, m, tl.z - tl.y, stage, ph, s, acc);
     }
   }
-  return grid_sync(ctl, SYNC_RESET_TILES | SYNC_RESET_GRAB, P.timeout_ns);
+  return grid_sync(ctl, gen, SYNC_RESET_TILES | SYNC_RESET_GRAB, sel, P.timeout_ns);
 }
 
 // Children y of a newly affected (x, q) with parent_q(y) == x become affected.
@@ -907,7 +869,7 @@ __device__ __forceinline__ bool take_masks_atomic(uint32_t *pend, uint32_t v, ui
 // or the tile budget is exhausted). Ends with a barrier that resets the ring.
 template <int NB, bool WITH_W, class Ph>
 __device__ bool async_phase(const MultiParams &P, const Adj &A, const uint32_t *items,
-                            uint32_t cnt, uint32_t *pend, Ph &ph, u64 *s, Acc &acc,
+                            uint32_t cnt, uint32_t *pend, Ph &ph, u64 *s, Acc &acc, uint32_t &gen,
                             uint32_t qratio) {
   Ctl *c = P.ctl;
   const uint32_t lane = lane_id();
@@ -916,7 +878,7 @@ __device__ bool async_phase(const MultiParams &P, const Adj &A, const uint32_t *
     const uint32_t v = items[i];
     if (atomicExch(P.inq + v, 1u) == 0u) async_push(P, v);
   }
-  if (!grid_sync(c, SYNC_RESET_Q0 | SYNC_RESET_Q1, P.timeout_ns)) return false;
+  if (!grid_sync(c, gen, SYNC_RESET_Q0 | SYNC_RESET_Q1, SEL_AFF, P.timeout_ns).ok) return false;
   for (;;) {
     const u64 item = async_pop(P);
     if (item == A_EMPTY) break;
@@ -980,7 +942,9 @@ __device__ bool async_phase(const MultiParams &P, const Adj &A, const uint32_t *
     __threadfence();
     if (lane == 0) atomicSub(&c->a_pend, 1u);
   }
-  return grid_sync(c, SYNC_RESET_ASYNC | SYNC_RESET_Q0 | SYNC_RESET_Q1, P.timeout_ns);
+  return grid_sync(c, gen, SYNC_RESET_ASYNC | SYNC_RESET_Q0 | SYNC_RESET_Q1, SEL_AFF,
+                   P.timeout_ns)
+      .ok;
 }
 
 // CTAs per SM the register allocation is sized for at 8 blocks of queries:
@@ -992,7 +956,7 @@ __device__ bool async_phase(const MultiParams &P, const Adj &A, const uint32_t *
 
 template <uint32_t ALGO, bool STORED, int NB>
 __global__ void __launch_bounds__(BLOCK, NB >= 8 ? DYCG_MULTI_MIN_BLOCKS : 3)
-    multi_repair_kernel(MultiParams P) {
+    multi_repair_kernel(const __grid_constant__ MultiParams P) {
   Ctl *ctl = P.ctl;
   Acc acc = {0, 0, 0, 0, 0, 0};
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1003,7 +967,8 @@ __global__ void __launch_bounds__(BLOCK, NB >= 8 ? DYCG_MULTI_MIN_BLOCKS : 3)
   const uint32_t epoch = *(volatile uint32_t *)&P.seq[0];
   const uint32_t tag0 = *(volatile uint32_t *)&P.seq[1];
   uint32_t tag = tag0 + 1;  // next unused wave tag (uniform over the grid)
-  uint32_t waves = 0;
+  uint32_t waves = 0, gen = 0, na = 0;
+  Snap sn;
   if (gtid == 0) ctl->stat[ST_T_START] = globaltimer_ns();
   __shared__ u64 s_state[WARPS][Q];  // edge-lane per-query state of each warp
   __shared__ uint2 s_stage[MULTI_MIN_TILE];  // staged slots of an edge-lane tile
@@ -1033,18 +998,20 @@ __global__ void __launch_bounds__(BLOCK, NB >= 8 ? DYCG_MULTI_MIN_BLOCKS : 3)
         enqueue_once(P, 0, e.y, tag0);
       }
     }
-    if (!grid_sync(ctl, 0, P.timeout_ns)) goto done;
+    sn = grid_sync(ctl, gen, 0, SEL_Q0, P.timeout_ns);
+    if (!sn.ok) goto done;
     // 2. invalidation waves (or one asynchronous phase)
     if (P.async) {
-      const uint32_t cnt = *(volatile uint32_t *)&ctl->snap_q[0];
+      const uint32_t cnt = sn.cnt;
       InvalidatePh<NB> ph{&P, P.inew[0], QPAR_ASYNC, tag++, epoch};
-      if (!async_phase<NB, false>(P, P.out, P.q[0], cnt, P.inew[0], ph, s, acc, P.qratio))
+      if (!async_phase<NB, false>(P, P.out, P.q[0], cnt, P.inew[0], ph, s, acc, gen,
+                                  P.qratio))
         goto done;
       waves++;
     } else {
       uint32_t cur = 0;
       for (uint32_t wave = 0;; wave++) {
-        const uint32_t cnt = *(volatile uint32_t *)&ctl->snap_q[cur];
+        const uint32_t cnt = sn.cnt;
         if (cnt == 0) break;
         if (wave >= P.max_waves) {
           if (gtid == 0) atomicCAS(&ctl->err, 0u, ERR_WAVES);
@@ -1054,9 +1021,10 @@ __global__ void __launch_bounds__(BLOCK, NB >= 8 ? DYCG_MULTI_MIN_BLOCKS : 3)
         InvalidatePh<NB> ph{&P, P.inew[par ^ 1], cur ^ 1, tag++, epoch};
         uint32_t *src = P.inew[par];
         auto prep = [&](uint32_t v, uint32_t (&m)[NB]) { return take_masks<NB>(src, v, true, m); };
-        if (!multi_expand<NB, false>(P, P.out, P.q[cur], cnt, prep, ph, s, s_stage, acc, cur,
-                                     cur ? SYNC_RESET_Q1 : SYNC_RESET_Q0, P.qratio))
-          goto done;
+        sn = multi_expand<NB, false>(P, P.out, P.q[cur], cnt, prep, ph, s, s_stage, acc, gen, cur,
+                                     cur ? SEL_Q0 : SEL_Q1, cur ? SYNC_RESET_Q1 : SYNC_RESET_Q0,
+                                     P.qratio);
+        if (!sn.ok) goto done;
         waves++;
         cur ^= 1;
       }
@@ -1064,7 +1032,8 @@ __global__ void __launch_bounds__(BLOCK, NB >= 8 ? DYCG_MULTI_MIN_BLOCKS : 3)
     if (gtid == 0) ctl->tphase[0] = globaltimer_ns();  // seeds + invalidation done
     // 3. reset the affected (v, q)
     {
-      const uint32_t na = *(volatile uint32_t *)&ctl->snap_aff;
+      // (complete: the invalidation's last barrier is behind)
+      na = *(volatile uint32_t *)&ctl->n_aff;
       for (uint32_t i = gw; i < na; i += nw) {
         const uint32_t v = P.aff[i];
 #pragma unroll
@@ -1073,12 +1042,13 @@ __global__ void __launch_bounds__(BLOCK, NB >= 8 ? DYCG_MULTI_MIN_BLOCKS : 3)
           if ((mk >> lane) & 1u) P.key[(u64)v * Q + k * 32 + lane] = KEY_INF;
         }
       }
-      if (!grid_sync(ctl, 0, P.timeout_ns)) goto done;
+      if (!grid_sync(ctl, gen, 0, SEL_AFF, P.timeout_ns).ok) goto done;
       // 4. pull over in-rows
       PullPh<ALGO, STORED, NB> ph{&P};
       auto prep = [&](uint32_t v, uint32_t (&m)[NB]) { return take_masks<NB>(P.affm, v, false, m); };
-      if (!multi_expand<NB, STORED>(P, P.in, P.aff, na, prep, ph, s, s_stage, acc, NO_QUEUE, 0,
-                                    P.pull_qratio))
+      if (!multi_expand<NB, STORED>(P, P.in, P.aff, na, prep, ph, s, s_stage, acc, gen, NO_QUEUE,
+                                    SEL_AFF, 0, P.pull_qratio)
+               .ok)
         goto done;
       if (gtid == 0) ctl->tphase[1] = globaltimer_ns();  // reset + pull done
     }
@@ -1087,7 +1057,6 @@ __global__ void __launch_bounds__(BLOCK, NB >= 8 ? DYCG_MULTI_MIN_BLOCKS : 3)
     // 5. frontier: affected (v, q) with a finite value, then insertion seeds
     const uint32_t ftag = tag++;
     if (P.phases & PH_DELETE) {
-      const uint32_t na = *(volatile uint32_t *)&ctl->snap_aff;
       for (uint32_t i = gw; i < na; i += nw) {
         const uint32_t v = P.aff[i];
         bool any = false;
@@ -1130,19 +1099,21 @@ __global__ void __launch_bounds__(BLOCK, NB >= 8 ? DYCG_MULTI_MIN_BLOCKS : 3)
       }
     }
   }
-  if (!grid_sync(ctl, 0, P.timeout_ns)) goto done;
+  sn = grid_sync(ctl, gen, 0, SEL_Q0, P.timeout_ns);
+  if (!sn.ok) goto done;
   if (gtid == 0) ctl->tphase[2] = globaltimer_ns();  // frontier + insertion seeds done
   // 6. closure waves (or one asynchronous phase)
   if ((P.phases & PH_CLOSE) && P.async) {
-    const uint32_t cnt = *(volatile uint32_t *)&ctl->snap_q[0];
+    const uint32_t cnt = sn.cnt;
     RelaxPh<ALGO, STORED, NB> ph{&P, P.nmask[0], QPAR_ASYNC, tag++};
-    if (!async_phase<NB, STORED>(P, P.out, P.q[0], cnt, P.nmask[0], ph, s, acc, P.qratio))
+    if (!async_phase<NB, STORED>(P, P.out, P.q[0], cnt, P.nmask[0], ph, s, acc, gen,
+                                 P.qratio))
       goto done;
     waves++;
   } else if (P.phases & PH_CLOSE) {
     uint32_t cur = 0;
     for (uint32_t wave = 0;; wave++) {
-      const uint32_t cnt = *(volatile uint32_t *)&ctl->snap_q[cur];
+      const uint32_t cnt = sn.cnt;
       if (cnt == 0) break;
       if (wave >= P.max_waves) {
         if (gtid == 0) atomicCAS(&ctl->err, 0u, ERR_WAVES);
@@ -1152,9 +1123,10 @@ __global__ void __launch_bounds__(BLOCK, NB >= 8 ? DYCG_MULTI_MIN_BLOCKS : 3)
       RelaxPh<ALGO, STORED, NB> ph{&P, P.nmask[par ^ 1], cur ^ 1, tag++};
       uint32_t *src = P.nmask[par];
       auto prep = [&](uint32_t v, uint32_t (&m)[NB]) { return take_masks<NB>(src, v, true, m); };
-      if (!multi_expand<NB, STORED>(P, P.out, P.q[cur], cnt, prep, ph, s, s_stage, acc, cur,
-                                    cur ? SYNC_RESET_Q1 : SYNC_RESET_Q0, P.qratio))
-        goto done;
+      sn = multi_expand<NB, STORED>(P, P.out, P.q[cur], cnt, prep, ph, s, s_stage, acc, gen, cur,
+                                    cur ? SEL_Q0 : SEL_Q1, cur ? SYNC_RESET_Q1 : SYNC_RESET_Q0,
+                                    P.qratio);
+      if (!sn.ok) goto done;
       waves++;
       cur ^= 1;
     }
@@ -1162,7 +1134,6 @@ __global__ void __launch_bounds__(BLOCK, NB >= 8 ? DYCG_MULTI_MIN_BLOCKS : 3)
   if (gtid == 0) ctl->tphase[3] = globaltimer_ns();  // closure done
   // 7. clear the snapshot's affected masks
   if (P.phases & PH_DELETE) {
-    const uint32_t na = *(volatile uint32_t *)&ctl->snap_aff;
     for (uint32_t i = gw; i < na; i += nw)
       if (lane < (uint32_t)NB) P.affm[(u64)P.aff[i] * NB + lane] = 0;
   }
@@ -1171,7 +1142,7 @@ done:
   __syncthreads();
   if (threadIdx.x == 0) atomicMax(&ctl->stat[ST_T_END], globaltimer_ns());
   if (gtid == 0) {
-    atomicAdd(&ctl->stat[ST_AFFECTED], (u64)ctl->snap_aff);
+    atomicAdd(&ctl->stat[ST_AFFECTED], (u64)na);
     ctl->waves = waves;
     ctl->wave_tag = tag;
     P.seq[0] = epoch + 1;

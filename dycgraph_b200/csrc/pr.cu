@@ -59,25 +59,25 @@ __device__ __forceinline__ bool pr_add(const PrParams *P, uint32_t dst, float c)
 
 // Pushes c to UNROLL targets per lane: the atomics first (independent, in
 // flight together), then Frontier::Add's crossing test on each result.
-template <int U>
 __device__ __forceinline__ void push_batch(const PrParams *P, uint32_t *outq, uint32_t *outc,
-                                           const uint32_t (&y)[U], const bool (&valid)[U], float c,
-                                           Acc &acc) {
-  float old[U];
+                                           const uint32_t (&y)[UNROLL],
+                                           const bool (&valid)[UNROLL], float c, Acc &acc) {
+  float old[UNROLL];
+  bool want[UNROLL];
 #pragma unroll
-  for (int u = 0; u < U; u++) old[u] = valid[u] ? atomicAdd(P->r + y[u], c) : 0.f;
+  for (int u = 0; u < UNROLL; u++) old[u] = valid[u] ? atomicAdd(P->r + y[u], c) : 0.f;
 #pragma unroll
-  for (int u = 0; u < U; u++) {
-    bool want = false;
+  for (int u = 0; u < UNROLL; u++) {
+    want[u] = false;
     if (valid[u]) {
       const float nv = old[u] + c;
       if (!isfinite(nv)) atomicCAS(&P->ctl->err, 0u, ERR_NONFINITE);
-      want = fabsf(old[u]) <= P->eps && fabsf(nv) > P->eps &&
-             atomicCAS(P->queued + y[u], 0u, 1u) == 0u;
+      want[u] = fabsf(old[u]) <= P->eps && fabsf(nv) > P->eps &&
+                atomicCAS(P->queued + y[u], 0u, 1u) == 0u;
       acc.improved++;
     }
-    warp_append(outq, outc, P->n, want, y[u], &P->ctl->err);
   }
+  append_batch(outq, outc, P->n, want, y, &P->ctl->err);
 }
 
 __device__ __forceinline__ uint32_t old_degree(const PrParams *P, uint32_t u) {
@@ -92,7 +92,11 @@ struct AmendOp {
   struct Row {
     float c;
   };
-  __device__ bool begin(uint32_t u, Row &row) {
+  __device__ bool admit(uint32_t, bool on) { return on; }
+  template <int G>
+  __device__ bool begin(uint32_t u, bool on, Row &row) {
+    row.c = 0.f;
+    if (!on) return false;
     const uint32_t dn = P->out.live[u], dold = old_degree(P, u);
     const float xu = P->x[u];
     if (!dn || dn == dold || xu == 0.f) return false;
@@ -102,13 +106,12 @@ struct AmendOp {
                  : P->alpha * xu / (float)dn;
     return row.c != 0.f;
   }
-  static constexpr int kBatch = 1;
-  template <int U>
-  __device__ void edges(uint32_t, const uint32_t (&y)[U], const bool (&valid)[U], Row &row,
-                        Acc &acc) {
+  __device__ void edges(uint32_t, const uint32_t (&y)[UNROLL], const uint32_t (&)[UNROLL],
+                        const bool (&valid)[UNROLL], Row &row, Acc &acc) {
     push_batch(P, outq, outc, y, valid, row.c, acc);
   }
-  __device__ void end(uint32_t, Row &) {}
+  template <int G>
+  __device__ void end(uint32_t, bool, Row &) {}
 };
 
 struct ScatterOp {
@@ -118,20 +121,23 @@ struct ScatterOp {
   struct Row {
     float c;
   };
-  __device__ bool begin(uint32_t v, Row &row) {
+  __device__ bool admit(uint32_t, bool on) { return on; }
+  template <int G>
+  __device__ bool begin(uint32_t v, bool on, Row &row) {
+    row.c = 0.f;
+    if (!on) return false;
     const float d = P->delta[v];
     const uint32_t deg = P->out.live[v];
     if (d == 0.f || !deg) return false;
     row.c = P->alpha * d / (float)deg;
     return true;
   }
-  static constexpr int kBatch = 1;
-  template <int U>
-  __device__ void edges(uint32_t, const uint32_t (&y)[U], const bool (&valid)[U], Row &row,
-                        Acc &acc) {
+  __device__ void edges(uint32_t, const uint32_t (&y)[UNROLL], const uint32_t (&)[UNROLL],
+                        const bool (&valid)[UNROLL], Row &row, Acc &acc) {
     push_batch(P, outq, outc, y, valid, row.c, acc);
   }
-  __device__ void end(uint32_t, Row &) {}
+  template <int G>
+  __device__ void end(uint32_t, bool, Row &) {}
 };
 
 // The per-occurrence shares of the amend: -alpha x[u]/deg_old for each
@@ -171,24 +177,25 @@ __device__ void amend_records(const PrParams &P, uint32_t cur, Acc &acc) {
   }
 }
 
-__global__ void __launch_bounds__(BLOCK) pr_kernel(PrParams P) {
+__global__ void __launch_bounds__(BLOCK) pr_kernel(const __grid_constant__ PrParams P) {
   Ctl *ctl = P.ctl;
   Acc acc = {0, 0, 0, 0, 0};
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t gstride = gridDim.x * blockDim.x;
-  uint32_t cur = P.cur;
+  uint32_t cur = P.cur, gen = 0;
+  Snap sn;
   if (P.phases & PR_AMEND) {
     amend_records(P, cur, acc);
     AmendOp op{&P, P.q[cur], &ctl->q_count[cur]};
-    if (!expand_rows<false>(P.out, P.sources, *P.n_sources, op, acc, P.tiles, ctl, 0,
-                            P.timeout_ns))
-      goto done;
+    sn = expand_rows<false>(P.out, P.sources, *P.n_sources, op, acc, P.tiles, ctl, gen,
+                            cur ? SEL_Q1 : SEL_Q0, 0, P.timeout_ns);
   } else {
-    if (!grid_sync(ctl, 0, P.timeout_ns)) goto done;
+    sn = grid_sync(ctl, gen, 0, cur ? SEL_Q1 : SEL_Q0, P.timeout_ns);
   }
+  if (!sn.ok) goto done;
   if (P.phases & PR_CONVERGE) {
     for (uint32_t round = 0; round < P.max_rounds; round++) {
-      const uint32_t cnt = *(volatile uint32_t *)&ctl->snap_q[cur];
+      const uint32_t cnt = sn.cnt;
       if (cnt == 0) break;
       // Consume
       for (uint32_t i = gtid; i < cnt; i += gstride) {
@@ -204,12 +211,15 @@ __global__ void __launch_bounds__(BLOCK) pr_kernel(PrParams P) {
           P.delta[v] = 0.f;
         }
       }
-      if (!grid_sync(ctl, cur ? SYNC_RESET_Q0 : SYNC_RESET_Q1, P.timeout_ns)) goto done;
+      sn = grid_sync(ctl, gen, cur ? SYNC_RESET_Q0 : SYNC_RESET_Q1, cur ? SEL_Q1 : SEL_Q0,
+                     P.timeout_ns);
+      if (!sn.ok) goto done;
       // Scatter
       ScatterOp op{&P, P.q[cur ^ 1], &ctl->q_count[cur ^ 1]};
-      if (!expand_rows<false>(P.out, P.q[cur], cnt, op, acc, P.tiles, ctl,
-                              cur ? SYNC_RESET_Q1 : SYNC_RESET_Q0, P.timeout_ns))
-        goto done;
+      sn = expand_rows<false>(P.out, P.q[cur], cnt, op, acc, P.tiles, ctl, gen,
+                              cur ? SEL_Q0 : SEL_Q1, cur ? SYNC_RESET_Q1 : SYNC_RESET_Q0,
+                              P.timeout_ns);
+      if (!sn.ok) goto done;
       cur ^= 1;
       if (gtid == 0) ctl->waves = round + 1;
     }

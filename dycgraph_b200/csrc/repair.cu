@@ -6,23 +6,29 @@
 //      where u is v's parent, v is affected (reset_del_edges,
 //      include/framework/variants/driver.cuh:401-441, IsDeletionDependency
 //      api.cuh:42-49; with parents always tight the rule reduces to parent==u).
+//      Whoever marks a vertex affected resets its state (reset_affected_values,
+//      driver.cuh:448-463).
 //   2. invalidation waves: children y of affected x (parent(y)==x) become
 //      affected (PushFunctorDB_Del, push_functor.h:1180-1213), over out-rows.
-//   3. reset affected state (reset_affected_values, driver.cuh:448-463).
-//   4. pull: each affected v takes min over live in-edges of
+//   3. pull: each affected v takes min over live in-edges of
 //      (value(x)+w, parent x) (GpuAffectedPullRelax, framework.cuh:189-263;
-//      equal values break toward the smaller parent).
-//   5. frontier: affected vertices with a finite value, plus insertion seeds
-//      (SeedAddedEdgeFrontier, framework.cuh:297-370).
-//   6. closure waves: push relaxation until the frontier is empty
+//      equal values break toward the smaller parent) and enters the frontier
+//      when it has a value; insertion seeds (SeedAddedEdgeFrontier,
+//      framework.cuh:297-370).
+//   4. closure waves: push relaxation until the frontier is empty
 //      (RunExactGpuClosure, framework.cuh:504-616, AccumulateBuffer
 //      samples/hybrid_sssp/hybrid_sssp.cu:125-145).
-// The reference drives phases 2 and 4 from the host with one synchronisation
-// per level/iteration; here the whole repair is a single launch.
+// The reference drives phases 2 and 3 from the host with one synchronisation
+// per level/iteration; here the whole repair is a single launch. What bounds it
+// on small and ordinary snapshots is latency: the grid barriers and each wave's
+// chain of dependent accesses, so phases are merged where their order does not
+// matter and a lane's independent accesses are issued together.
 #include "frontier.cuh"
 #include "internal.h"
 
 namespace dycg {
+
+constexpr int REPAIR_BLOCK = 1024;
 
 struct RepairParams {
   Adj out, in;
@@ -45,7 +51,6 @@ struct RepairParams {
   uint32_t phases;
   uint32_t max_waves;
   uint32_t delta;           // ordered closure: expand values < wave min + delta (0: unordered)
-  uint32_t *q2;             // ordered closure: the wave's bucket
   uint32_t *tag_dev;        // non-null: wave tags start at *tag_dev, which the
                             // launch advances past the tags it used
   u64 timeout_ns;
@@ -57,333 +62,289 @@ __device__ __forceinline__ u64 reset_key(uint32_t v) {
   return ALGO == ALGO_CC ? pack_key(v, 0) : KEY_INF;
 }
 
-// Children of an affected vertex become affected.
+// Children of an affected vertex become affected; whoever marks one resets its
+// key at once (nobody needs its old parent any more: an affected vertex enters
+// the list once), so no pass over the affected list is spent on that.
 template <uint32_t ALGO>
 struct InvalidateOp {
   const RepairParams *P;
   struct Row {};
-  __device__ bool begin(uint32_t, Row &) { return true; }
-  __device__ void edge(uint32_t x, uint32_t y, uint32_t, bool valid, Row &, Acc &) {
-    bool want = false;
-    if (valid && !(ALGO != ALGO_CC && y == P->source)) {
-      if (key_parent1(ld_key(P->key + y)) == x + 1u)
-        want = atomicExch(P->mark + y, P->epoch) != P->epoch;
+  __device__ bool admit(uint32_t, bool on) { return on; }
+  template <int G>
+  __device__ bool begin(uint32_t, bool on, Row &) { return on; }
+  __device__ void edges(uint32_t x, const uint32_t (&y)[UNROLL], const uint32_t (&)[UNROLL],
+                        const bool (&valid)[UNROLL], Row &, Acc &) {
+    u64 k[UNROLL];
+    uint32_t old[UNROLL];
+    bool want[UNROLL];
+#pragma unroll
+    for (int u = 0; u < UNROLL; u++) k[u] = valid[u] ? ld_key(P->key + y[u]) : 0;
+#pragma unroll
+    for (int u = 0; u < UNROLL; u++) {
+      want[u] = valid[u] && !(ALGO != ALGO_CC && y[u] == P->source) && key_parent1(k[u]) == x + 1u;
+      if (want[u]) old[u] = atomicExch(P->mark + y[u], P->epoch);
     }
-    warp_append(P->aff, &P->ctl->n_aff, P->n, want, y, &P->ctl->err);
+#pragma unroll
+    for (int u = 0; u < UNROLL; u++) {
+      want[u] = want[u] && old[u] != P->epoch;
+      if (want[u]) P->key[y[u]] = reset_key<ALGO>(y[u]);
+    }
+    append_batch(P->aff, &P->ctl->n_aff, P->n, want, y, &P->ctl->err);
   }
-  __device__ void end(uint32_t, Row &) {}
+  template <int G>
+  __device__ void end(uint32_t, bool, Row &) {}
 };
 
-// Affected v pulls the best candidate over its live in-edges.
+// Ordered closure: ctl->vmin holds the complement of the next wave's minimum
+// (so that a cleared control block means "none yet").
+__device__ __forceinline__ void note_min(Ctl *ctl, uint32_t value) {
+  value = __reduce_min_sync(0xffffffffu, value);
+  if (lane_id() == 0 && value != INF32) atomicMax(&ctl->vmin, ~value);
+}
+
+// Affected v pulls the best candidate over its live in-edges and enters the
+// closure's first frontier when it has a value (a CC vertex always has its own
+// id). A vertex lowered later, by an insertion seed of the same phase, enters
+// it through that seed.
 template <uint32_t ALGO, bool STORED>
 struct PullOp {
   const RepairParams *P;
+  uint32_t tag;
   struct Row {
     u64 best;
   };
-  __device__ bool begin(uint32_t, Row &r) {
+  __device__ bool admit(uint32_t, bool on) { return on; }
+  template <int G>
+  __device__ bool begin(uint32_t, bool on, Row &r) {
     r.best = KEY_INF;
-    return true;
+    return on;
   }
-  __device__ void edge(uint32_t v, uint32_t x, uint32_t w, bool valid, Row &r, Acc &) {
-    if (!valid) return;
-    const u64 kx = ld_key(P->key + x);
-    const uint32_t vx = key_value(kx);
-    if (vx == INF32) return;
-    const u64 c = (u64)vx + (STORED ? w : rule_weight<ALGO>(x, v));
-    if (c >= INF32) return;
-    const u64 cand = pack_key((uint32_t)c, x + 1u);
-    r.best = cand < r.best ? cand : r.best;
-  }
-  __device__ void end(uint32_t v, Row &r) {
-    const u64 m = warp_min_all(r.best);
-    if (lane_id() == 0 && m != KEY_INF) {
-      if (Strict<ALGO, STORED>::value) strict_lower(P->key + v, m);
-      else atomicMin(P->key + v, m);
+  __device__ void edges(uint32_t v, const uint32_t (&x)[UNROLL], const uint32_t (&w)[UNROLL],
+                        const bool (&valid)[UNROLL], Row &r, Acc &) {
+    u64 k[UNROLL];
+#pragma unroll
+    for (int u = 0; u < UNROLL; u++) k[u] = valid[u] ? ld_key(P->key + x[u]) : KEY_INF;
+#pragma unroll
+    for (int u = 0; u < UNROLL; u++) {
+      const uint32_t vx = key_value(k[u]);
+      if (vx == INF32) continue;
+      const u64 c = (u64)vx + (STORED ? w[u] : rule_weight<ALGO>(x[u], v));
+      if (c >= INF32) continue;
+      const u64 cand = pack_key((uint32_t)c, x[u] + 1u);
+      r.best = cand < r.best ? cand : r.best;
     }
+  }
+  template <int G>
+  __device__ void end(uint32_t v, bool on, Row &r) {
+    u64 m = r.best;
+    if (G == 32) {
+      m = warp_min_all(m);
+    } else {
+#pragma unroll
+      for (int o = G / 2; o; o >>= 1) {
+        const u64 x = __shfl_xor_sync(0xffffffffu, m, o);
+        m = x < m ? x : m;
+      }
+    }
+    bool want[1] = {on && (lane_id() & (G - 1)) == 0 && (ALGO == ALGO_CC || m != KEY_INF)};
+    const uint32_t val[1] = {v};
+    if (want[0]) {
+      if (m != KEY_INF) lower_from<Strict<ALGO, STORED>::value>(P->key + v, m, ld_key(P->key + v));
+      want[0] = atomicExch(P->wtag + v, tag) != tag;
+    }
+    if (P->delta)
+      note_min(P->ctl, want[0] ? min(key_value(m), ALGO == ALGO_CC ? v : INF32) : INF32);
+    append_batch(P->q[0], &P->ctl->q_count[0], P->n, want, val, &P->ctl->err);
   }
 };
 
 // Push relaxation of the out-edges of a frontier vertex. In the ordered
-// closure (vmin set) every improvement also lowers *vmin, the next wave's
-// running minimum.
+// closure (P->delta) only vertices below thr are expanded: the others are
+// carried to the next queue, and every carried value and improvement lowers
+// the next wave's minimum.
 template <uint32_t ALGO, bool STORED>
 struct RelaxOp {
   const RepairParams *P;
   uint32_t *outq;
   uint32_t *outc;
   uint32_t tag;
-  uint32_t *vmin;  // ordered closure: running minimum of the next wave (or null)
+  uint32_t thr;
+  static constexpr bool STRICT = Strict<ALGO, STORED>::value;
   struct Row {
-    uint32_t dv;
+    uint32_t dv, imp;  // the vertex's value; the lowest value this lane pushed
   };
-  __device__ bool begin(uint32_t x, Row &r) {
+  __device__ bool admit(uint32_t v, bool on) {
+    if (!P->delta) return on;
+    const bool lead = (lane_id() & 7) == 0;  // a group's lanes hold the same item
+    const uint32_t d = on ? key_value(ld_key(P->key + v)) : INF32;
+    // one read decides for the whole group
+    const uint32_t dv = __shfl_sync(0xffffffffu, d, 0, 8);
+    const bool later = on && dv != INF32 && dv >= thr;
+    if (__any_sync(0xffffffffu, later)) {
+      const uint32_t val[1] = {v};
+      const bool want[1] = {later && lead && atomicExch(P->wtag + v, tag) != tag};
+      append_batch(outq, outc, P->n, want, val, &P->ctl->err);
+      note_min(P->ctl, later ? dv : INF32);
+    }
+    return on && dv < thr;
+  }
+  template <int G>
+  __device__ bool begin(uint32_t x, bool on, Row &r) {
     // one read, broadcast: the key may change under concurrent relaxations
-    r.dv = __shfl_sync(0xffffffffu, key_value(ld_key(P->key + x)), 0);
+    r.dv = __shfl_sync(0xffffffffu, on ? key_value(ld_key(P->key + x)) : INF32, 0, G);
+    r.imp = INF32;
     return r.dv != INF32;
   }
-  __device__ void edge(uint32_t x, uint32_t y, uint32_t w, bool valid, Row &r, Acc &acc) {
-    bool want = false;
-    uint32_t imp = INF32;  // value this lane lowered y to
-    if (valid) {
-      const u64 c = (u64)r.dv + (STORED ? w : rule_weight<ALGO>(x, y));
-      if (c < INF32) {
-        const u64 cand = pack_key((uint32_t)c, x + 1u);
-        bool lowered = false;
-        if (Strict<ALGO, STORED>::value) {
-          lowered = strict_lower(P->key + y, cand);
-        } else if (cand < ld_key(P->key + y)) {
-          lowered = key_value(atomicMin(P->key + y, cand)) > (uint32_t)c;
-        }
-        if (lowered) {
-          acc.improved++;
-          want = atomicExch(P->wtag + y, tag) != tag;
-          imp = (uint32_t)c;
-        }
+  __device__ void edges(uint32_t x, const uint32_t (&y)[UNROLL], const uint32_t (&w)[UNROLL],
+                        const bool (&valid)[UNROLL], Row &r, Acc &acc) {
+    // a lane's four keys, then its four first attempts, then its four tags:
+    // each set of independent accesses in flight together
+    u64 cand[UNROLL], cur[UNROLL], got[UNROLL];
+    bool want[UNROLL];
+#pragma unroll
+    for (int u = 0; u < UNROLL; u++) {
+      const u64 c = (u64)r.dv + (STORED ? w[u] : rule_weight<ALGO>(x, y[u]));
+      cand[u] = valid[u] && c < INF32 ? pack_key((uint32_t)c, x + 1u) : KEY_INF;
+      cur[u] = cand[u] != KEY_INF ? ld_key(P->key + y[u]) : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < UNROLL; u++)
+      want[u] = first_lower<STRICT>(P->key + y[u], cand[u], cur[u], got[u]);
+    uint32_t old[UNROLL];
+#pragma unroll
+    for (int u = 0; u < UNROLL; u++) {
+      want[u] = want[u] && lowered<STRICT>(P->key + y[u], cand[u], cur[u], got[u]);
+      if (want[u]) {
+        acc.improved++;
+        r.imp = min(r.imp, key_value(cand[u]));
+        old[u] = atomicExch(P->wtag + y[u], tag);
       }
     }
-    warp_append(outq, outc, P->n, want, y, &P->ctl->err);
-    if (vmin) {
-      imp = __reduce_min_sync(0xffffffffu, imp);
-      if (lane_id() == 0 && imp != INF32) atomicMin(vmin, imp);
-    }
+#pragma unroll
+    for (int u = 0; u < UNROLL; u++) want[u] = want[u] && old[u] != tag;
+    append_batch(outq, outc, P->n, want, y, &P->ctl->err);
   }
-  __device__ void end(uint32_t, Row &) {}
+  template <int G>
+  __device__ void end(uint32_t, bool, Row &r) {
+    if (P->delta) note_min(P->ctl, r.imp);
+  }
 };
 
-// One wave of the ordered closure in a single pass: a warp takes 32
-// consecutive queue items, its lanes split them by value (below thr: expand
-// now; at or above: carry to the next queue, with the carried values' minimum
-// lowering the next wave's running minimum, one atomic per warp), then the
-// warp expands the items kept for now one by one (rows longer than HEAVY as
-// CTA tiles after the barrier, as expand_rows does).
-template <bool WITH_W, class Op>
-__device__ bool expand_ordered(const RepairParams &P, const uint32_t *items, uint32_t cnt,
-                               uint32_t thr, Op &op, Acc &acc, Ctl *ctl, uint32_t reset_flags) {
-  const Adj &A = P.out;
-  const uint32_t lane = lane_id();
-  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t i0 = gw * 32; i0 < cnt; i0 += nw * 32) {
-    const uint32_t i = i0 + lane;
-    uint32_t v = 0, dv = INF32;
-    if (i < cnt) {
-      v = items[i];
-      dv = key_value(ld_key(P.key + v));
-    }
-    const bool now = dv < thr;
-    const bool carry = dv != INF32 && !now && atomicExch(P.wtag + v, op.tag) != op.tag;
-    warp_append(op.outq, op.outc, P.n, carry, v, &ctl->err);
-    const uint32_t cm = __reduce_min_sync(0xffffffffu, carry ? dv : INF32);
-    if (lane == 0 && cm != INF32) atomicMin(op.vmin, cm);
-    unsigned todo = __ballot_sync(0xffffffffu, now);
-    while (todo) {
-      const int src = __ffs(todo) - 1;
-      todo &= todo - 1;
-      const uint32_t x = __shfl_sync(0xffffffffu, v, src);
-      const uint32_t len = A.len[x];
-      if (len > HEAVY) {
-        if (lane == 0) {
-          const uint32_t nt = (len + TILE - 1) / TILE;
-          const uint32_t base = atomicAdd(&ctl->tile_count, nt);
-          if (base + nt > P.tiles.cap) {
-            atomicCAS(&ctl->err, 0u, ERR_TILES);
-          } else {
-            for (uint32_t t = 0; t < nt; t++)
-              P.tiles.tiles[base + t] = make_uint4(x, t * TILE, min(len, (t + 1) * TILE), 0);
-          }
-        }
-        continue;
-      }
-      warp_slots<WITH_W>(A, x, A.off[x], 0, len, 32, op, acc);
-    }
-  }
-  if (!grid_sync(ctl, reset_flags, P.timeout_ns)) return false;
-  const uint32_t nt = min(*(volatile uint32_t *)&ctl->snap_tiles, P.tiles.cap);
-  if (nt == 0) return true;
-  const uint32_t wib = threadIdx.x >> 5;
-  for (uint32_t t = blockIdx.x; t < nt; t += gridDim.x) {
-    const uint4 tl = P.tiles.tiles[t];
-    warp_slots<WITH_W>(A, tl.x, A.off[tl.x], tl.y + wib * 32, tl.z, blockDim.x, op, acc);
-  }
-  return grid_sync(ctl, SYNC_RESET_TILES, P.timeout_ns);
-}
-
+// 1024-thread CTAs, one per SM: the same warps in flight as four CTAs of 256,
+// and a quarter of the arrivals at every grid barrier (512 and 768 threads: the
+// same on short waves, 3-9% slower on 100K-update snapshots). Measured with the
+// merged phases and the batched accesses, kernel time per snapshot before ->
+// now: R-MAT 16 SSSP 2K updates 0.24 -> 0.14 ms, R-MAT 20 BFS 10K 0.24 -> 0.12
+// ms, R-MAT 21 SSSP 100K 0.73 -> 0.36 ms, 1024^2 grid SSSP 1K (1,580 ordered
+// waves) 39.4 -> 20.2 ms.
 template <uint32_t ALGO, bool STORED>
-__global__ void __launch_bounds__(BLOCK) repair_kernel(RepairParams P) {
+__global__ void __launch_bounds__(REPAIR_BLOCK, 1) repair_kernel(const __grid_constant__ RepairParams P) {
   Ctl *ctl = P.ctl;
   Acc acc = {0, 0, 0, 0, 0};
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t gstride = gridDim.x * blockDim.x;
   const uint32_t lane = lane_id();
   const uint32_t tag_base = P.tag_dev ? *(volatile uint32_t *)P.tag_dev : P.tag_base;
+  // short record lists: warp k of every block before warp k + 1 of any
+  const uint32_t first = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32;
+  uint32_t gen = 0, na = 0, cur = 0;
+  Snap sn;
   if (gtid == 0) ctl->stat[ST_T_START] = globaltimer_ns();
 
   if (P.phases & PH_DELETE) {
     // 1. deletion seeds (warp-uniform loop so appends can aggregate)
     const uint32_t n_del = *P.n_del_ptr;
-    for (uint32_t i0 = gtid - lane; i0 < n_del; i0 += gstride) {
+    for (uint32_t i0 = first; i0 < n_del; i0 += gstride) {
       const uint32_t i = i0 + lane;
-      bool want = false;
-      uint32_t v = 0;
+      bool want[1] = {false};
+      uint32_t v[1] = {0};
       if (i < n_del && P.del_found[i] != 0) {
         const uint2 e = P.del_uv[i];
-        v = e.y;
-        if (!(ALGO != ALGO_CC && v == P.source) &&
-            key_parent1(ld_key(P.key + v)) == e.x + 1u)
-          want = atomicExch(P.mark + v, P.epoch) != P.epoch;
-      }
-      warp_append(P.aff, &ctl->n_aff, P.n, want, v, &ctl->err);
-    }
-    if (!grid_sync(ctl, 0, P.timeout_ns)) goto done;
-    // 2. invalidation waves over the growing affected list
-    {
-      uint32_t lo = 0;
-      for (;;) {
-        const uint32_t hi = *(volatile uint32_t *)&ctl->snap_aff;
-        if (hi == lo) break;
-        InvalidateOp<ALGO> op{&P};
-        if (!expand_rows<false>(P.out, P.aff + lo, hi - lo, op, acc, P.tiles, ctl, 0,
-                                P.timeout_ns, P.claimed))
-          goto done;
-        lo = hi;
-      }
-    }
-    if (gtid == 0) ctl->tphase[0] = globaltimer_ns();  // seeds + invalidation done
-    // 3. reset
-    {
-      const uint32_t na = *(volatile uint32_t *)&ctl->snap_aff;
-      for (uint32_t i = gtid; i < na; i += gstride) {
-        const uint32_t v = P.aff[i];
-        P.key[v] = reset_key<ALGO>(v);
-      }
-      if (!grid_sync(ctl, 0, P.timeout_ns)) goto done;
-      // 4. pull over incoming rows
-      PullOp<ALGO, STORED> op{&P};
-      if (!expand_rows<STORED>(P.in, P.aff, na, op, acc, P.tiles, ctl, 0, P.timeout_ns, P.claimed))
-        goto done;
-      if (gtid == 0) ctl->tphase[1] = globaltimer_ns();  // reset + pull done
-      // 5a. frontier from affected vertices with a finite value
-      for (uint32_t i0 = gtid - lane; i0 < na; i0 += gstride) {
-        const uint32_t i = i0 + lane;
-        bool want = false;
-        uint32_t v = 0;
-        if (i < na) {
-          v = P.aff[i];
-          if (key_value(ld_key(P.key + v)) != INF32)
-            want = atomicExch(P.wtag + v, tag_base) != tag_base;
+        v[0] = e.y;
+        if (!(ALGO != ALGO_CC && e.y == P.source) &&
+            key_parent1(ld_key(P.key + e.y)) == e.x + 1u) {
+          want[0] = atomicExch(P.mark + e.y, P.epoch) != P.epoch;
+          if (want[0]) P.key[e.y] = reset_key<ALGO>(e.y);
         }
-        warp_append(P.q[0], &ctl->q_count[0], P.n, want, v, &ctl->err);
       }
+      append_batch(P.aff, &ctl->n_aff, P.n, want, v, &ctl->err);
     }
+    sn = grid_sync(ctl, gen, 0, SEL_AFF, P.timeout_ns);
+    // 2. invalidation waves over the growing affected list
+    while (sn.ok && sn.cnt != na) {
+      InvalidateOp<ALGO> op{&P};
+      const uint32_t lo = na;
+      na = sn.cnt;
+      sn = expand_rows<false>(P.out, P.aff + lo, na - lo, op, acc, P.tiles, ctl, gen, SEL_AFF, 0,
+                              P.timeout_ns, P.claimed);
+    }
+    if (!sn.ok) goto done;
+    if (gtid == 0) ctl->tphase[0] = globaltimer_ns();  // seeds + invalidation done
   }
+  // 3. insertion seeds and the pull over the affected vertices' in-rows, one
+  // phase: whatever either reads is an upper bound of a live path, and every
+  // vertex either lowers enters the first frontier
   if (P.phases & PH_INSERT) {
-    // 5b. insertion seeds
-    for (uint32_t i0 = gtid - lane; i0 < P.n_add; i0 += gstride) {
+    for (uint32_t i0 = first; i0 < P.n_add; i0 += gstride) {
       const uint32_t i = i0 + lane;
-      bool want = false;
-      uint32_t v = 0;
+      bool want[1] = {false};
+      uint32_t v[1] = {0}, imp = INF32;
       const uint3 e = i < P.n_add ? P.add_uvw[i] : make_uint3(INF32, INF32, 0);
       if (e.x < P.n) {
-        v = e.y;
+        v[0] = e.y;
         const uint32_t du = key_value(ld_key(P.key + e.x));
         if (du != INF32) {
           const u64 c = (u64)du + (STORED ? e.z : rule_weight<ALGO>(e.x, e.y));
-          if (c < INF32) {
-            const u64 cand = pack_key((uint32_t)c, e.x + 1u);
-            bool lowered = false;
-            if (Strict<ALGO, STORED>::value) {
-              lowered = strict_lower(P.key + v, cand);
-            } else if (cand < ld_key(P.key + v)) {
-              lowered = key_value(atomicMin(P.key + v, cand)) > (uint32_t)c;
-            }
-            if (lowered) want = atomicExch(P.wtag + v, tag_base) != tag_base;
+          if (c < INF32 &&
+              lower_from<Strict<ALGO, STORED>::value>(
+                  P.key + e.y, pack_key((uint32_t)c, e.x + 1u), ld_key(P.key + e.y))) {
+            want[0] = atomicExch(P.wtag + e.y, tag_base) != tag_base;
+            imp = (uint32_t)c;
           }
         }
       }
-      warp_append(P.q[0], &ctl->q_count[0], P.n, want, v, &ctl->err);
+      if (P.delta) note_min(ctl, imp);
+      append_batch(P.q[0], &ctl->q_count[0], P.n, want, v, &ctl->err);
     }
   }
-  if (!grid_sync(ctl, SYNC_RESET_VMIN, P.timeout_ns)) goto done;
-  if (gtid == 0) ctl->tphase[2] = globaltimer_ns();  // frontier + insertion seeds done
-  // 6. closure waves
-  if ((P.phases & PH_CLOSE) && P.delta) {
-    // Ordered (bucketed) closure for high-diameter graphs, the B200 form of
-    // the reference's ordered insertion schedule (framework.cuh:537-556):
-    // each wave expands only the frontier vertices whose value is below the
-    // wave's minimum + delta and carries the rest to the next wave, so a
-    // vertex is expanded about once instead of once per improvement. The
-    // next wave's minimum is kept on the fly (carried values and every
-    // improvement lower ctl->vmin, which the wave's closing barrier snapshots
-    // and resets), so only the first wave needs a reduction pass. SSSP and
-    // BFS split each wave's queue into a compact bucket first (a barrier),
-    // which spreads the bucket's rows over all warps (their buckets hold
-    // runs of consecutive queue entries); CC splits and expands in one pass
-    // (its waves are mostly carried entries, for which the split barrier is
-    // the larger cost).
-    uint32_t cur = 0;
-    {
-      const uint32_t cnt = *(volatile uint32_t *)&ctl->snap_q[0];
-      uint32_t m = INF32;
-      for (uint32_t i = gtid; i < cnt; i += gstride)
-        m = min(m, key_value(ld_key(P.key + P.q[0][i])));
-      for (int o = 16; o; o >>= 1) m = min(m, __shfl_down_sync(0xffffffffu, m, o));
-      if (lane == 0 && m != INF32) atomicMin(&ctl->vmin, m);
-      if (!grid_sync(ctl, SYNC_RESET_VMIN, P.timeout_ns)) goto done;
-    }
-    for (uint32_t wave = 0;; wave++) {
-      const uint32_t cnt = *(volatile uint32_t *)&ctl->snap_q[cur];
-      if (cnt == 0) break;
+  if (!(P.phases & (PH_DELETE | PH_INSERT)) && P.delta) {
+    // static solve: the minimum of the frontier it was given
+    const uint32_t cnt = *(volatile uint32_t *)&ctl->q_count[0];
+    for (uint32_t i0 = first; i0 < cnt; i0 += gstride)
+      note_min(ctl, i0 + lane < cnt ? key_value(ld_key(P.key + P.q[0][i0 + lane])) : INF32);
+  }
+  if (na) {
+    PullOp<ALGO, STORED> op{&P, tag_base};
+    sn = expand_rows<STORED>(P.in, P.aff, na, op, acc, P.tiles, ctl, gen, SEL_Q0, SYNC_RESET_VMIN,
+                             P.timeout_ns, P.claimed);
+  } else {
+    sn = grid_sync(ctl, gen, SYNC_RESET_VMIN, SEL_Q0, P.timeout_ns);
+  }
+  if (!sn.ok) goto done;
+  // (the two stages share one phase: its time is reported as the pull's)
+  if (gtid == 0) ctl->tphase[1] = ctl->tphase[2] = globaltimer_ns();
+  // 4. closure waves. Ordered (P.delta, for high-diameter graphs, the B200 form
+  // of the reference's ordered insertion schedule, framework.cuh:537-556): each
+  // wave expands only the frontier vertices whose value is below the wave's
+  // minimum + delta and carries the rest to the next wave, so a vertex is
+  // expanded about once instead of once per improvement. One pass and one
+  // barrier per wave: the expanding warps themselves carry what is above the
+  // threshold, an item per warp (or group), so that the wave's rows spread over
+  // all warps whatever their place in the queue, and the next wave's minimum is
+  // kept on the fly and published by the closing barrier.
+  if (P.phases & PH_CLOSE) {
+    for (uint32_t wave = 0; sn.cnt; wave++) {
       if (wave >= P.max_waves) {
         if (gtid == 0) atomicCAS(&ctl->err, 0u, ERR_WAVES);
         break;
       }
-      const uint32_t tag = tag_base + 1 + wave;
-      const uint32_t vm = *(volatile uint32_t *)&ctl->snap_vmin;
-      const uint32_t thr = vm > INF32 - P.delta ? INF32 : vm + P.delta;
-      RelaxOp<ALGO, STORED> op{&P, P.q[cur ^ 1], &ctl->q_count[cur ^ 1], tag, &ctl->vmin};
-      const uint32_t close = (cur ? SYNC_RESET_Q1 : SYNC_RESET_Q0) | SYNC_RESET_VMIN;
-      if (ALGO == ALGO_CC) {
-        if (!expand_ordered<STORED>(P, P.q[cur], cnt, thr, op, acc, ctl, close)) goto done;
-      } else {
-        // split: values below thr form this wave's bucket, the rest carry over
-        for (uint32_t i0 = gtid - lane; i0 < cnt; i0 += gstride) {
-          const uint32_t i = i0 + lane;
-          uint32_t v = 0, d = INF32;
-          if (i < cnt) {
-            v = P.q[cur][i];
-            d = key_value(ld_key(P.key + v));
-          }
-          const bool now = d < thr;
-          const bool carry = !now && d != INF32 && atomicExch(P.wtag + v, tag) != tag;
-          warp_append(P.q2, &ctl->q_count[2], P.n, now, v, &ctl->err);
-          warp_append(P.q[cur ^ 1], &ctl->q_count[cur ^ 1], P.n, carry, v, &ctl->err);
-          const uint32_t cm = __reduce_min_sync(0xffffffffu, carry ? d : INF32);
-          if (lane == 0 && cm != INF32) atomicMin(&ctl->vmin, cm);
-        }
-        if (!grid_sync(ctl, cur ? SYNC_RESET_Q1 : SYNC_RESET_Q0, P.timeout_ns)) goto done;
-        const uint32_t nb = *(volatile uint32_t *)&ctl->snap_q[2];
-        if (!expand_rows<STORED>(P.out, P.q2, nb, op, acc, P.tiles, ctl,
-                                 SYNC_RESET_Q2 | SYNC_RESET_VMIN, P.timeout_ns, P.claimed))
-          goto done;
-      }
-      if (gtid == 0) ctl->waves = wave + 1;
-      cur ^= 1;
-    }
-  } else if (P.phases & PH_CLOSE) {
-    uint32_t cur = 0;
-    for (uint32_t wave = 0;; wave++) {
-      const uint32_t cnt = *(volatile uint32_t *)&ctl->snap_q[cur];
-      if (cnt == 0) break;
-      if (wave >= P.max_waves) {
-        if (gtid == 0) atomicCAS(&ctl->err, 0u, ERR_WAVES);
-        break;
-      }
-      RelaxOp<ALGO, STORED> op{&P, P.q[cur ^ 1], &ctl->q_count[cur ^ 1], tag_base + 1 + wave,
-                               nullptr};
-      if (!expand_rows<STORED>(P.out, P.q[cur], cnt, op, acc, P.tiles, ctl,
-                               cur ? SYNC_RESET_Q1 : SYNC_RESET_Q0, P.timeout_ns, P.claimed))
-        goto done;
+      const uint32_t thr = sn.vmin > INF32 - P.delta ? INF32 : sn.vmin + P.delta;
+      RelaxOp<ALGO, STORED> op{&P, P.q[cur ^ 1], &ctl->q_count[cur ^ 1], tag_base + 1 + wave, thr};
+      sn = expand_rows<STORED>(P.out, P.q[cur], sn.cnt, op, acc, P.tiles, ctl, gen,
+                               cur ? SEL_Q0 : SEL_Q1,
+                               (cur ? SYNC_RESET_Q1 : SYNC_RESET_Q0) | SYNC_RESET_VMIN,
+                               P.timeout_ns, P.claimed);
+      if (!sn.ok) goto done;
       if (gtid == 0) ctl->waves = wave + 1;
       cur ^= 1;
     }
@@ -392,7 +353,7 @@ __global__ void __launch_bounds__(BLOCK) repair_kernel(RepairParams P) {
 done:
   acc.flush(ctl);
   if (gtid == 0) {
-    atomicAdd(&ctl->stat[ST_AFFECTED], (u64)ctl->snap_aff);
+    atomicAdd(&ctl->stat[ST_AFFECTED], (u64) * (volatile uint32_t *)&ctl->n_aff);
     // every block read *tag_dev before the first barrier
     if (P.tag_dev) *P.tag_dev = tag_base + ctl->waves + 2;
   }
@@ -446,20 +407,19 @@ static cudaError_t launch_one(const RepairLaunch &L, cudaStream_t s) {
   P.phases = L.phases;
   P.max_waves = L.max_waves;
   P.delta = L.delta;
-  P.q2 = L.q2;
   P.tag_dev = L.tag_dev;
   P.timeout_ns = L.timeout_ns;
   P.claimed = L.sched != 0;
   static int blocks_per_sm = -1;
   if (blocks_per_sm < 0) {
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &blocks_per_sm, repair_kernel<ALGO, STORED>, BLOCK, 0);
+        &blocks_per_sm, repair_kernel<ALGO, STORED>, REPAIR_BLOCK, 0);
     if (e != cudaSuccess) return e;
   }
   const int grid = blocks_per_sm * L.num_sms;
   void *args[] = {&P};
-  return cudaLaunchCooperativeKernel((const void *)repair_kernel<ALGO, STORED>, grid, BLOCK,
-                                     args, 0, s);
+  return cudaLaunchCooperativeKernel((const void *)repair_kernel<ALGO, STORED>, grid,
+                                     REPAIR_BLOCK, args, 0, s);
 }
 
 cudaError_t launch_repair(const RepairLaunch &L, cudaStream_t s) {

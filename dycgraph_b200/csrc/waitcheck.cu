@@ -21,7 +21,8 @@ __global__ void wait_check_kernel(Ctl *ctl, const uint32_t *never, int absent, u
     }
     return;
   }
-  grid_sync(ctl, 0, limit_ns);
+  uint32_t gen = 0;
+  grid_sync(ctl, gen, 0, SEL_Q0, limit_ns);
 }
 
 }  // namespace dycg

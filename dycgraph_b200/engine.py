@@ -58,7 +58,7 @@ _STAT_PHASE = ["ms_phase_invalidate", "ms_phase_pull", "ms_phase_seed", "ms_phas
 
 # Bytes of the engine's per-snapshot device control block, which every
 # snapshot call reads back to the host (static_assert in csrc/common.cuh).
-CTL_BYTES = 2904
+CTL_BYTES = 1024
 
 
 class BatchStats(ctypes.Structure):
