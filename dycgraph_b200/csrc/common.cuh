@@ -177,26 +177,6 @@ __device__ __forceinline__ u64 globaltimer_ns() {
   return t;
 }
 
-// Warp-aggregated append of `val` by the lanes with want=true. The calling
-// code keeps the warp converged (loops are warp-uniform).
-__device__ __forceinline__ bool warp_append(uint32_t *q, uint32_t *count, uint32_t cap,
-                                            bool want, uint32_t val, uint32_t *err) {
-  unsigned mask = __activemask();
-  unsigned m = __ballot_sync(mask, want);
-  if (!m) return true;
-  int leader = __ffs(m) - 1;
-  uint32_t base = 0;
-  if ((int)lane_id() == leader) base = atomicAdd(count, (uint32_t)__popc(m));
-  base = __shfl_sync(mask, base, leader);
-  uint32_t rank = __popc(m & ((1u << lane_id()) - 1));
-  if (base + __popc(m) > cap) {
-    if ((int)lane_id() == leader) atomicExch(err, ERR_QUEUE);
-    return false;
-  }
-  if (want) q[base + rank] = val;
-  return true;
-}
-
 __device__ __forceinline__ u64 warp_sum(u64 x) {
   for (int o = 16; o; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
   return x;

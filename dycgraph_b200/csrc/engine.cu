@@ -34,6 +34,7 @@ namespace dycg {
 
 static u64 round_up(u64 x, u64 m) { return (x + m - 1) / m * m; }
 static void fill_phases(dycg_batch_stats *s, const Ctl &c);
+constexpr size_t CTL_CLEAR = 2 * sizeof(Ctl) + 64;  // control blocks and batch counters
 
 Engine::Engine(const dycg_options &opt) : opt_(opt) {
   if (opt_.algo > DYCG_ALGO_PR) throw Error(DYCG_EINVAL, "unknown algorithm");
@@ -75,9 +76,6 @@ Engine::~Engine() {
   if (h_rec_) cudaFreeHost(h_rec_);
   if (d_rec_) cudaFree(d_rec_);
   if (h_bctl_) cudaFreeHost(h_bctl_);
-  for (void *p : {(void *)dbufs_.k_in, (void *)dbufs_.k_out, (void *)dbufs_.v_in,
-                  (void *)dbufs_.v_out, dbufs_.temp})
-    cudaFree(p);
   if (tx_) cudaFree(tx_);
   if (ty_) cudaFree(ty_);
   for (auto &e : pev_)
@@ -290,15 +288,15 @@ void Engine::finish_load() {
   const u64 tcap = maxslots / TILE + maxslots / HEAVY + 4096;
   tile_cap_ = (uint32_t)std::min<u64>(tcap, 0x7FFFFFFFull);
   tiles_ = (uint4 *)dmalloc((u64)tile_cap_ * sizeof(uint4));
-  ctl_ = (Ctl *)dmalloc(sizeof(Ctl));
+  // the snapshot's control block, the mutation launch's, and the batch counters,
+  // cleared together before every snapshot
+  ctl_ = (Ctl *)dmalloc(CTL_CLEAR);
+  mctl_ = ctl_ + 1;
+  counts_ = (uint32_t *)(ctl_ + 2);
   void *hc = nullptr;
   CK(cudaHostAlloc(&hc, sizeof(Ctl), cudaHostAllocDefault));
   hallocs_.push_back(hc);
   h_ctl_ = (Ctl *)hc;
-  void *hdp = nullptr;
-  CK(cudaHostAlloc(&hdp, 8, cudaHostAllocDefault));
-  hallocs_.push_back(hdp);
-  h_dpacked_ = (u64 *)hdp;
   if (opt_.algo == DYCG_ALGO_PR) {
     x_ = (float *)dmalloc((n + 1ull) * 4);
     r_ = (float *)dmalloc((n + 1ull) * 4);
@@ -516,7 +514,7 @@ void Engine::load_grid(uint32_t side, uint32_t permille, uint32_t radius, uint64
 void Engine::init() {
   check_loaded();
   if (inited_) throw Error(DYCG_ESTATE, "engine already initialised");
-  CK(cudaMemsetAsync(ctl_, 0, sizeof(Ctl), st_));
+  CK(cudaMemsetAsync(ctl_, 0, CTL_CLEAR, st_));
   const u64 timeout = 120ull * 1000000000ull;
   if (policy_ == DYCG_CACHE_LEARNED) policy_alloc();
   if (nq_) {
@@ -536,7 +534,7 @@ void Engine::init() {
     L.q0 = q0_;
     L.q1 = q1_;
     L.sources = touched_ ? touched_ : q0_;
-    L.n_sources = counts_ ? counts_ + 4 : nullptr;
+    L.n_sources = counts_;
     L.tiles = tiles_;
     L.tile_cap = tile_cap_;
     L.ctl = ctl_;
@@ -607,8 +605,6 @@ void Engine::reserve_batch(size_t max_records) {
     for (uint32_t c = 1024; c <= top; c *= 2) graph_for(c);
   } else {
     ensure_batch(std::max<size_t>(max_records, 1));
-    // deferred deletions: hub rows' unsorted suffixes, a few slots per record
-    ensure_defer(4ull * max_records);
   }
   sync_check("reserve batch");
 }
@@ -626,174 +622,93 @@ void Engine::ensure_batch(size_t cnt) {
     batch_allocs_.push_back(p);
     return p;
   };
-  k_tmp_out_ = (u64 *)al(c * 8);
-  k_tmp_in_ = (u64 *)al(c * 8);
-  k_del_out_ = (u64 *)al(c * 8);
-  k_del_in_ = (u64 *)al(c * 8);
-  k_add_out_ = (u64 *)al(c * 8);
-  k_add_in_ = (u64 *)al(c * 8);
-  w_tmp_ = (uint32_t *)al(c * 4);
-  w_add_out_ = (uint32_t *)al(c * 4);
-  w_add_in_ = (uint32_t *)al(c * 4);
-  uv_out_ = (uint2 *)al(c * 8);
-  uv_in_ = (uint2 *)al(c * 8);
-  mult_out_ = (uint32_t *)al(c * 4);
-  mult_in_ = (uint32_t *)al(c * 4);
-  found_out_ = (uint32_t *)al(c * 4);
-  seg_out_ = (uint3 *)al(c * 12);
-  seg_in_ = (uint3 *)al(c * 12);
-  add_uvw_ = (uint3 *)al(c * 12);
-  touched_ = (uint32_t *)al(c * 2 * 4);
-  counts_ = (uint32_t *)al(64);
-  reloc_.rec = (RelocRec *)al(c * sizeof(RelocRec));
-  reloc_.cap = (uint32_t)c;
-  {
-    const u64 maxslots = std::max(out_.slots, in_.slots);
-    const u64 cc = std::min<u64>(maxslots / RELOC_CHUNK + c + 1024, 0x7FFFFFFFull);
-    reloc_.chunks = (uint2 *)al(cc * sizeof(uint2));
-    reloc_.chunk_cap = (uint32_t)cc;
+  const size_t dirs = has_in_ ? 2 : 1;
+  for (size_t l = 0; l < 4; l++)
+    lists_.rec[l] = l % 2 < dirs ? (Rec *)al(c * sizeof(Rec)) : nullptr;
+  if (c > INGEST_BLOCK_MAX) {  // the device-wide sort of all lists
+    const size_t all = 2 * dirs * c;
+    keys_ = (u64 *)al(all * 8);
+    keys_sorted_ = (u64 *)al(all * 8);
+    if (stored_) {
+      w_ = (uint32_t *)al(all * 4);
+      w_sorted_ = (uint32_t *)al(all * 4);
+    }
+    sort_bytes_ = ingest_temp_bytes(all);
+    sort_temp_ = al(sort_bytes_);
   }
-  reloc_.n_reloc = counts_ + 8;
-  reloc_.n_chunks = counts_ + 9;
-  tombs_.pos = (u64 *)al(c * 8);
-  tombs_.count = counts_ + 10;
-  tombs_.cap = (uint32_t)c;
-  defer_.on = true;
-  defer_.rem = (uint32_t *)al(c * 4);
-  defer_.row_u = (uint32_t *)al(c * 4);
-  defer_.row_base = (u64 *)al(c * 8);
-  defer_.packed = (u64 *)(counts_ + 12);  // 8-byte aligned slot of the counters
-  defer_.cap_rows = (uint32_t)c;
-  d_edges_ = (dycg_edge_dev *)al(c * 2 * sizeof(dycg_edge_dev));
-  runs_.flags = (uint32_t *)al(c * 4);
-  runs_.pos = (uint32_t *)al(c * 4);
-  runs_.start = (uint32_t *)al(c * 4);
-  runs_.valid = counts_ + 14;
-  size_t a = 0, b = 0;
-  CK(sort_keys(nullptr, a, k_tmp_out_, k_del_out_, (uint32_t)c, st_));
-  CK(sort_pairs(nullptr, b, k_tmp_out_, k_add_out_, w_tmp_, w_add_out_, (uint32_t)c, st_));
-  cub_bytes_ = std::max(std::max(a, b), unique_runs_temp_bytes((uint32_t)c));
-  cub_temp_ = al(cub_bytes_);
-  runs_.temp = cub_temp_;  // used between the sorts, on the same stream
-  runs_.temp_bytes = cub_bytes_;
-  if (h_stage_) {
-    cudaFreeHost(h_stage_);
-    hallocs_.erase(std::find(hallocs_.begin(), hallocs_.end(), (void *)h_stage_));
+  found_ = (uint32_t *)al(c * 4);
+  touched_ = (uint32_t *)al(c * 2 * 4);
+  const u64 slots = out_.slots + (has_in_ ? in_.slots : 0);
+  reloc_.rec = (RelocRec *)al(dirs * c * sizeof(RelocRec));
+  reloc_.cap = (uint32_t)(dirs * c);
+  const u64 cc = std::min<u64>(slots / RELOC_CHUNK + dirs * c + 1024, 0x7FFFFFFFull);
+  reloc_.chunks = (uint2 *)al(cc * sizeof(uint2));
+  reloc_.chunk_cap = (uint32_t)cc;
+  // whole chunks of the deferred suffixes, and one part chunk per row
+  suffix_cap_ = (uint32_t)std::min<u64>(slots / SUFFIX_CHUNK + dirs * c + 16, 0x7FFFFFFFull);
+  suffix_ = (uint4 *)al((u64)suffix_cap_ * sizeof(uint4));
+  suffix_ids_ = (uint32_t *)al((u64)std::min(suffix_cap_, SUFFIX_KEEP) * SUFFIX_CHUNK * 4);
+  for (size_t d = 0; d < dirs; d++) {
+    rem_[d] = (uint32_t *)al(c * 4);
+    matches_[d] = (uint32_t *)al(c * 4);
+  }
+  const size_t stage = sizeof(BatchHdr) + c * 2 * sizeof(dycg_edge);
+  d_hdr_ = (BatchHdr *)al(stage);
+  d_edges_ = (dycg_edge_dev *)(d_hdr_ + 1);
+  if (h_hdr_) {
+    cudaFreeHost(h_hdr_);
+    hallocs_.erase(std::find(hallocs_.begin(), hallocs_.end(), (void *)h_hdr_));
+    h_hdr_ = nullptr;
   }
   void *hs = nullptr;
-  CK(cudaHostAlloc(&hs, c * 2 * sizeof(dycg_edge), cudaHostAllocDefault));
+  CK(cudaHostAlloc(&hs, stage, cudaHostAllocDefault));
   hallocs_.push_back(hs);
-  h_stage_ = (dycg_edge *)hs;
+  h_hdr_ = (BatchHdr *)hs;
   bcap_ = c;
 }
 
-// Deletions of one adjacency direction. Rows with a long unsorted suffix are
-// matched by sort-merge; that needs the gathered size on the host (one
-// synchronisation), so a captured graph keeps the per-record scan.
-void Engine::delete_direction(const Adj &A, const uint2 *uv, const uint32_t *mult,
-                              const uint32_t *n_ptr, uint32_t nd, uint32_t *found,
-                              int count_missing, bool capture) {
-  if (capture) {
-    CK(launch_delete_rows(A, uv, mult, n_ptr, nd, found, ctl_, count_missing, tombs_, mut_ctas_,
-                          st_));
-    launches_ += 2;
-    return;
-  }
-  CK(launch_delete_prefix(A, uv, mult, n_ptr, nd, found, ctl_, count_missing, tombs_, defer_,
-                          mut_ctas_, st_));
-  CK(cudaMemcpyAsync(h_dpacked_, defer_.packed, 8, cudaMemcpyDeviceToHost, st_));
-  sync_check("deferred deletions");
-  const u64 pk = *h_dpacked_;
-  const uint32_t nrows = (uint32_t)(pk >> 40);
-  const u64 total = pk & ((1ull << 40) - 1);
-  if (total > dbuf_cap_) ensure_defer(total);
-  CK(launch_delete_suffix(A, uv, n_ptr, nd, found, ctl_, count_missing, tombs_, defer_, nrows,
-                          total, dbufs_, st_));
-  launches_ += 2 + (nrows ? 7 : 0);
-}
-
-// Sort buffers of the deferred deletions, for at least `slots` suffix slots.
-// They grow geometrically (at least doubling), and reserve_batch sizes them
-// ahead, because an allocation between a snapshot's stage events leaves the
-// GPU idle for as long as the driver takes (hundreds of ms when another
-// process holds the driver's locks, e.g. a monitoring query).
-void Engine::ensure_defer(u64 slots) {
-  if (slots <= dbuf_cap_) return;
-  CK(cudaStreamSynchronize(st_));
-  for (void *p : {(void *)dbufs_.k_in, (void *)dbufs_.k_out, (void *)dbufs_.v_in,
-                  (void *)dbufs_.v_out, dbufs_.temp})
-    cudaFree(p);
-  dbufs_ = DeferBufs{};
-  const u64 c = std::max<u64>({slots + slots / 2, dbuf_cap_ * 2, 1ull << 20});
-  dbuf_cap_ = 0;
-  CK(cudaMalloc((void **)&dbufs_.k_in, c * 8));
-  CK(cudaMalloc((void **)&dbufs_.k_out, c * 8));
-  CK(cudaMalloc((void **)&dbufs_.v_in, c * 4));
-  CK(cudaMalloc((void **)&dbufs_.v_out, c * 4));
-  dbufs_.temp_bytes = delete_sort_temp_bytes(c);
-  CK(cudaMalloc(&dbufs_.temp, std::max<size_t>(dbufs_.temp_bytes, 16)));
-  dbuf_cap_ = c;
-}
-
 // Device half of a snapshot on st_: counters reset, ingest, mutation and
-// repair, no host synchronisation. capture: being recorded into a CUDA graph
-// (no stage events, no touched-source pass).
-void Engine::enqueue_snapshot(const dycg_edge_dev *d_dels, size_t nd, const dycg_edge_dev *d_adds,
-                              size_t na, bool capture) {
-  CK(cudaMemsetAsync(ctl_, 0, sizeof(Ctl), st_));
-  CK(cudaMemsetAsync(counts_, 0, 64, st_));
-  if (opt_.algo == DYCG_ALGO_PR) {
-    // carried frontier length
+// repair of the batch d_hdr_ names, no host synchronisation. nd, na: its
+// records, or with capture (being recorded into a CUDA graph: no stage events,
+// no touched-source pass) the most a batch of the class has.
+void Engine::enqueue_snapshot(size_t nd, size_t na, bool capture) {
+  CK(cudaMemsetAsync(ctl_, 0, CTL_CLEAR, st_));
+  launches_++;
+  if (opt_.algo == DYCG_ALGO_PR && pr_count_ && !(nd + na)) {
+    // carried frontier length (with records, the ingest stores it)
     h_ctl_->q_count[pr_cur_] = pr_count_;
     CK(cudaMemcpyAsync(&ctl_->q_count[pr_cur_], &h_ctl_->q_count[pr_cur_], 4,
                        cudaMemcpyHostToDevice, st_));
+    launches_++;
   }
-  launches_ += 2;
   // ---- ingest
-  u64 *invalid = &ctl_->stat[ST_INVALID];
-  size_t tb = cub_bytes_;
-  if (nd) {
-    CK(launch_prep_keys(d_dels, (uint32_t)nd, n_, k_tmp_out_, has_in_ ? k_tmp_in_ : nullptr,
-                        nullptr, invalid, st_));
-    CK(sort_keys(cub_temp_, tb, k_tmp_out_, k_del_out_, (uint32_t)nd, st_));
-    CK(launch_unique_runs(k_del_out_, (uint32_t)nd, uv_out_, mult_out_, counts_ + 0,
-                          (uint32_t)bcap_, &ctl_->err, runs_, st_));
-    launches_ += 5;
-    if (has_in_) {
-      tb = cub_bytes_;
-      CK(sort_keys(cub_temp_, tb, k_tmp_in_, k_del_in_, (uint32_t)nd, st_));
-      CK(launch_unique_runs(k_del_in_, (uint32_t)nd, uv_in_, mult_in_, counts_ + 1,
-                            (uint32_t)bcap_, &ctl_->err, runs_, st_));
-      launches_ += 4;
-    }
-  }
-  if (na) {
-    tb = cub_bytes_;
-    CK(launch_prep_keys(d_adds, (uint32_t)na, n_, k_tmp_out_, has_in_ ? k_tmp_in_ : nullptr,
-                        w_tmp_, invalid, st_));
-    CK(sort_pairs(cub_temp_, tb, k_tmp_out_, k_add_out_, w_tmp_, w_add_out_, (uint32_t)na, st_));
-    CK(launch_row_segments(k_add_out_, (uint32_t)na, seg_out_, counts_ + 2, (uint32_t)bcap_,
-                           &ctl_->err, runs_, st_));
-    CK(launch_keys_to_uvw(k_add_out_, w_add_out_, (uint32_t)na, add_uvw_, st_));
-    launches_ += 4;
-    if (has_in_) {
-      tb = cub_bytes_;
-      CK(sort_pairs(cub_temp_, tb, k_tmp_in_, k_add_in_, w_tmp_, w_add_in_, (uint32_t)na, st_));
-      CK(launch_row_segments(k_add_in_, (uint32_t)na, seg_in_, counts_ + 3, (uint32_t)bcap_,
-                             &ctl_->err, runs_, st_));
-      launches_ += 2;
-    }
+  IngestLaunch I{};
+  I.hdr = d_hdr_;
+  I.lists = lists_;
+  I.nd = (uint32_t)nd;
+  I.na = (uint32_t)na;
+  I.n = n_;
+  I.has_in = has_in_;
+  I.with_w = stored_;
+  I.keys = keys_;
+  I.keys_sorted = keys_sorted_;
+  I.w = w_;
+  I.w_sorted = w_sorted_;
+  I.temp = sort_temp_;
+  I.temp_bytes = sort_bytes_;
+  I.ctl = ctl_;
+  if (opt_.algo == DYCG_ALGO_PR) {
+    I.carry_q = pr_cur_;
+    I.carry = pr_count_;
   }
   // distinct touched sources (PR amends and the touched_sources counter);
   // a captured graph would replay one epoch, so replays leave it out
-  if (!capture) {
-    ++touch_epoch_;
-    if (nd) CK(launch_touched(k_del_out_, (uint32_t)nd, touch_, touch_epoch_, touched_, counts_ + 4,
-                              ctl_, st_));
-    if (na) CK(launch_touched(k_add_out_, (uint32_t)na, touch_, touch_epoch_, touched_, counts_ + 4,
-                              ctl_, st_));
-    launches_ += (nd ? 1 : 0) + (na ? 1 : 0);
-  }
+  if (!capture)
+    I.touch = Touch{touch_, ++touch_epoch_, touched_, counts_, out_.live,
+                    opt_.algo == DYCG_ALGO_PR ? delta_ : nullptr};
+  uint32_t launched = 0;
+  CK(launch_ingest(I, &launched, st_));
+  launches_ += launched;
   if (!capture) CK(cudaEventRecord(ev_[1], st_));
   // the previous call's page staging (side stream) ends before this snapshot
   // reads or writes adjacency (a capture begins only after a join)
@@ -809,45 +724,49 @@ void Engine::enqueue_snapshot(const dycg_edge_dev *d_dels, size_t nd, const dycg
     PL.q0 = q0_;
     PL.q1 = q1_;
     PL.sources = touched_;
-    PL.n_sources = counts_ + 4;
+    PL.n_sources = counts_;
     PL.tiles = tiles_;
     PL.tile_cap = tile_cap_;
     PL.ctl = ctl_;
     PL.n = n_;
     PL.cur = pr_cur_;
-    PL.del_uv = uv_out_;
-    PL.del_found = found_out_;
-    PL.n_del = counts_ + 0;
-    PL.add_uvw = add_uvw_;
-    PL.n_add = (uint32_t)na;
+    PL.hdr = d_hdr_;
+    PL.dels = lists_.rec[0];
+    PL.del_found = found_;
+    PL.adds = lists_.rec[2];
     PL.eps = opt_.epsilon;
     PL.alpha = opt_.alpha;
     PL.max_rounds = opt_.max_rounds;
     PL.timeout_ns = timeout;
     PL.num_sms = num_sms_;
-    // the amend after the mutation needs each touched source's old degree
-    if (nd + na) {
-      CK(launch_pr_old_degree(touched_, counts_ + 4, (uint32_t)(nd + na), out_.live, delta_, st_));
-      launches_++;
-    }
   }
   // ---- mutation
   const Adj A_out = adj(out_);
   const Adj A_in = has_in_ ? adj(in_) : A_out;
-  if (nd) {
-    delete_direction(A_out, uv_out_, mult_out_, counts_ + 0, (uint32_t)nd, found_out_, 1, capture);
-    if (has_in_)
-      delete_direction(A_in, uv_in_, mult_in_, counts_ + 1, (uint32_t)nd, nullptr, 0, capture);
-  }
-  if (na) {
-    CK(launch_add_rows(A_out, k_add_out_, w_add_out_, seg_out_, counts_ + 2, (uint32_t)na,
-                       reloc_, ctl_, mut_ctas_, st_));
-    launches_ += 3;
-    if (has_in_) {
-      CK(launch_add_rows(A_in, k_add_in_, w_add_in_, seg_in_, counts_ + 3, (uint32_t)na, reloc_,
-                         ctl_, mut_ctas_, st_));
-      launches_ += 3;
+  if (nd + na) {
+    MutParams M{};
+    M.adj[0] = A_out;
+    M.adj[1] = A_in;
+    M.dirs = has_in_ ? 2 : 1;
+    M.deletions = nd != 0;
+    M.insertions = na != 0;
+    M.hdr = d_hdr_;
+    for (int d = 0; d < 2; d++) {
+      M.dels[d] = lists_.rec[d];
+      M.adds[d] = lists_.rec[2 + d];
+      M.rem[d] = rem_[d];
+      M.matches[d] = matches_[d];
     }
+    M.found = found_;
+    M.suffix = suffix_;
+    M.suffix_cap = suffix_cap_;
+    M.suffix_ids = suffix_ids_;
+    M.reloc = reloc_;
+    M.ctl = ctl_;
+    M.mctl = mctl_;
+    M.timeout_ns = timeout;
+    CK(launch_mutate(M, (uint32_t)std::max(nd, na), mut_ctas_, st_));
+    launches_++;
   }
   if (!capture) CK(cudaEventRecord(ev_[2], st_));
   // learned admission / trace features, between mutation and repair: rows
@@ -860,8 +779,9 @@ void Engine::enqueue_snapshot(const dycg_edge_dev *d_dels, size_t nd, const dycg
     CK(launch_pr(PL, st_));
     launches_++;
   } else if (nq_) {
-    if (tune_) tune_repair((uint32_t)nd, (uint32_t)na, timeout);
-    else repair_queries((uint32_t)nd, (uint32_t)na, timeout);
+    const uint32_t phases = (nd ? PH_DELETE : 0) | (na ? PH_INSERT : 0) | PH_CLOSE;
+    if (tune_) tune_repair(phases, timeout);
+    else repair_queries(phases, timeout);
   } else {
     RepairLaunch L{};
     L.out = A_out;
@@ -875,11 +795,10 @@ void Engine::enqueue_snapshot(const dycg_edge_dev *d_dels, size_t nd, const dycg
     L.tiles = tiles_;
     L.tile_cap = tile_cap_;
     L.ctl = ctl_;
-    L.del_uv = uv_out_;
-    L.del_found = found_out_;
-    L.n_del_ptr = counts_ + 0;
-    L.add_uvw = add_uvw_;
-    L.n_add = (uint32_t)na;
+    L.hdr = d_hdr_;
+    L.dels = lists_.rec[0];
+    L.del_found = found_;
+    L.adds = lists_.rec[2];
     L.n = n_;
     L.source = opt_.source;
     L.epoch = ++epoch_;
@@ -912,18 +831,20 @@ void Engine::apply(const dycg_edge *dels, size_t nd, const dycg_edge *adds, size
   ensure_batch(std::max<size_t>(std::max(nd, na), 1));
   const uint64_t l0 = launches_;
   CK(cudaEventRecord(ev_[0], st_));
-  const dycg_edge_dev *d_dels = (const dycg_edge_dev *)dels;
-  const dycg_edge_dev *d_adds = (const dycg_edge_dev *)adds;
+  // the batch header and, from host arrays, its records behind it: one copy
+  *h_hdr_ = BatchHdr{(const dycg_edge_dev *)dels, (const dycg_edge_dev *)adds, (uint32_t)nd,
+                     (uint32_t)na, {0, 0}};
+  size_t bytes = sizeof(BatchHdr);
   if (!device_ptrs) {
-    if (nd) std::memcpy(h_stage_, dels, nd * sizeof(dycg_edge));
-    if (na) std::memcpy(h_stage_ + nd, adds, na * sizeof(dycg_edge));
-    if (nd + na)
-      CK(cudaMemcpyAsync(d_edges_, h_stage_, (nd + na) * sizeof(dycg_edge),
-                         cudaMemcpyHostToDevice, st_));
-    d_dels = d_edges_;
-    d_adds = d_edges_ + nd;
+    dycg_edge *h = (dycg_edge *)(h_hdr_ + 1);
+    if (nd) std::memcpy(h, dels, nd * sizeof(dycg_edge));
+    if (na) std::memcpy(h + nd, adds, na * sizeof(dycg_edge));
+    h_hdr_->dels = d_edges_;
+    h_hdr_->adds = d_edges_ + nd;
+    bytes += (nd + na) * sizeof(dycg_edge);
   }
-  enqueue_snapshot(d_dels, nd, d_adds, na, false);
+  CK(cudaMemcpyAsync(d_hdr_, h_hdr_, bytes, cudaMemcpyHostToDevice, st_));
+  enqueue_snapshot(nd, na, false);
   CK(cudaMemcpyAsync(h_ctl_, ctl_, sizeof(Ctl), cudaMemcpyDeviceToHost, st_));
   if (nq_) {
     if (qmode_ == DYCG_QUERIES_PER_QUERY)
@@ -1113,7 +1034,7 @@ void Engine::set_query_queue(uint32_t scheme) {
   drop_graphs();  // captured graphs hold the old scheme
 }
 
-MultiLaunch Engine::multi_launch(uint32_t phases, uint32_t n_add, u64 timeout) {
+MultiLaunch Engine::multi_launch(uint32_t phases, u64 timeout) {
   MultiLaunch L{};
   L.out = adj(out_);
   L.in = has_in_ ? adj(in_) : L.out;
@@ -1133,11 +1054,10 @@ MultiLaunch Engine::multi_launch(uint32_t phases, uint32_t n_add, u64 timeout) {
   L.tile_cap = mtile_cap_;
   L.ctl = ctl_;
   L.seq = seq_;
-  L.del_uv = uv_out_;
-  L.del_found = found_out_;
-  L.n_del_ptr = counts_;
-  L.add_uvw = add_uvw_;
-  L.n_add = n_add;
+  L.hdr = d_hdr_;
+  L.dels = lists_.rec[0];
+  L.del_found = found_;
+  L.adds = lists_.rec[2];
   L.n = n_;
   L.nb = qnb_;
   L.phases = phases;
@@ -1174,7 +1094,7 @@ void Engine::init_queries(u64 timeout) {
   if (qmode_ == DYCG_QUERIES_BATCHED) {
     CK(launch_multi_init(qkey_, n_, qnb_, d_sources_, nmask_[0], q0_, wtag_, seq_, ctl_, sched_,
                          st_));
-    CK(launch_multi(multi_launch(PH_CLOSE, 0, timeout), st_));
+    CK(launch_multi(multi_launch(PH_CLOSE, timeout), st_));
     launches_ += 3;
     CK(cudaMemcpyAsync(h_ctl_, ctl_, sizeof(Ctl), cudaMemcpyDeviceToHost, st_));
     sync_check("init queries");
@@ -1228,10 +1148,9 @@ void Engine::init_queries(u64 timeout) {
 }
 
 // Repair of every query after the snapshot's mutation (asynchronous).
-void Engine::repair_queries(uint32_t nd, uint32_t na, u64 timeout) {
-  const uint32_t phases = (nd ? PH_DELETE : 0) | (na ? PH_INSERT : 0) | PH_CLOSE;
+void Engine::repair_queries(uint32_t phases, u64 timeout) {
   if (qmode_ == DYCG_QUERIES_BATCHED) {
-    CK(launch_multi(multi_launch(phases, na, timeout), st_));
+    CK(launch_multi(multi_launch(phases, timeout), st_));
     launches_++;
     return;
   }
@@ -1249,11 +1168,10 @@ void Engine::repair_queries(uint32_t nd, uint32_t na, u64 timeout) {
     L.tiles = tiles_;
     L.tile_cap = tile_cap_;
     L.ctl = qctl_ + q;
-    L.del_uv = uv_out_;
-    L.del_found = found_out_;
-    L.n_del_ptr = counts_;
-    L.add_uvw = add_uvw_;
-    L.n_add = na;
+    L.hdr = d_hdr_;
+    L.dels = lists_.rec[0];
+    L.del_found = found_;
+    L.adds = lists_.rec[2];
     L.n = n_;
     L.epoch = ++epoch_;
     L.phases = phases;
@@ -1290,12 +1208,11 @@ void Engine::gather_query(uint32_t q, uint32_t *values, uint32_t *parents) {
 // same saved state (keys, page hotness, counters); keeps the fastest mapping
 // and ends with that mapping's run, so the engine state and the stage events
 // describe one ordinary repair.
-void Engine::tune_repair(uint32_t nd, uint32_t na, u64 timeout) {
+void Engine::tune_repair(uint32_t phases, u64 timeout) {
   if (qmode_ != DYCG_QUERIES_BATCHED) {
-    repair_queries(nd, na, timeout);
+    repair_queries(phases, timeout);
     return;
   }
-  const uint32_t phases = (nd ? PH_DELETE : 0) | (na ? PH_INSERT : 0) | PH_CLOSE;
   const u64 kbytes = (u64)n_ * qnb_ * 32 * 8, hbytes = (u64)npages_ * 4;
   struct Scratch {
     void *p[3] = {nullptr, nullptr, nullptr};
@@ -1334,7 +1251,7 @@ void Engine::tune_repair(uint32_t nd, uint32_t na, u64 timeout) {
     tile_ = t;
     sched_ = q;
     CK(cudaEventRecord(sc.a, st_));
-    CK(launch_multi(multi_launch(phases, na, timeout), st_));
+    CK(launch_multi(multi_launch(phases, timeout), st_));
     CK(cudaEventRecord(sc.b, st_));
     CK(cudaMemcpyAsync(h_ctl_, ctl_, sizeof(Ctl), cudaMemcpyDeviceToHost, st_));
     sync_check("tune");
@@ -1373,7 +1290,7 @@ void Engine::tune_repair(uint32_t nd, uint32_t na, u64 timeout) {
   sched_ = best.queue;
   drop_graphs();
   CK(cudaEventRecord(ev_[2], st_));  // the stage boundary of the kept run
-  CK(launch_multi(multi_launch(phases, na, timeout), st_));
+  CK(launch_multi(multi_launch(phases, timeout), st_));
   launches_++;
   sync_check("tune final");  // scratch is released on return
 }
@@ -1400,8 +1317,8 @@ void Engine::drop_graphs() {
   graphs_.clear();
 }
 
-// Graph of one snapshot of padded size cls (records at d_edges_: deletions
-// [0, cls), insertions [cls, 2 cls)), captured on first use.
+// Graph of one snapshot of up to cls deletions and as many insertions (the
+// batch d_hdr_ names when it runs), captured on first use.
 const Engine::SnapshotGraph &Engine::graph_for(uint32_t cls) {
   auto it = graphs_.find(cls);
   if (it != graphs_.end()) return it->second;
@@ -1410,7 +1327,7 @@ const Engine::SnapshotGraph &Engine::graph_for(uint32_t cls) {
   const uint64_t l0 = launches_;
   CK(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal));
   try {
-    enqueue_snapshot(d_edges_, cls, d_edges_ + cls, cls, true);
+    enqueue_snapshot(cls, cls, true);
   } catch (...) {
     cudaStreamEndCapture(st_, &g);
     if (g) cudaGraphDestroy(g);
@@ -1483,8 +1400,11 @@ void Engine::apply_batches(const dycg_edge *dels, const uint64_t *nd, const dycg
   if (count > bctl_cap_) {
     if (h_bctl_) cudaFreeHost(h_bctl_);
     h_bctl_ = nullptr;
+    h_bhdr_ = nullptr;
     bctl_cap_ = 0;
-    CK(cudaHostAlloc((void **)&h_bctl_, (u64)count * sizeof(Ctl), cudaHostAllocDefault));
+    CK(cudaHostAlloc((void **)&h_bctl_, (u64)count * (sizeof(Ctl) + sizeof(BatchHdr)),
+                     cudaHostAllocDefault));
+    h_bhdr_ = (BatchHdr *)(h_bctl_ + count);
     bctl_cap_ = count;
   }
   while (bev_.size() < 2 * (size_t)count) {
@@ -1497,14 +1417,9 @@ void Engine::apply_batches(const dycg_edge *dels, const uint64_t *nd, const dycg
   for (uint32_t i = 0; i < count; i++) {
     cls[i] = cls_of(std::max<u64>(std::max(nd[i], na[i]), 1));
     const SnapshotGraph &g = graph_for(cls[i]);
-    // padding records carry out-of-range ids: ingest drops them
-    CK(cudaMemsetAsync(d_edges_, 0xFF, 2ull * cls[i] * sizeof(dycg_edge), st_));
-    if (nd[i])
-      CK(cudaMemcpyAsync(d_edges_, d_dels + od, nd[i] * sizeof(dycg_edge),
-                         cudaMemcpyDeviceToDevice, st_));
-    if (na[i])
-      CK(cudaMemcpyAsync(d_edges_ + cls[i], d_adds + oa, na[i] * sizeof(dycg_edge),
-                         cudaMemcpyDeviceToDevice, st_));
+    // the class's graph reads the batch where it lies and takes its own counts
+    h_bhdr_[i] = BatchHdr{d_dels + od, d_adds + oa, (uint32_t)nd[i], (uint32_t)na[i], {0, 0}};
+    CK(cudaMemcpyAsync(d_hdr_, h_bhdr_ + i, sizeof(BatchHdr), cudaMemcpyHostToDevice, st_));
     CK(cudaEventRecord(bev_[2 * i], st_));
     CK(cudaGraphLaunch(g.exec, st_));
     CK(cudaEventRecord(bev_[2 * i + 1], st_));
@@ -1537,8 +1452,7 @@ void Engine::apply_batches(const dycg_edge *dels, const uint64_t *nd, const dycg
       s->deletions = nd[i];
       s->insertions = na[i];
       s->missing_deletes = c.stat[ST_MISSING];
-      // padding records count as invalid in the device counter
-      s->invalid_updates = c.stat[ST_INVALID] - (2ull * cls[i] - nd[i] - na[i]);
+      s->invalid_updates = c.stat[ST_INVALID];
       s->relocated_rows = c.stat[ST_RELOCATED];
       s->affected = c.stat[ST_AFFECTED];
       s->expanded = c.stat[ST_EXPANDED];
@@ -1659,19 +1573,12 @@ void Engine::policy_prefetch(size_t nd, size_t na, bool capture) {
     CK(launch_page_rows(in_.off, in_.len, n_, in_.page_base, page_shift_, prows_, pmax_, pperiod_,
                         st_));
   CK(launch_period_step(pperiod_, st_));
-  if (nd) {
-    CK(launch_page_delta(k_del_out_, (uint32_t)nd, out_.off, out_.page_base, page_shift_, pdelta_,
-                         st_));
-    if (has_in_)
-      CK(launch_page_delta(k_del_in_, (uint32_t)nd, in_.off, in_.page_base, page_shift_, pdelta_,
-                           st_));
-  }
-  if (na) {
-    CK(launch_page_delta(k_add_out_, (uint32_t)na, out_.off, out_.page_base, page_shift_, pdelta_,
-                         st_));
-    if (has_in_)
-      CK(launch_page_delta(k_add_in_, (uint32_t)na, in_.off, in_.page_base, page_shift_, pdelta_,
-                           st_));
+  for (uint32_t l = 0; l < 4; l++) {
+    const Arena &A = l % 2 ? in_ : out_;
+    const size_t cap = l < 2 ? nd : na;
+    if (cap && lists_.rec[l])
+      CK(launch_page_delta(lists_.rec[l], d_hdr_, l >= 2, (uint32_t)cap, A.off, A.page_base,
+                           page_shift_, pdelta_, st_));
   }
   CK(launch_features(page_hits_, hist_, age_, pdelta_, prows_, pmax_, npages_, feat_, st_));
   launches_ += 5 + (has_in_ ? 1 : 0) + (nd ? 1 : 0) * (has_in_ ? 2 : 1) +

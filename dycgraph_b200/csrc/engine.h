@@ -103,9 +103,8 @@ class Engine {
   Adj adj(const Arena &A) const;
   void sync_check(const char *where);
   void fill_stats(dycg_batch_stats *s, float ms[4]);
-  void enqueue_snapshot(const dycg_edge_dev *d_dels, size_t nd, const dycg_edge_dev *d_adds,
-                        size_t na, bool capture);
-  void tune_repair(uint32_t nd, uint32_t na, u64 timeout);
+  void enqueue_snapshot(size_t nd, size_t na, bool capture);
+  void tune_repair(uint32_t phases, u64 timeout);
   struct SnapshotGraph {
     cudaGraphExec_t exec;
     uint64_t kernels;
@@ -113,16 +112,13 @@ class Engine {
   const SnapshotGraph &graph_for(uint32_t cls);
   void drop_graphs();
   void policy_alloc();
-  void delete_direction(const Adj &A, const uint2 *uv, const uint32_t *mult,
-                        const uint32_t *n_ptr, uint32_t nd, uint32_t *found, int count_missing,
-                        bool capture);
   void policy_prefetch(size_t nd, size_t na, bool capture);
   void hotness_round(bool initial, bool side = false);
   void join_staging();
   void maintenance_device();
   void init_queries(u64 timeout);
-  void repair_queries(uint32_t nd, uint32_t na, u64 timeout);
-  MultiLaunch multi_launch(uint32_t phases, uint32_t n_add, u64 timeout);
+  void repair_queries(uint32_t phases, u64 timeout);
+  MultiLaunch multi_launch(uint32_t phases, u64 timeout);
   void *dmalloc(size_t bytes);
   void dfree_all();
 
@@ -155,7 +151,7 @@ class Engine {
            *touch_ = nullptr;
   uint4 *tiles_ = nullptr;
   uint32_t tile_cap_ = 0;
-  Ctl *ctl_ = nullptr, *h_ctl_ = nullptr;
+  Ctl *ctl_ = nullptr, *mctl_ = nullptr, *h_ctl_ = nullptr;
   float *x_ = nullptr, *r_ = nullptr, *delta_ = nullptr;
   uint32_t *queued_ = nullptr;
   uint32_t pr_cur_ = 0, pr_count_ = 0;
@@ -184,6 +180,7 @@ class Engine {
   std::map<uint32_t, SnapshotGraph> graphs_;
   std::vector<cudaEvent_t> bev_;
   Ctl *h_bctl_ = nullptr;
+  BatchHdr *h_bhdr_ = nullptr;  // behind h_bctl_
   uint32_t bctl_cap_ = 0;
   void *h_rec_ = nullptr, *d_rec_ = nullptr;
   u64 hrec_bytes_ = 0;
@@ -208,25 +205,18 @@ class Engine {
 
   // batch buffers
   size_t bcap_ = 0;
-  u64 *k_tmp_out_ = nullptr, *k_tmp_in_ = nullptr, *k_del_out_ = nullptr, *k_del_in_ = nullptr,
-      *k_add_out_ = nullptr, *k_add_in_ = nullptr;
-  uint32_t *w_tmp_ = nullptr, *w_add_out_ = nullptr, *w_add_in_ = nullptr;
-  uint2 *uv_out_ = nullptr, *uv_in_ = nullptr;
-  uint32_t *mult_out_ = nullptr, *mult_in_ = nullptr, *found_out_ = nullptr;
-  uint3 *seg_out_ = nullptr, *seg_in_ = nullptr, *add_uvw_ = nullptr;
-  uint32_t *touched_ = nullptr, *counts_ = nullptr;
-  RunScratch runs_{};  // run finder scratch (unique deletions, row segments)
+  Lists lists_{};  // ingested record lists (ingest.cu)
+  u64 *keys_ = nullptr, *keys_sorted_ = nullptr;  // device-wide sort of large batches
+  uint32_t *w_ = nullptr, *w_sorted_ = nullptr;
+  void *sort_temp_ = nullptr;
+  size_t sort_bytes_ = 0;
+  uint32_t *found_ = nullptr, *touched_ = nullptr, *counts_ = nullptr;
   Reloc reloc_{};
-  Tombs tombs_{};
-  DeferDel defer_{};
-  void ensure_defer(u64 slots);
-  DeferBufs dbufs_{};
-  u64 dbuf_cap_ = 0;
-  u64 *h_dpacked_ = nullptr;  // pinned
+  uint4 *suffix_ = nullptr;  // long-suffix deletions (mutate.cu)
+  uint32_t suffix_cap_ = 0, *suffix_ids_ = nullptr;
+  uint32_t *rem_[2] = {}, *matches_[2] = {};
+  BatchHdr *d_hdr_ = nullptr, *h_hdr_ = nullptr;  // header, records behind it
   dycg_edge_dev *d_edges_ = nullptr;
-  dycg_edge *h_stage_ = nullptr;
-  void *cub_temp_ = nullptr;
-  size_t cub_bytes_ = 0;
   std::vector<void *> batch_allocs_;
   uint64_t launches_ = 0;
 };

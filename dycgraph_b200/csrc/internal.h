@@ -13,6 +13,21 @@ struct dycg_edge_dev {
   uint32_t u, v, w;
 };
 
+// One snapshot's records as the device sees them (written by the host ahead of
+// the snapshot's kernels, so a captured snapshot serves any batch of its class).
+struct BatchHdr {
+  const dycg_edge_dev *dels, *adds;
+  uint32_t nd, na;
+  uint32_t pad[2];
+};
+
+// Entry of an ingested record list (ingest.cu): row, neighbour, weight
+// (insertions) or the row's records from this one on (deletions, at run heads),
+// and at the first entry of a run its length, else 0 -- equal (row, neighbour)
+// for deletions, equal row for insertions. Row INF32: a record with an endpoint
+// out of range (sorted last).
+typedef uint4 Rec;
+
 constexpr uint32_t PH_DELETE = 1, PH_INSERT = 2, PH_CLOSE = 4;
 constexpr uint32_t PR_AMEND = 1, PR_CONVERGE = 2;
 
@@ -23,11 +38,10 @@ struct RepairLaunch {
   uint4 *tiles;
   uint32_t tile_cap;
   Ctl *ctl;
-  const uint2 *del_uv;
+  const BatchHdr *hdr;
+  const Rec *dels;            // by source; del_found: occurrences removed, at run heads
   const uint32_t *del_found;
-  const uint32_t *n_del_ptr;
-  const uint3 *add_uvw;
-  uint32_t n_add;
+  const Rec *adds;
   uint32_t n, source, epoch, tag_base, phases, max_waves;
   uint32_t delta;  // ordered closure bucket width (0: unordered)
   uint32_t *tag_dev;  // optional device wave-tag counter (replaces tag_base)
@@ -53,11 +67,10 @@ struct MultiLaunch {
   uint32_t tile_cap;
   Ctl *ctl;
   uint32_t *seq;                // device {epoch, next wave tag}, advanced by each launch
-  const uint2 *del_uv;
+  const BatchHdr *hdr;
+  const Rec *dels;
   const uint32_t *del_found;
-  const uint32_t *n_del_ptr;
-  const uint3 *add_uvw;
-  uint32_t n_add;
+  const Rec *adds;
   uint32_t n, nb, phases, max_waves;
   uint32_t qratio;              // query lanes when 4*active >= qratio*min(len,32)
   uint32_t pull_qratio;         // the same rule for the pull phase
@@ -89,10 +102,10 @@ struct PrLaunch {
   float *x, *r, *delta;
   uint32_t *queued, *q0, *q1;
   const uint32_t *sources, *n_sources;  // touched sources
-  const uint2 *del_uv;                   // distinct deleted pairs, occurrences found
-  const uint32_t *del_found, *n_del;
-  const uint3 *add_uvw;                  // inserted occurrences
-  uint32_t n_add;
+  const BatchHdr *hdr;
+  const Rec *dels;                       // deleted pairs, occurrences found at run heads
+  const uint32_t *del_found;
+  const Rec *adds;                       // inserted occurrences
   uint4 *tiles;
   uint32_t tile_cap;
   Ctl *ctl;
@@ -103,93 +116,80 @@ struct PrLaunch {
   int num_sms;
 };
 cudaError_t launch_pr(const PrLaunch &L, cudaStream_t s);
-cudaError_t launch_pr_old_degree(const uint32_t *sources, const uint32_t *n_sources,
-                                 uint32_t max_sources, const uint32_t *live, float *delta,
-                                 cudaStream_t s);
 cudaError_t launch_pr_init(float *x, float *r, uint32_t *queued, uint32_t *q0, uint32_t n,
                            float base, Ctl *ctl, cudaStream_t s);
 
-// ingest + mutation
-cudaError_t launch_prep_keys(const dycg_edge_dev *e, uint32_t cnt, uint32_t n, u64 *kout,
-                             u64 *kin, uint32_t *w, u64 *invalid, cudaStream_t s);
-cudaError_t sort_keys(void *temp, size_t &temp_bytes, const u64 *in, u64 *out, uint32_t cnt,
-                      cudaStream_t s);
-cudaError_t sort_pairs(void *temp, size_t &temp_bytes, const u64 *kin, u64 *kout,
-                       const uint32_t *vin, uint32_t *vout, uint32_t cnt, cudaStream_t s);
-// Scratch of the run finder (per batch capacity; temp = CUB scan storage).
-struct RunScratch {
-  uint32_t *flags, *pos, *start, *valid;
+// ingest (ingest.cu)
+struct Lists {
+  Rec *rec[4];  // deletions by source / destination, insertions by source / destination
+};
+// Distinct sources of the batch's valid records (tag null: not wanted), with
+// their degrees before the mutation for PageRank.
+struct Touch {
+  uint32_t *tag;
+  uint32_t epoch;
+  uint32_t *list, *count;
+  const uint32_t *live;
+  float *old_degree;
+};
+constexpr uint32_t INGEST_BLOCK_MAX = 8192;  // records of a list one CTA sorts
+struct IngestLaunch {
+  const BatchHdr *hdr;
+  Lists lists;
+  uint32_t nd, na;      // records of each kind, or a replayed class's capacities
+  uint32_t n;
+  bool has_in, with_w;
+  u64 *keys, *keys_sorted;  // device-wide form: all lists' keys and weights
+  uint32_t *w, *w_sorted;
   void *temp;
   size_t temp_bytes;
+  Touch touch;
+  Ctl *ctl;
+  uint32_t carry_q, carry;  // PageRank: carried frontier (queue, length)
 };
-size_t unique_runs_temp_bytes(uint32_t cnt);
-cudaError_t launch_unique_runs(const u64 *k, uint32_t cnt, uint2 *uv, uint32_t *mult,
-                               uint32_t *n_out, uint32_t cap, uint32_t *err, const RunScratch &S,
-                               cudaStream_t s);
-cudaError_t launch_row_segments(const u64 *k, uint32_t cnt, uint3 *seg, uint32_t *n_out,
-                                uint32_t cap, uint32_t *err, const RunScratch &S, cudaStream_t s);
-// Deleted occurrences found by the read-only search, written afterwards.
-struct Tombs {
-  u64 *pos;
-  uint32_t *count;
-  uint32_t cap;
-};
-// ctas: CTAs of the warp-per-record mutation kernels (0: one warp per record,
-// up to the grid cap)
-cudaError_t launch_delete_rows(const Adj &A, const uint2 *uv, const uint32_t *mult,
-                               const uint32_t *n_ptr, uint32_t max_n, uint32_t *found, Ctl *ctl,
-                               int count_missing, const Tombs &T, uint32_t ctas, cudaStream_t s);
-// Deletions in rows whose unsorted suffix exceeds DEFER_SUFFIX slots are
-// matched by sort-merge (gather the live suffix slots once, stable sort by
-// (row, neighbour), binary search per record) instead of a suffix scan per
-// record, whose cost grows with (records in the row) x (suffix length).
-constexpr uint32_t DEFER_SUFFIX = 1024;
-struct DeferDel {
-  bool on;
-  uint32_t *rem;       // per record: occurrences left after the sorted-prefix pass
-  u64 *packed;         // (deferred rows << 40) | suffix slots reserved
-  uint32_t *row_u;     // deferred rows, in reservation order
-  u64 *row_base;       // first gather index of each deferred row
-  uint32_t cap_rows;
-};
-struct DeferBufs {
-  u64 *k_in, *k_out;
-  uint32_t *v_in, *v_out;
-  void *temp;
-  size_t temp_bytes;
-};
-// pass over the sorted prefixes (and short suffixes); long suffixes deferred
-cudaError_t launch_delete_prefix(const Adj &A, const uint2 *uv, const uint32_t *mult,
-                                 const uint32_t *n_ptr, uint32_t max_n, uint32_t *found, Ctl *ctl,
-                                 int count_missing, const Tombs &T, const DeferDel &D,
-                                 uint32_t ctas, cudaStream_t s);
-size_t delete_sort_temp_bytes(u64 total);
-// sort-merge of the deferred suffixes (total gathered slots, nrows rows), then
-// the tombstones of all found occurrences
-cudaError_t launch_delete_suffix(const Adj &A, const uint2 *uv, const uint32_t *n_ptr,
-                                 uint32_t max_n, uint32_t *found, Ctl *ctl, int count_missing,
-                                 const Tombs &T, const DeferDel &D, uint32_t nrows, u64 total,
-                                 const DeferBufs &B, cudaStream_t s);
+size_t ingest_temp_bytes(uint64_t records);
+cudaError_t launch_ingest(const IngestLaunch &L, uint32_t *launches, cudaStream_t s);
 
+// mutation (mutate.cu)
+// Deletions in rows with a long unsorted suffix are matched with all the row's
+// records at once, SUFFIX_CHUNK slots per warp, instead of a suffix scan per
+// record, whose cost grows with (records in the row) x (suffix length). It costs
+// another phase (~15 us), so it pays from three records on (DEFER_RECORDS) once
+// the suffix is longer than a group's two steps (DEFER_SHORT), and for any number
+// of records above DEFER_SUFFIX slots (eight dependent host-link steps of a warp).
+// Scanning rows up to 1024 slots per record instead took 1.90 ms of a 100K-update
+// R-MAT 21 snapshot's mutation, this rule 1.14.
+constexpr uint32_t DEFER_SUFFIX = 1024, DEFER_SHORT = 64, DEFER_RECORDS = 3;
+constexpr uint32_t SUFFIX_CHUNK = 256, SUFFIX_KEEP = 16384;  // 16 MB of ids
 // Relocation bookkeeping for rows that outgrow their block.
 constexpr uint32_t RELOC_CHUNK = 1024;
 struct RelocRec {
-  uint32_t row, seg, len, pad;
+  uint32_t row, seg, len, dir;
   u64 old_off, new_off;
 };
 struct Reloc {
   RelocRec *rec;
   uint2 *chunks;
-  uint32_t *n_reloc, *n_chunks;
   uint32_t cap, chunk_cap;
 };
-cudaError_t launch_add_rows(const Adj &A, const u64 *k, const uint32_t *w, const uint3 *seg,
-                            const uint32_t *n_ptr, uint32_t max_n, const Reloc &R, Ctl *ctl,
-                            uint32_t ctas, cudaStream_t s);
-cudaError_t launch_keys_to_uvw(const u64 *k, const uint32_t *w, uint32_t cnt, uint3 *out,
-                               cudaStream_t s);
-cudaError_t launch_touched(const u64 *k, uint32_t cnt, uint32_t *tag, uint32_t epoch,
-                           uint32_t *list, uint32_t *n_out, Ctl *ctl, cudaStream_t s);
+struct MutParams {
+  Adj adj[2];                // outgoing, incoming
+  uint32_t dirs;             // directions kept: 1 or 2
+  bool deletions, insertions;
+  const BatchHdr *hdr;
+  const Rec *dels[2], *adds[2];
+  uint32_t *found;           // occurrences removed per record (by source)
+  uint32_t *rem[2], *matches[2];  // long suffixes: wanted and matching occurrences
+  uint4 *suffix;             // chunks: first record, end record, chunk, direction | chunks << 1
+  uint32_t suffix_cap;
+  uint32_t *suffix_ids;      // the first SUFFIX_KEEP chunks' slots, between the passes
+  Reloc reloc;
+  Ctl *ctl, *mctl;           // snapshot counters; this launch's barrier and queues
+  u64 timeout_ns;
+};
+// records: the longer of the two kinds (or the class's capacity); ctas: most
+// CTAs to launch
+cudaError_t launch_mutate(const MutParams &M, uint32_t records, uint32_t ctas, cudaStream_t s);
 
 // cache
 // Device-resident admission state: the free-slot count and the plan of the
@@ -251,8 +251,9 @@ cudaError_t launch_page_rows(const u64 *off, const uint32_t *len, uint32_t n, ui
 cudaError_t launch_page_rows_clear(uint32_t *rows, uint32_t *maxlen, uint32_t npages,
                                    const uint32_t *period, cudaStream_t s);
 cudaError_t launch_period_step(uint32_t *period, cudaStream_t s);
-cudaError_t launch_page_delta(const u64 *keys, uint32_t cnt, const u64 *off, uint32_t page_base,
-                              uint32_t page_shift, uint32_t *delta, cudaStream_t s);
+cudaError_t launch_page_delta(const Rec *recs, const BatchHdr *hdr, bool adds, uint32_t cap,
+                              const u64 *off, uint32_t page_base, uint32_t page_shift,
+                              uint32_t *delta, cudaStream_t s);
 cudaError_t launch_features(const uint32_t *hits, const float *hist, const uint8_t *age,
                             const uint32_t *delta, const uint32_t *rows, const uint32_t *maxlen,
                             uint32_t npages, void *x, cudaStream_t s);

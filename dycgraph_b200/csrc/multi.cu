@@ -51,11 +51,10 @@ struct MultiParams {
   Tiles tiles;
   Ctl *ctl;
   uint32_t *seq;
-  const uint2 *del_uv;
+  const BatchHdr *hdr;
+  const Rec *dels;
   const uint32_t *del_found;
-  const uint32_t *n_del_ptr;
-  const uint3 *add_uvw;
-  uint32_t n_add;
+  const Rec *adds;
   uint32_t n, phases, max_waves, qratio, pull_qratio, heavy, tile;
   uint32_t sched;   // item distribution: 0 static, 1 claimed (dycg_query_mapping.queue bit 0)
   bool ranges;      // wave queues ordered by vertex range (dycg_query_mapping.queue bit 1)
@@ -976,10 +975,10 @@ __global__ void __launch_bounds__(BLOCK, NB >= 8 ? DYCG_MULTI_MIN_BLOCKS : 3)
 
   if (P.phases & PH_DELETE) {
     // 1. seeds: (v, q) with parent_q(v) == u for a deleted (u, v); one warp per record
-    const uint32_t n_del = *P.n_del_ptr;
+    const uint32_t n_del = P.hdr->nd;
     for (uint32_t i = gw; i < n_del; i += nw) {
       if (!P.del_found[i]) continue;
-      const uint2 e = P.del_uv[i];
+      const Rec e = P.dels[i];
       bool any = false;
 #pragma unroll
       for (int k = 0; k < NB; k++) {
@@ -1075,8 +1074,9 @@ __global__ void __launch_bounds__(BLOCK, NB >= 8 ? DYCG_MULTI_MIN_BLOCKS : 3)
       }
     }
     if (P.phases & PH_INSERT) {
-      for (uint32_t i = gw; i < P.n_add; i += nw) {
-        const uint3 e = P.add_uvw[i];
+      const uint32_t n_add = P.hdr->na;
+      for (uint32_t i = gw; i < n_add; i += nw) {
+        const Rec e = P.adds[i];
         if (e.x >= P.n || e.y >= P.n) continue;
         bool any = false;
 #pragma unroll
@@ -1211,11 +1211,10 @@ static cudaError_t launch_multi_t(const MultiLaunch &L, cudaStream_t s) {
   P.tiles = Tiles{L.tiles, L.tile_cap};
   P.ctl = L.ctl;
   P.seq = L.seq;
-  P.del_uv = L.del_uv;
+  P.hdr = L.hdr;
+  P.dels = L.dels;
   P.del_found = L.del_found;
-  P.n_del_ptr = L.n_del_ptr;
-  P.add_uvw = L.add_uvw;
-  P.n_add = L.n_add;
+  P.adds = L.adds;
   P.n = L.n;
   P.phases = L.phases;
   P.max_waves = L.max_waves;

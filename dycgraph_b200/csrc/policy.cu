@@ -86,14 +86,15 @@ __global__ void page_rows_kernel(const u64 *off, const uint32_t *len, uint32_t n
   }
 }
 
-// Update records per page: each sorted batch key (row << 32 | neighbour) names
-// the row it touches in this arena.
-__global__ void page_delta_kernel(const u64 *keys, uint32_t cnt, const u64 *off,
+// Update records per page: each list entry names the row it touches in this
+// arena.
+__global__ void page_delta_kernel(const Rec *recs, const BatchHdr *hdr, bool adds, const u64 *off,
                                   uint32_t page_base, uint32_t page_shift, uint32_t *delta) {
+  const uint32_t cnt = adds ? hdr->na : hdr->nd;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
-    const u64 k = keys[i];
-    if (k == KEY_INF) continue;
-    atomicAdd(delta + page_base + (uint32_t)(off[(uint32_t)(k >> 32)] >> page_shift), 1u);
+    const uint32_t row = recs[i].x;
+    if (row == INF32) continue;
+    atomicAdd(delta + page_base + (uint32_t)(off[row] >> page_shift), 1u);
   }
 }
 
@@ -713,10 +714,12 @@ cudaError_t launch_period_step(uint32_t *period, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_page_delta(const u64 *keys, uint32_t cnt, const u64 *off, uint32_t page_base,
-                              uint32_t page_shift, uint32_t *delta, cudaStream_t s) {
-  if (!cnt) return cudaSuccess;
-  page_delta_kernel<<<grid_for(cnt), BLOCK, 0, s>>>(keys, cnt, off, page_base, page_shift, delta);
+cudaError_t launch_page_delta(const Rec *recs, const BatchHdr *hdr, bool adds, uint32_t cap,
+                              const u64 *off, uint32_t page_base, uint32_t page_shift,
+                              uint32_t *delta, cudaStream_t s) {
+  if (!cap) return cudaSuccess;
+  page_delta_kernel<<<grid_for(cap), BLOCK, 0, s>>>(recs, hdr, adds, off, page_base, page_shift,
+                                                    delta);
   return cudaGetLastError();
 }
 

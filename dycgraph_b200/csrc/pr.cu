@@ -33,11 +33,10 @@ struct PrParams {
   uint32_t *q[2];
   const uint32_t *sources;  // touched sources (amend)
   const uint32_t *n_sources;
-  const uint2 *del_uv;      // distinct deleted (u, v) pairs and occurrences found
+  const BatchHdr *hdr;
+  const Rec *dels;          // deleted (u, v); occurrences found at run heads, 0 elsewhere
   const uint32_t *del_found;
-  const uint32_t *n_del;
-  const uint3 *add_uvw;     // inserted occurrences (u >= n: invalid record)
-  uint32_t n_add;
+  const Rec *adds;          // inserted occurrences (u >= n: invalid record)
   Tiles tiles;
   Ctl *ctl;
   uint32_t n;
@@ -144,36 +143,33 @@ struct ScatterOp {
 // deleted occurrence, +alpha x[u]/deg_old for each inserted one (together with
 // the row pass that makes it alpha x[u]/deg_new). Appends into q[cur].
 __device__ void amend_records(const PrParams &P, uint32_t cur, Acc &acc) {
-  const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t gstride = gridDim.x * blockDim.x;
+  const uint32_t lane = lane_id();
+  const uint32_t first = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32;
+  const uint32_t step = gridDim.x * blockDim.x;
   uint32_t *q = P.q[cur], *qc = &P.ctl->q_count[cur];
-  const uint32_t nd = *P.n_del;
-  for (uint32_t i = gtid; i < nd; i += gstride) {
-    const uint32_t f = P.del_found[i];
-    bool want = false;
-    const uint2 e = P.del_uv[i];
-    if (f) {
-      const uint32_t dold = old_degree(&P, e.x);
-      const float xu = P.x[e.x];
-      if (dold && xu != 0.f) {
-        want = pr_add(&P, e.y, -P.alpha * xu * (float)f / (float)dold);
-        acc.improved++;
+  const uint32_t nd = P.hdr->nd, na = P.hdr->na;
+  for (int adds = 0; adds < 2; adds++) {
+    const uint32_t cnt = adds ? na : nd;
+    const Rec *list = adds ? P.adds : P.dels;
+    for (uint32_t i0 = first; i0 < cnt; i0 += step) {  // warp-uniform
+      const uint32_t i = i0 + lane;
+      const Rec e = i < cnt ? list[i] : make_uint4(INF32, INF32, 0, 0);
+      bool want[1] = {false};
+      const uint32_t v[1] = {e.y};
+      // (a record has both endpoints in range or neither)
+      const uint32_t f = e.x >= P.n ? 0u : adds ? 1u : P.del_found[i];
+      if (f) {
+        const uint32_t dold = old_degree(&P, e.x);
+        const float xu = P.x[e.x];
+        if (dold && xu != 0.f) {
+          const float c = adds ? P.alpha * xu / (float)dold
+                               : -P.alpha * xu * (float)f / (float)dold;
+          want[0] = pr_add(&P, e.y, c);
+          acc.improved++;
+        }
       }
+      append_batch(q, qc, P.n, want, v, &P.ctl->err);
     }
-    warp_append(q, qc, P.n, want, e.y, &P.ctl->err);
-  }
-  for (uint32_t i = gtid; i < P.n_add; i += gstride) {
-    const uint3 e = P.add_uvw[i];
-    bool want = false;
-    if (e.x < P.n && e.y < P.n) {
-      const uint32_t dold = old_degree(&P, e.x);
-      const float xu = P.x[e.x];
-      if (dold && xu != 0.f) {
-        want = pr_add(&P, e.y, P.alpha * xu / (float)dold);
-        acc.improved++;
-      }
-    }
-    warp_append(q, qc, P.n, want, e.y, &P.ctl->err);
   }
 }
 
@@ -255,11 +251,10 @@ cudaError_t launch_pr(const PrLaunch &L, cudaStream_t s) {
   P.q[1] = L.q1;
   P.sources = L.sources;
   P.n_sources = L.n_sources;
-  P.del_uv = L.del_uv;
+  P.hdr = L.hdr;
+  P.dels = L.dels;
   P.del_found = L.del_found;
-  P.n_del = L.n_del;
-  P.add_uvw = L.add_uvw;
-  P.n_add = L.n_add;
+  P.adds = L.adds;
   P.tiles = Tiles{L.tiles, L.tile_cap};
   P.ctl = L.ctl;
   P.n = L.n;
@@ -278,26 +273,6 @@ cudaError_t launch_pr(const PrLaunch &L, cudaStream_t s) {
   void *args[] = {&P};
   return cudaLaunchCooperativeKernel((const void *)pr_kernel, blocks_per_sm * L.num_sms, BLOCK,
                                      args, 0, s);
-}
-
-// deg_old of every touched source, kept in the delta array until the amend
-__global__ void pr_old_degree_kernel(const uint32_t *sources, const uint32_t *n_sources,
-                                     const uint32_t *live, float *delta) {
-  const uint32_t cnt = *n_sources;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt;
-       i += gridDim.x * blockDim.x) {
-    const uint32_t u = sources[i];
-    delta[u] = __uint_as_float(live[u]);
-  }
-}
-
-cudaError_t launch_pr_old_degree(const uint32_t *sources, const uint32_t *n_sources,
-                                 uint32_t max_sources, const uint32_t *live, float *delta,
-                                 cudaStream_t s) {
-  if (!max_sources) return cudaSuccess;
-  const int grid = (int)std::min<u64>((max_sources + BLOCK - 1) / BLOCK, 148ull * 16);
-  pr_old_degree_kernel<<<grid, BLOCK, 0, s>>>(sources, n_sources, live, delta);
-  return cudaGetLastError();
 }
 
 cudaError_t launch_pr_init(float *x, float *r, uint32_t *queued, uint32_t *q0, uint32_t n,

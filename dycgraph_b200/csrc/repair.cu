@@ -39,11 +39,10 @@ struct RepairParams {
   uint32_t *q[2];
   Tiles tiles;
   Ctl *ctl;
-  const uint2 *del_uv;      // unique deleted (u,v)
-  const uint32_t *del_found; // occurrences removed per unique record
-  const uint32_t *n_del_ptr; // device count of unique records
-  const uint3 *add_uvw;     // valid insertions (u,v,w)
-  uint32_t n_add;
+  const BatchHdr *hdr;
+  const Rec *dels;          // deleted (u,v); del_found: occurrences removed
+  const uint32_t *del_found;
+  const Rec *adds;          // insertions (u,v,w)
   uint32_t n;
   uint32_t source;
   uint32_t epoch;
@@ -253,13 +252,13 @@ __global__ void __launch_bounds__(REPAIR_BLOCK, 1) repair_kernel(const __grid_co
 
   if (P.phases & PH_DELETE) {
     // 1. deletion seeds (warp-uniform loop so appends can aggregate)
-    const uint32_t n_del = *P.n_del_ptr;
+    const uint32_t n_del = P.hdr->nd;
     for (uint32_t i0 = first; i0 < n_del; i0 += gstride) {
       const uint32_t i = i0 + lane;
       bool want[1] = {false};
       uint32_t v[1] = {0};
       if (i < n_del && P.del_found[i] != 0) {
-        const uint2 e = P.del_uv[i];
+        const Rec e = P.dels[i];
         v[0] = e.y;
         if (!(ALGO != ALGO_CC && e.y == P.source) &&
             key_parent1(ld_key(P.key + e.y)) == e.x + 1u) {
@@ -285,11 +284,12 @@ __global__ void __launch_bounds__(REPAIR_BLOCK, 1) repair_kernel(const __grid_co
   // phase: whatever either reads is an upper bound of a live path, and every
   // vertex either lowers enters the first frontier
   if (P.phases & PH_INSERT) {
-    for (uint32_t i0 = first; i0 < P.n_add; i0 += gstride) {
+    const uint32_t n_add = P.hdr->na;
+    for (uint32_t i0 = first; i0 < n_add; i0 += gstride) {
       const uint32_t i = i0 + lane;
       bool want[1] = {false};
       uint32_t v[1] = {0}, imp = INF32;
-      const uint3 e = i < P.n_add ? P.add_uvw[i] : make_uint3(INF32, INF32, 0);
+      const Rec e = i < n_add ? P.adds[i] : make_uint4(INF32, INF32, 0, 0);
       if (e.x < P.n) {
         v[0] = e.y;
         const uint32_t du = key_value(ld_key(P.key + e.x));
@@ -395,11 +395,10 @@ static cudaError_t launch_one(const RepairLaunch &L, cudaStream_t s) {
   P.q[1] = L.q1;
   P.tiles = Tiles{L.tiles, L.tile_cap};
   P.ctl = L.ctl;
-  P.del_uv = L.del_uv;
+  P.hdr = L.hdr;
+  P.dels = L.dels;
   P.del_found = L.del_found;
-  P.n_del_ptr = L.n_del_ptr;
-  P.add_uvw = L.add_uvw;
-  P.n_add = L.n_add;
+  P.adds = L.adds;
   P.n = L.n;
   P.source = L.source;
   P.epoch = L.epoch;
