@@ -269,7 +269,7 @@ __global__ void resolve_positions_kernel(const u64 *pos, u64 count, const u64 *p
     }
     for (uint32_t s = 0; s < len && k < len; s++) {
       const uint2 pr = read_pair_rw(A, off + s);
-      if (slot_deleted_rw(A, off + s, pr.x)) continue;
+      if (slot_deleted_rw(A, off + s)) continue;
       if (k == 0) {
         v = pr.x;
         w = pr.y;
@@ -299,7 +299,7 @@ __global__ void row_edges_kernel(Adj A, const uint32_t *sources, u64 count, u64 
       for (int t = 0; t < 16 && !got; t++) {
         const uint32_t k = (uint32_t)(mix64(seed ^ mix64(i * 16 + t + 1)) % len);
         const uint2 pr = read_pair_rw(A, off + k);
-        if (!slot_deleted_rw(A, off + k, pr.x)) {
+        if (!slot_deleted_rw(A, off + k)) {
           v = pr.x & VMASK;
           w = pr.y;
           got = true;
@@ -307,7 +307,7 @@ __global__ void row_edges_kernel(Adj A, const uint32_t *sources, u64 count, u64 
       }
       for (uint32_t k = 0; k < len && !got; k++) {
         const uint2 pr = read_pair_rw(A, off + k);
-        if (!slot_deleted_rw(A, off + k, pr.x)) {
+        if (!slot_deleted_rw(A, off + k)) {
           v = pr.x & VMASK;
           w = pr.y;
           got = true;

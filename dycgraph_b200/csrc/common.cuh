@@ -1,12 +1,13 @@
 // common.cuh -- shared device types and helpers of the B200 delta-repair engine.
 //
 // Adjacency layout (one arena per direction, pinned + mapped host memory):
-//   dst[slot]  uint32 neighbour id; bit 31 set = deleted occurrence (tombstone)
+//   dst[slot]  uint32 neighbour id
 //   w[slot]    uint32 weight (only when weights are stored)
 // Each vertex owns a block [off, off+cap) of slots; [0,len) is in use, of which
-// [0,srt) is sorted by neighbour id (tombstones keep their id bits, so binary
-// search still works) and [srt,len) holds appended occurrences in insertion
-// order; live = occurrences in use minus tombstones.
+// [0,srt) is sorted by neighbour id and [srt,len) holds appended occurrences in
+// insertion order; a deleted slot keeps its id (so binary search still works)
+// and has its bit set in the HBM deletion bitmap until its row is compacted;
+// live = occurrences in use minus deleted ones.
 //
 // The arena is split into pages of 2^page_shift slots. page_slot[page] names
 // the HBM cache slot holding a copy of the page, or PAGE_NONE. Every write goes
@@ -29,7 +30,7 @@ namespace dycg {
 typedef unsigned long long u64;
 
 constexpr uint32_t PAGE_NONE = 0xFFFFFFFFu;
-constexpr uint32_t TOMB = 0x80000000u;
+constexpr uint32_t TOMB = 0x80000000u;  // marks a deleted slot in registers and staging
 constexpr uint32_t VMASK = 0x7FFFFFFFu;
 constexpr uint32_t INF32 = 0xFFFFFFFFu;
 constexpr u64 KEY_INF = ~0ull;
@@ -233,14 +234,14 @@ __device__ __forceinline__ uint2 read_pair_rw(const Adj &a, u64 p) {
   return make_uint2(*q, 0u);
 }
 
-// Deleted: tombstone bit in the slot (materialised by a row relocation) or the
-// slot's bit in the HBM deletion bitmap (set by the deletion kernels).
-__device__ __forceinline__ bool slot_deleted(const Adj &a, u64 p, uint32_t d) {
-  return (d & TOMB) || ((__ldg(a.tbits + (p >> 5)) >> (p & 31)) & 1u);
+// Deleted: the slot's bit in the HBM deletion bitmap.
+__device__ __forceinline__ bool slot_deleted(const Adj &a, u64 p) {
+  return (__ldg(a.tbits + (p >> 5)) >> (p & 31)) & 1u;
 }
 
-__device__ __forceinline__ bool slot_deleted_rw(const Adj &a, u64 p, uint32_t d) {
-  return (d & TOMB) || ((*(volatile uint32_t *)(a.tbits + (p >> 5)) >> (p & 31)) & 1u);
+// Same, for kernels that also set bits (no read-only cache path).
+__device__ __forceinline__ bool slot_deleted_rw(const Adj &a, u64 p) {
+  return (*(volatile uint32_t *)(a.tbits + (p >> 5)) >> (p & 31)) & 1u;
 }
 
 // Write-through store of one slot: host arena (one 8-byte store with

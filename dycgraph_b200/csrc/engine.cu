@@ -176,6 +176,7 @@ void Engine::build_direction(Arena &A, const u64 *keys, const uint32_t *wv, u64 
   const u64 permille = opt_.arena_headroom_permille ? opt_.arena_headroom_permille : 125;
   const u64 head = std::max<u64>(total / 1000 * permille, 1ull << 20);
   A.slots = round_up(total + head, page);
+  A.scarce = total + head / 2;
   A.pages = (uint32_t)(A.slots >> page_shift_);
   A.stride = stored_ ? 2 : 1;
   A.fence_shift = stored_ ? 4 : 5;
@@ -640,6 +641,7 @@ void Engine::ensure_batch(size_t cnt) {
   touched_ = (uint32_t *)al(c * 2 * 4);
   const u64 slots = out_.slots + (has_in_ ? in_.slots : 0);
   reloc_.rec = (RelocRec *)al(dirs * c * sizeof(RelocRec));
+  reloc_.wide = (uint32_t *)al(dirs * c * 4);
   reloc_.cap = (uint32_t)(dirs * c);
   const u64 cc = std::min<u64>(slots / RELOC_CHUNK + dirs * c + 1024, 0x7FFFFFFFull);
   reloc_.chunks = (uint2 *)al(cc * sizeof(uint2));
@@ -762,6 +764,8 @@ void Engine::enqueue_snapshot(size_t nd, size_t na, bool capture) {
     M.suffix_cap = suffix_cap_;
     M.suffix_ids = suffix_ids_;
     M.reloc = reloc_;
+    M.scarce[0] = out_.scarce;
+    M.scarce[1] = in_.scarce;
     M.ctl = ctl_;
     M.mctl = mctl_;
     M.timeout_ns = timeout;
@@ -1862,7 +1866,7 @@ void Engine::get_row(uint32_t v, int incoming, uint32_t *dst, uint32_t *w, uint3
   for (uint32_t s = 0; s < len; s++) {
     const u64 p = off + s;
     const uint32_t d = A.h_dst[p * A.stride];
-    if ((d & TOMB) || ((bits[(p >> 5) - w0] >> (p & 31)) & 1u)) continue;
+    if ((bits[(p >> 5) - w0] >> (p & 31)) & 1u) continue;
     if (k < cap) {
       if (dst) dst[k] = d;
       if (w) w[k] = A.stride == 2 ? A.h_dst[p * 2 + 1] : 0u;
@@ -1886,7 +1890,7 @@ void Engine::export_csr(uint64_t *off, uint32_t *dst, uint32_t *w) {
     for (uint32_t s = 0; s < l[v]; s++) {
       const u64 p = o[v] + s;
       const uint32_t d = out_.h_dst[p * out_.stride];
-      if ((d & TOMB) || ((bits[p >> 5] >> (p & 31)) & 1u)) continue;
+      if ((bits[p >> 5] >> (p & 31)) & 1u) continue;
       if (dst) dst[q] = d;
       if (w) w[q] = out_.stride == 2 ? out_.h_dst[p * 2 + 1] : 0u;
       q++;

@@ -34,7 +34,7 @@ struct Arena {
   uint32_t stride = 1;        // words per slot: 1 (id) or 2 (id, weight)
   uint32_t fence_shift = 5;   // one fence per 128 bytes of slots
   uint32_t *tbits = nullptr;  // HBM deletion bitmap
-  u64 slots = 0;
+  u64 slots = 0, scarce = 0;  // slots in all; top past which space is scarce
   uint32_t pages = 0, page_base = 0;
   u64 *off = nullptr;
   uint32_t *len = nullptr, *cap = nullptr, *srt = nullptr, *live = nullptr;

@@ -222,7 +222,7 @@ __device__ __forceinline__ void group_slots(const Adj &A, uint32_t v, bool on, u
         } else {
           d[u] = read_dst(A, p, cached[u]);
         }
-        if (slot_deleted(A, p, d[u])) d[u] |= TOMB;
+        if (slot_deleted(A, p)) d[u] |= TOMB;
       }
     }
 #pragma unroll

@@ -161,7 +161,7 @@ cudaError_t launch_ingest(const IngestLaunch &L, uint32_t *launches, cudaStream_
 // R-MAT 21 snapshot's mutation, this rule 1.14.
 constexpr uint32_t DEFER_SUFFIX = 1024, DEFER_SHORT = 64, DEFER_RECORDS = 3;
 constexpr uint32_t SUFFIX_CHUNK = 256, SUFFIX_KEEP = 16384;  // 16 MB of ids
-// Relocation bookkeeping for rows that outgrow their block.
+// Bookkeeping of rows whose block is full: new_off == old_off, compacted in place.
 constexpr uint32_t RELOC_CHUNK = 1024;
 struct RelocRec {
   uint32_t row, seg, len, dir;
@@ -169,7 +169,8 @@ struct RelocRec {
 };
 struct Reloc {
   RelocRec *rec;
-  uint2 *chunks;
+  uint2 *chunks;      // of rows that move
+  uint32_t *wide;     // long rows that stay
   uint32_t cap, chunk_cap;
 };
 struct MutParams {
@@ -184,6 +185,7 @@ struct MutParams {
   uint32_t suffix_cap;
   uint32_t *suffix_ids;      // the first SUFFIX_KEEP chunks' slots, between the passes
   Reloc reloc;
+  u64 scarce[2];             // arena top from which full rows stay in their blocks if they can
   Ctl *ctl, *mctl;           // snapshot counters; this launch's barrier and queues
   u64 timeout_ns;
 };

@@ -164,7 +164,7 @@ __device__ __forceinline__ void walk(const Adj &A, u64 off, uint32_t b, uint32_t
         } else {
           d[u] = read_dst(A, p, cached[u]);
         }
-        if (slot_deleted(A, p, d[u])) d[u] |= TOMB;
+        if (slot_deleted(A, p)) d[u] |= TOMB;
       }
     }
 #pragma unroll
@@ -309,7 +309,7 @@ __device__ __forceinline__ void stage_slots(const Adj &A, uint32_t v, uint32_t b
       } else {
         d = read_dst(A, p, cached);
       }
-      if (slot_deleted(A, p, d)) d |= TOMB;
+      if (slot_deleted(A, p)) d |= TOMB;
       const bool valid = !(d & TOMB);
       if (cached) acc.hbm += valid ? bytes : 4u;
       else acc.link += valid ? bytes : 4u;

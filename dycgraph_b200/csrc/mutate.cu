@@ -5,8 +5,8 @@
 // (include/groute/graphs/source_local_chunk_store.h:220-406,
 // BuildDeletionPlan :685-739): a deletion requested r times removes r live
 // occurrences (fewer if fewer exist: the rest are counted missing), additions
-// append occurrences, and a row that outgrows its block moves to a new
-// power-of-two block at the arena tail. Rows stay sorted in their prefix, so
+// append occurrences, and a row whose block is full drops its deleted slots and,
+// if it outgrew the block, moves to a new power-of-two block at the arena tail. Rows stay sorted in their prefix, so
 // a deletion finds its target through the HBM fence index and one 128-byte
 // read of the row instead of the reference's linear row scan. A deletion sets
 // a bit of the HBM deletion bitmap (no host-link write).
@@ -33,6 +33,7 @@ namespace dycg {
 namespace {
 
 constexpr int MUT_BLOCK = 512;
+constexpr uint32_t COMPACT_WARP = 1024;  // longest row that one warp compacts
 
 struct Counts {
   uint32_t link = 0, hbm = 0, missing = 0, moved = 0;
@@ -65,7 +66,7 @@ __device__ __forceinline__ uint32_t take_slots(const Adj &A, u64 off, uint32_t s
 #pragma unroll
     for (int u = 0; u < U; u++) {
       const uint32_t x = s + u * W + gl;
-      d[u] = TOMB;
+      d[u] = 0;
       b[u] = 1;
       if (go && x < end) {
         const u64 p = off + x;
@@ -79,10 +80,10 @@ __device__ __forceinline__ uint32_t take_slots(const Adj &A, u64 off, uint32_t s
     for (int u = 0; u < U; u++) {
       const uint32_t x = s + u * W + gl;
       const bool in = go && x < end;
-      const bool live = in && d[u] == target && !b[u];  // (a tombstone bit differs)
+      const bool live = in && d[u] == target && !b[u];
       const unsigned lm = (__ballot_sync(0xffffffffu, live) >> gsh) & gmask;
       const unsigned pm =
-          (__ballot_sync(0xffffffffu, in && sorted && (d[u] & VMASK) > target) >> gsh) & gmask;
+          (__ballot_sync(0xffffffffu, in && sorted && d[u] > target) >> gsh) & gmask;
       if (live && (uint32_t)__popc(lm & ((1u << gl) - 1)) < rem) {
         const u64 p = off + x;
         atomicOr(A.tbits + (p >> 5), 1u << (p & 31));
@@ -264,7 +265,7 @@ __device__ void suffix_chunk(const MutParams &M, uint32_t c, Counts &C) {
       if (s < e) {
         const u64 p = off + s;
         const uint32_t x = read_dst_rw(A, p);
-        if (!slot_deleted_rw(A, p, x)) d[u] = x;
+        if (!slot_deleted_rw(A, p)) d[u] = x;
         if (page_of(A, p) == pg0) same++;
         else atomicAdd(A.page_hits + page_of(A, p), 1u);
         if (cached) C.hbm += 4; else C.link += 4;
@@ -369,88 +370,197 @@ __device__ void append_slots(const MutParams &M, uint32_t dir, uint32_t pos, uin
   }
 }
 
-// Then, the deletions done, the descriptors: a row that does not fit gets a new
-// power-of-two block (with headroom) at the arena tail; its descriptor moves at
-// once, while the copy of the old slots and the append are left to the
-// relocation phase, so a large row is copied by many warps.
+// Then, the deletions done, the descriptors. A row that does not fit drops its
+// deleted slots on its way to a new power-of-two block (with headroom) at the
+// arena tail, or in its own block: when they are half of it (the copy then pays
+// for itself), and, once half of the arena's headroom is used, whenever the live
+// occurrences and a reserve fit. While there is headroom a row with few deleted
+// slots gets the block its slots ask for. So a stream of balanced updates cannot
+// eat the arena (2,000-update snapshots on R-MAT 16 used to after some 5,000 of
+// them) and no repair reads a slot deleted long ago for ever. Rows that change
+// their slots are left to the relocation phase.
 __device__ void append_rows(const MutParams &M, uint32_t dir, uint32_t pos, uint32_t na,
                             Counts &C) {
   const Adj &A = M.adj[dir];
   const Rec r = pos < na ? M.adds[dir][pos] : make_uint4(INF32, INF32, 0u, 0u);
   const uint32_t row = r.x, count = r.w;
   if (!count) return;
-  const uint32_t len = A.len[row];
-  if ((u64)len + count <= A.cap[row]) {
+  const uint32_t len = A.len[row], cap = A.cap[row], live = A.live[row];
+  if ((u64)len + count <= cap) {
     A.len[row] = len + count;
-    A.live[row] += count;
+    A.live[row] = live + count;
     // appends stay in the unsorted suffix (no host-link read here); an
     // empty row takes its sorted run of appends as its sorted prefix
     if (len == 0) A.srt[row] = count;
     return;
   }
-  const u64 need = (u64)len + count;
-  const uint32_t ncap = next_pow2_u32((uint32_t)(need + need / 8 + 1));
-  const u64 noff = atomicAdd(A.top, (u64)ncap);
+  const auto block = [](u64 slots) { return next_pow2_u32((uint32_t)(slots + slots / 8 + 1)); };
+  const u64 need = (u64)live + count, off = A.off[row];
+  const bool scarce = *(volatile u64 *)A.top > M.scarce[dir];
+  const uint32_t tight = block(need);
+  if (tight > cap || !(scarce || need <= cap / 2)) {
+    const uint32_t ncap = scarce ? tight : block((u64)len + count);
+    const u64 noff = atomicAdd(A.top, (u64)ncap);
+    const uint32_t nchunk = (len + RELOC_CHUNK - 1) / RELOC_CHUNK;
+    const uint32_t cb = atomicAdd(&M.mctl->tile_count, nchunk);
+    const uint32_t k = atomicAdd(&M.mctl->q_count[1], 1u);
+    if (noff + ncap > A.arena || k >= M.reloc.cap || cb + nchunk > M.reloc.chunk_cap) {
+      atomicCAS(&M.ctl->err, 0u, ERR_ARENA);
+      return;
+    }
+    M.reloc.rec[k] = RelocRec{row, pos, len, dir, off, noff};
+    for (uint32_t c = 0; c < nchunk; c++) M.reloc.chunks[cb + c] = make_uint2(k, c);
+    A.off[row] = noff;
+    A.cap[row] = ncap;
+    C.moved++;
+    return;
+  }
   const uint32_t k = atomicAdd(&M.mctl->q_count[1], 1u);
-  const uint32_t nchunk = (len + RELOC_CHUNK - 1) / RELOC_CHUNK;
-  const uint32_t cb = atomicAdd(&M.mctl->tile_count, nchunk);
-  if (noff + ncap > A.arena || k >= M.reloc.cap || cb + nchunk > M.reloc.chunk_cap) {
+  if (k >= M.reloc.cap) {
     atomicCAS(&M.ctl->err, 0u, ERR_ARENA);
     return;
   }
-  M.reloc.rec[k] = RelocRec{row, pos, len, dir, A.off[row], noff};
-  for (uint32_t c = 0; c < nchunk; c++) M.reloc.chunks[cb + c] = make_uint2(k, c);
-  A.off[row] = noff;
-  A.cap[row] = ncap;
-  C.moved++;
+  M.reloc.rec[k] = RelocRec{row, pos, len, dir, off, off};
+  // a long row takes a whole CTA
+  if (len > COMPACT_WARP) M.reloc.wide[atomicAdd(&M.mctl->q_count[2], 1u)] = k;
 }
 
-// Warp per RELOC_CHUNK slots of a relocated row: verbatim copy (tombstones
-// included, so the sorted prefix and the live count stay valid), eight loads
+// Deleted slots among the first `count` of the row at off (warp-collective).
+__device__ __forceinline__ uint32_t dead_slots(const Adj &A, u64 off, uint32_t count) {
+  if (!count) return 0;
+  const u64 w0 = off >> 5, w1 = (off + count - 1) >> 5;
+  uint32_t dead = 0;
+  for (u64 w = w0 + lane_id(); w <= w1; w += 32) {
+    uint32_t b = *(volatile uint32_t *)(A.tbits + w);
+    if (w == w0) b &= ~0u << (off & 31);
+    if (w == w1) b &= ~0u >> (31 - ((off + count - 1) & 31));
+    dead += __popc(b);
+  }
+  return __reduce_add_sync(0xffffffffu, dead);
+}
+
+// Warp per RELOC_CHUNK slots of a row that moves: its live slots in order,
+// behind those of the chunks before it (the bitmap tells how many), eight loads
 // in flight per lane.
 __device__ void relocate_chunk(const MutParams &M, uint2 ch, Counts &C) {
   const RelocRec rec = M.reloc.rec[ch.x];
   const Adj &A = M.adj[rec.dir];
   const uint32_t bytes = 4u * A.stride;
   const uint32_t b = ch.y * RELOC_CHUNK, e = min(rec.len, b + RELOC_CHUNK);
+  u64 to = rec.new_off + b - dead_slots(A, rec.old_off, b);
   constexpr uint32_t PER = 8;
   for (uint32_t s0 = b; s0 < e; s0 += PER * 32) {
     uint2 v[PER];
+    bool live[PER];
 #pragma unroll
     for (uint32_t t = 0; t < PER; t++) {
       const uint32_t s = s0 + t * 32 + lane_id();
+      live[t] = false;
       if (s < e) {
         v[t] = read_pair_rw(A, rec.old_off + s);
-        // a slot deleted through the bitmap keeps its deletion as a tombstone bit
-        if (slot_deleted_rw(A, rec.old_off + s, v[t].x)) v[t].x |= TOMB;
+        live[t] = !slot_deleted_rw(A, rec.old_off + s);
+        C.link += bytes;
       }
     }
 #pragma unroll
     for (uint32_t t = 0; t < PER; t++) {
-      const uint32_t s = s0 + t * 32 + lane_id();
-      if (s < e) {
-        const bool c = write_slot(A, rec.new_off + s, v[t].x, v[t].y);
-        C.link += 2 * bytes;
+      const unsigned lm = __ballot_sync(0xffffffffu, live[t]);
+      if (live[t]) {
+        const bool c =
+            write_slot(A, to + __popc(lm & ((1u << lane_id()) - 1)), v[t].x, v[t].y);
+        C.link += bytes;
         if (c) C.hbm += bytes;
       }
+      to += __popc(lm);
     }
   }
 }
 
-// Warp per relocated row: append its segment after the copied slots.
-__device__ void relocate_append(const MutParams &M, const RelocRec &rec) {
+// The same within a row's own block, by T threads (a warp, or a CTA with sm):
+// T * 4 slots at a time are read before the live ones among them are written,
+// never past what has been read, and their deletion bits are cleared.
+template <uint32_t T>
+__device__ void compact_row(const MutParams &M, const RelocRec &rec, uint32_t *sm, Counts &C) {
+  const Adj &A = M.adj[rec.dir];
+  const uint32_t bytes = 4u * A.stride;
+  const uint32_t me = T == 32 ? lane_id() : threadIdx.x, warp = me >> 5;
+  constexpr uint32_t PER = 4, W = T / 32;
+  u64 to = rec.old_off;
+  for (uint32_t s0 = 0; s0 < rec.len; s0 += PER * T) {
+    uint2 v[PER];
+    unsigned lm[PER];
+#pragma unroll
+    for (uint32_t t = 0; t < PER; t++) {
+      const uint32_t s = s0 + t * T + me;
+      const u64 p = rec.old_off + s;
+      bool live = false;
+      if (s < rec.len) {
+        v[t] = read_pair_rw(A, p);
+        live = !slot_deleted_rw(A, p);
+        if (!live) atomicAnd(A.tbits + (p >> 5), ~(1u << (p & 31)));
+        C.link += bytes;
+      }
+      lm[t] = __ballot_sync(0xffffffffu, live);
+      if (T > 32 && lane_id() == 0) sm[t * W + warp] = __popc(lm[t]);
+    }
+    // every read of this step is done before any write of it
+    if (T > 32) __syncthreads();
+    else __syncwarp();
+#pragma unroll
+    for (uint32_t t = 0; t < PER; t++) {
+      uint32_t before = 0, all = __popc(lm[t]);
+      if (T > 32) {
+        all = 0;
+        for (uint32_t w = 0; w < W; w++) {
+          if (w == warp) before = all;
+          all += sm[t * W + w];
+        }
+      }
+      if ((lm[t] >> lane_id()) & 1u) {
+        const u64 p = to + before + __popc(lm[t] & ((1u << lane_id()) - 1));
+        if (p != rec.old_off + s0 + t * T + me) {
+          const bool c = write_slot(A, p, v[t].x, v[t].y);
+          C.link += bytes;
+          if (c) C.hbm += bytes;
+        }
+      }
+      to += all;
+    }
+    if (T > 32) __syncthreads();  // (sm is free again)
+  }
+}
+
+// A row's inserted occurrences behind its live slots, and its descriptor; sorted:
+// live slots of its sorted prefix. T threads, me-th of them.
+__device__ void finish_row(const MutParams &M, const RelocRec &rec, uint32_t sorted, uint32_t me,
+                           uint32_t T) {
   const Adj &A = M.adj[rec.dir];
   const Rec *list = M.adds[rec.dir];
-  const uint32_t count = list[rec.seg].w;
-  for (uint32_t j = lane_id(); j < count; j += 32) {
+  const uint32_t count = list[rec.seg].w, live = A.live[rec.row];
+  for (uint32_t j = me; j < count; j += T) {
     const Rec x = list[rec.seg + j];
-    write_slot(A, rec.new_off + rec.len + j, x.y, x.z);
+    write_slot(A, rec.new_off + live + j, x.y, x.z);
   }
-  if (lane_id() == 0) {
-    if (rec.len == 0) A.srt[rec.row] = count;
-    A.len[rec.row] = rec.len + count;
-    A.live[rec.row] += count;
+  if (T == 32) __syncwarp();
+  else __syncthreads();  // every thread has read the old descriptor
+  if (me == 0) {
+    A.srt[rec.row] = live ? sorted : count;
+    A.len[rec.row] = live + count;
+    A.live[rec.row] = live + count;
   }
+}
+
+// Warp per listed row: rows that moved get their insertions, short ones that
+// stay are compacted first.
+__device__ void finish_warp(const MutParams &M, const RelocRec &rec, Counts &C) {
+  const Adj &A = M.adj[rec.dir];
+  const bool stays = rec.new_off == rec.old_off;
+  if (stays && rec.len > COMPACT_WARP) return;  // a CTA's
+  const uint32_t srt = A.srt[rec.row];
+  const uint32_t sorted = srt - dead_slots(A, rec.old_off, srt);
+  __syncwarp();
+  if (stays) compact_row<32>(M, rec, nullptr, C);
+  finish_row(M, rec, sorted, lane_id(), 32);
 }
 
 }  // namespace
@@ -504,7 +614,18 @@ __global__ void __launch_bounds__(MUT_BLOCK, 1)
     sn = grid_sync(M.mctl, gen, 0, SEL_Q1, M.timeout_ns);
     if (sn.ok && !*(volatile uint32_t *)&M.ctl->err) {
       for (uint32_t i = gw; i < sn.tiles; i += nw) relocate_chunk(M, M.reloc.chunks[i], C);
-      for (uint32_t i = gw; i < sn.cnt; i += nw) relocate_append(M, M.reloc.rec[i]);
+      for (uint32_t i = gw; i < sn.cnt; i += nw) finish_warp(M, M.reloc.rec[i], C);
+      const uint32_t wide = *(volatile uint32_t *)&M.mctl->q_count[2];
+      __shared__ uint32_t sm[4 * MUT_BLOCK / 32];
+      for (uint32_t i = blockIdx.x; i < wide; i += gridDim.x) {
+        const RelocRec rec = M.reloc.rec[M.reloc.wide[i]];
+        const Adj &A = M.adj[rec.dir];
+        const uint32_t srt = A.srt[rec.row];
+        const uint32_t sorted = srt - dead_slots(A, rec.old_off, srt);
+        __syncthreads();  // (before any warp clears bits)
+        compact_row<MUT_BLOCK>(M, rec, sm, C);
+        finish_row(M, rec, sorted, threadIdx.x, MUT_BLOCK);
+      }
     }
   }
   if (!sn.ok && threadIdx.x == 0) atomicCAS(&M.ctl->err, 0u, ERR_BARRIER);
