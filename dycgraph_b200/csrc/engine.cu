@@ -8,11 +8,14 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <fstream>
 #include <sstream>
+#include <system_error>
+#include <thread>
 #include <unordered_set>
 
 #include <fcntl.h>
@@ -34,6 +37,8 @@ namespace dycg {
 
 static u64 round_up(u64 x, u64 m) { return (x + m - 1) / m * m; }
 static void fill_phases(dycg_batch_stats *s, const Ctl &c);
+constexpr u64 FETCH_CHUNK = 1u << 20;  // bytes of one pinned chunk of the result ring
+constexpr u64 FETCH_THREADS = 6u << 20;  // results from which helper threads store them
 constexpr size_t CTL_CLEAR = 2 * sizeof(Ctl) + 64;  // control blocks and batch counters
 
 Engine::Engine(const dycg_options &opt) : opt_(opt) {
@@ -85,6 +90,8 @@ Engine::~Engine() {
   for (auto &e : ev_)
     if (e) cudaEventDestroy(e);
   for (auto &e : fev_)
+    if (e) cudaEventDestroy(e);
+  for (auto &e : fetch_ev_)
     if (e) cudaEventDestroy(e);
   if (fst_) cudaStreamDestroy(fst_);
   if (st_) cudaStreamDestroy(st_);
@@ -298,6 +305,13 @@ void Engine::finish_load() {
   CK(cudaHostAlloc(&hc, sizeof(Ctl), cudaHostAllocDefault));
   hallocs_.push_back(hc);
   h_ctl_ = (Ctl *)hc;
+  void *hr = nullptr;
+  fetch_slots_ = (uint32_t)std::min<u64>((2ull * n * 4 + FETCH_CHUNK - 1) / FETCH_CHUNK + 1, 8);
+  CK(cudaHostAlloc(&hr, (u64)fetch_slots_ * FETCH_CHUNK, cudaHostAllocMapped));
+  hallocs_.push_back(hr);
+  h_fetch_ = (char *)hr;
+  for (uint32_t i = 0; i < fetch_slots_; i++)
+    CK(cudaEventCreateWithFlags(&fetch_ev_[i], cudaEventDisableTiming));
   if (opt_.algo == DYCG_ALGO_PR) {
     x_ = (float *)dmalloc((n + 1ull) * 4);
     r_ = (float *)dmalloc((n + 1ull) * 4);
@@ -1196,14 +1210,105 @@ void Engine::gather_query(uint32_t q, uint32_t *values, uint32_t *parents) {
   check_loaded();
   if (!nq_) throw Error(DYCG_ESTATE, "no queries set");
   if (q >= nq_) throw Error(DYCG_EINVAL, "query index out of range");
+  if (qmode_ == DYCG_QUERIES_BATCHED) fetch_keys(qkey_, qnb_ * 32, q, values, parents);
+  else fetch_keys(qkey_ + (u64)q * n_, 0, 0, values, parents);
+}
+
+// ---- results to the host ----------------------------------------------------
+
+// Values and parents of n keys into the caller's arrays (either may be null),
+// split on the device.
+void Engine::fetch_keys(const u64 *key, uint32_t Q, uint32_t q, uint32_t *values,
+                        uint32_t *parents) {
+  const u64 bytes = (u64)n_ * 4;
+  if (2 * bytes <= FETCH_CHUNK) {
+    // a small result goes straight to the pinned buffer: one launch, one wait
+    uint32_t *hv = (uint32_t *)h_fetch_, *dv = nullptr;
+    CK(cudaHostGetDevicePointer((void **)&dv, h_fetch_, 0));
+    CK(launch_multi_gather(key, n_, Q, q, dv, dv + n_, st_));
+    sync_check("gather");
+    if (values) std::memcpy(values, hv, bytes);
+    if (parents) std::memcpy(parents, hv + n_, bytes);
+    return;
+  }
   // q0_/q1_ (n+1 entries each) are idle between calls: use them as staging
-  if (qmode_ == DYCG_QUERIES_BATCHED)
-    CK(launch_multi_gather(qkey_, n_, qnb_ * 32, q, q0_, q1_, st_));
-  else
-    CK(launch_multi_gather(qkey_ + (u64)q * n_, n_, 0, 0, q0_, q1_, st_));
-  if (values) CK(cudaMemcpyAsync(values, q0_, (u64)n_ * 4, cudaMemcpyDeviceToHost, st_));
-  if (parents) CK(cudaMemcpyAsync(parents, q1_, (u64)n_ * 4, cudaMemcpyDeviceToHost, st_));
-  sync_check("gather query");
+  CK(launch_multi_gather(key, n_, Q, q, q0_, q1_, st_));
+  fetch(q0_, values, q1_, parents, bytes);
+}
+
+// Two device arrays of `bytes` each into ordinary host memory (a null
+// destination is skipped), through a ring of pinned chunks: the copies run at
+// the link's rate (a copy to pageable memory goes through one driver thread's
+// staging), and helper threads empty the ring, since one thread's stores into
+// fresh pages reach a fraction of that rate. This thread alone talks to the
+// device: it announces a chunk when its copy has arrived and sends the next one
+// into a slot once the slot's last chunk has been stored. Below FETCH_THREADS
+// bytes the helpers' start costs more than they save.
+void Engine::fetch(const void *d0, void *h0, const void *d1, void *h1, u64 bytes) {
+  const u64 all = (h0 ? bytes : 0) + (h1 ? bytes : 0);
+  if (all < FETCH_THREADS) {
+    if (h0) CK(cudaMemcpyAsync(h0, d0, bytes, cudaMemcpyDeviceToHost, st_));
+    if (h1) CK(cudaMemcpyAsync(h1, d1, bytes, cudaMemcpyDeviceToHost, st_));
+    sync_check("fetch");
+    return;
+  }
+  struct Part {
+    const char *d;
+    char *h;
+    size_t n;
+  };
+  std::vector<Part> parts;
+  for (int k = 0; k < 2; k++) {
+    const char *d = (const char *)(k ? d1 : d0);
+    char *h = (char *)(k ? h1 : h0);
+    for (u64 o = 0; h && o < bytes; o += FETCH_CHUNK)
+      parts.push_back({d + o, h + o, (size_t)std::min<u64>(FETCH_CHUNK, bytes - o)});
+  }
+  const uint32_t slots = fetch_slots_, total = (uint32_t)parts.size();
+  std::atomic<uint32_t> arrived{0}, taken{0};
+  std::vector<std::atomic<uint8_t>> stored(total);
+  for (auto &s : stored) s.store(0, std::memory_order_relaxed);
+  auto store_one = [&]() {  // the next chunk that nobody has taken; false: none left
+    const uint32_t i = taken.fetch_add(1);
+    if (i >= total) return false;
+    while (arrived.load(std::memory_order_acquire) <= i) std::this_thread::yield();
+    if (arrived.load(std::memory_order_acquire) <= total)  // (above: the copies failed)
+      std::memcpy(parts[i].h, h_fetch_ + (u64)(i % slots) * FETCH_CHUNK, parts[i].n);
+    stored[i].store(1, std::memory_order_release);
+    return true;
+  };
+  auto send = [&](uint32_t i) {
+    cudaError_t x = cudaMemcpyAsync(h_fetch_ + (u64)(i % slots) * FETCH_CHUNK, parts[i].d,
+                                    parts[i].n, cudaMemcpyDeviceToHost, st_);
+    return x != cudaSuccess ? x : cudaEventRecord(fetch_ev_[i % slots], st_);
+  };
+  cudaError_t x = cudaSuccess;
+  for (uint32_t i = 0; i < std::min(slots, total) && x == cudaSuccess; i++) x = send(i);
+  std::vector<std::thread> crew;
+  try {
+    for (int t = 0; t < 3 && x == cudaSuccess; t++)
+      crew.emplace_back([&]() {
+        while (store_one()) {
+        }
+      });
+  } catch (const std::system_error &) {
+    // fewer helpers, or none: this thread stores what is left
+  }
+  for (uint32_t i = 0; i < total && x == cudaSuccess; i++) {
+    x = cudaEventSynchronize(fetch_ev_[i % slots]);
+    if (x != cudaSuccess) break;
+    arrived.store(i + 1, std::memory_order_release);
+    if (crew.empty()) store_one();
+    // slots freed meanwhile (in order) take the chunks that follow
+    if (i + slots < total) {
+      while (!stored[i].load(std::memory_order_acquire)) std::this_thread::yield();
+      x = send(i + slots);
+    }
+  }
+  if (x != cudaSuccess) arrived.store(total + 1, std::memory_order_release);
+  for (std::thread &t : crew) t.join();
+  cudaStreamSynchronize(st_);
+  CK(x);
 }
 
 // ---- mapping autotuner and multi-snapshot replay ------------------------------
@@ -1822,23 +1927,13 @@ void Engine::gather(uint32_t *values, uint32_t *parents) {
     gather_query(0, values, parents);
     return;
   }
-  std::vector<u64> k(n_);
-  CK(cudaMemcpyAsync(k.data(), key_, (u64)n_ * 8, cudaMemcpyDeviceToHost, st_));
-  sync_check("gather");
-  for (uint32_t v = 0; v < n_; v++) {
-    const uint32_t val = key_value(k[v]);
-    const uint32_t p1 = key_parent1(k[v]);
-    if (values) values[v] = val;
-    if (parents) parents[v] = (val == INF32 || p1 == 0) ? INF32 : p1 - 1;
-  }
+  fetch_keys(key_, 0, 0, values, parents);
 }
 
 void Engine::gather_ranks(float *ranks, float *residuals) {
   check_loaded();
   if (opt_.algo != DYCG_ALGO_PR) throw Error(DYCG_EINVAL, "not a PageRank engine");
-  if (ranks) CK(cudaMemcpyAsync(ranks, x_, (u64)n_ * 4, cudaMemcpyDeviceToHost, st_));
-  if (residuals) CK(cudaMemcpyAsync(residuals, r_, (u64)n_ * 4, cudaMemcpyDeviceToHost, st_));
-  sync_check("gather ranks");
+  fetch(x_, ranks, r_, residuals, (u64)n_ * 4);
 }
 
 // Host bitmap words covering slots [first, first + count) of arena A.

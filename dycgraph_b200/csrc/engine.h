@@ -119,6 +119,8 @@ class Engine {
   void init_queries(u64 timeout);
   void repair_queries(uint32_t phases, u64 timeout);
   MultiLaunch multi_launch(uint32_t phases, u64 timeout);
+  void fetch_keys(const u64 *key, uint32_t Q, uint32_t q, uint32_t *values, uint32_t *parents);
+  void fetch(const void *d0, void *h0, const void *d1, void *h1, u64 bytes);
   void *dmalloc(size_t bytes);
   void dfree_all();
 
@@ -152,6 +154,9 @@ class Engine {
   uint4 *tiles_ = nullptr;
   uint32_t tile_cap_ = 0;
   Ctl *ctl_ = nullptr, *mctl_ = nullptr, *h_ctl_ = nullptr;
+  char *h_fetch_ = nullptr;  // results' way to the host: ring of pinned chunks
+  uint32_t fetch_slots_ = 0;
+  cudaEvent_t fetch_ev_[8] = {};
   float *x_ = nullptr, *r_ = nullptr, *delta_ = nullptr;
   uint32_t *queued_ = nullptr;
   uint32_t pr_cur_ = 0, pr_count_ = 0;
