@@ -153,31 +153,43 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 
 // ---- inference on the 5th-generation tensor cores (tcgen05) ---------------------
 
-// A CTA of 4 warps serves 128 pages per tile: layer 1 and layer 2 are
-// tcgen05.mma products (M = 128 pages, N = 64 hidden units, K = 16 per
-// instruction, BF16 operands from shared memory, FP32 accumulators in tensor
-// memory), issued by one thread; each thread then reads its page's row of
-// the accumulator back with tcgen05.ld (warp w owns tensor-memory lanes
-// 32w..32w+31) for the bias / ReLU epilogue, the BF16 hi + lo split of the
-// layer-1 activations (both parts go through layer 2, so the activations keep
-// FP32-level precision: h = hi + lo to ~2^-17 relative, while a single BF16
-// rounding missed the float64 oracle's tolerance by 60-190x) and the final
-// FP32 dot product. Operands sit in shared
-// memory in the no-swizzle K-major layout of 8-row x 16-byte core matrices:
+// A warpgroup serves 128 pages per tile: layer 1 and layer 2 are tcgen05.mma
+// products (M = 128 pages, N = 64 hidden units, K = 16 per instruction, BF16
+// operands, FP32 accumulators in tensor memory), issued by one thread; each
+// thread then reads its page's row of the accumulator back with tcgen05.ld (warp
+// w of the group owns tensor-memory lanes 32w..32w+31) for the epilogues: ReLU
+// and the BF16 hi + lo split of the layer-1 activations (both parts go through
+// layer 2, so the activations keep FP32-level precision: h = hi + lo to ~2^-17
+// relative, while a single BF16 rounding missed the float64 oracle's tolerance by
+// 60-190x), then bias, ReLU and the final FP32 dot product. Layer 1's bias is a
+// weight row on a constant input column (K is padded from 8 to 16 anyway).
+// What bounds it is the epilogues: their issue slots (~450 instructions per page
+// row) and, with the A operands in shared memory, its bandwidth (32 KB stored and
+// 48 KB read by the MMAs per tile); HBM's share is 6 us of 1.85M pages, the MMAs'
+// ~15. So the A operands stay in tensor memory (tcgen05.st, two BF16 per 32-bit
+// column, lane = row), FP32 sums and products come two per instruction (f32x2),
+// the split takes packed conversions, and one CTA of four independent warpgroups
+// per SM (128 of the 512 columns each) shares the weights and covers each
+// other's load, MMA and barrier latencies. 1.85M pages: 104 us with scalar
+// epilogues and A in shared memory, 77 now (half the issue slots; the rest is the
+// chain load - MMA - epilogue - MMA - epilogue of the four groups in flight).
+// The weights sit in shared memory in the no-swizzle K-major layout of 8-row x
+// 16-byte core matrices:
 // element (row, k) of an operand with KC chunks of 8 along K lives at
 // ((row / 8) * KC + k / 8) * 128 + (row % 8) * 16 + (k % 8) * 2 bytes, so the
 // descriptor's leading byte offset (next core matrix along K) is 128 and its
 // stride byte offset (next 8 rows) is KC * 128.
 namespace tc {
 constexpr uint32_t M = 128, N = 64;
-constexpr uint32_t SM_A1 = 0;                  // 128 x 16 (KC 2): 4 KB
-constexpr uint32_t SM_B1 = SM_A1 + 4096;       // 64 x 16 (KC 2): 2 KB
-constexpr uint32_t SM_A2H = SM_B1 + 2048;      // 128 x 64 (KC 8): 16 KB
-constexpr uint32_t SM_A2L = SM_A2H + 16384;    // 16 KB
-constexpr uint32_t SM_B2 = SM_A2L + 16384;     // 64 x 64 (KC 8): 8 KB
-constexpr uint32_t SM_BIAS = SM_B2 + 8192;     // b1, b2, W3 (BF16-rounded, FP32): 768 B
-constexpr uint32_t SM_BAR = SM_BIAS + 768;     // mbarrier (8 B) + tensor-memory address (4 B)
-constexpr uint32_t SM_BYTES = SM_BAR + 16;
+constexpr uint32_t GROUPS = 4;                 // warpgroups per CTA
+constexpr uint32_t SM_B1 = 0;                  // 64 x 16 (KC 2): 2 KB
+constexpr uint32_t SM_B2 = SM_B1 + 2048;       // 64 x 64 (KC 8): 8 KB
+constexpr uint32_t SM_BIAS = SM_B2 + 8192;     // b2, W3 (BF16-rounded, FP32): 512 B
+constexpr uint32_t SM_BAR = SM_BIAS + 512;     // mbarriers (8 B each), tensor-memory address
+constexpr uint32_t SM_BYTES = SM_BAR + 8 * GROUPS + 16;
+// a group's tensor-memory columns: accumulator 0..63 (both layers in turn), A
+// operand 64..127 (layer 1's 8 columns, then layer 2's hi and lo, 32 each)
+constexpr uint32_t T_A = 64, T_LO = 32, T_GROUP = 128;
 // idesc: D FP32 (bits 4-5 = 1), A and B BF16 (bits 7-9, 10-12 = 1), both
 // K-major, N >> 3 in bits 17-22, M >> 4 in bits 24-28
 constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
@@ -200,16 +212,44 @@ __device__ __forceinline__ void mma(uint32_t d_tmem, u64 a, u64 b, uint32_t accu
       :
       : "r"(d_tmem), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(0u));
 }
+// the same with A in tensor memory
+__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, u64 b,
+                                       uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}\n"
+      :
+      : "r"(d_tmem), "r"(a_tmem), "l"(b), "r"(IDESC), "r"(accumulate), "r"(0u));
+}
+// 8 / 16 32-bit columns of this thread's tensor-memory lane (warp-collective)
+__device__ __forceinline__ void st8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};\n"
+               :
+               : "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
+                 "r"(r[7]), "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, "
+      "%10, %11, %12, %13, %14, %15};\n"
+      :
+      : "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]),
+        "r"(r[15]), "r"(taddr)
+      : "memory");
+}
 __device__ __forceinline__ void commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
                :
                : "r"(bar)
                : "memory");
 }
-// bounded wait on the mbarrier's phase; false when the limit ran out
+// bounded wait on the mbarrier's phase; false when the limit ran out (the timer
+// is looked at only by waits that outlast 64 attempts)
 __device__ __forceinline__ bool wait(uint32_t bar, uint32_t phase) {
-  const u64 t0 = globaltimer_ns();
-  for (;;) {
+  u64 t0 = 0;
+  for (uint32_t tries = 1;; tries++) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred P1;\n\tmbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
@@ -218,7 +258,10 @@ __device__ __forceinline__ bool wait(uint32_t bar, uint32_t phase) {
         : "r"(bar), "r"(phase)
         : "memory");
     if (done) return true;
-    if (globaltimer_ns() - t0 > 1000000000ull) return false;
+    if (tries % 64) continue;
+    const u64 t = globaltimer_ns();
+    if (!t0) t0 = t;
+    else if (t - t0 > 1000000000ull) return false;
   }
 }
 // 32 FP32 columns of this thread's tensor-memory lane (warp-collective)
@@ -238,10 +281,29 @@ __device__ __forceinline__ void ld32(uint32_t taddr, float *v) {
 #pragma unroll
   for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
 }
-// 64 FP32 columns of this thread's tensor-memory lane, in two 32-column loads
+// 64 FP32 columns of this thread's tensor-memory lane (one load, one wait)
 __device__ __forceinline__ void ld64(uint32_t taddr, float (&v)[64]) {
-  ld32(taddr, v);
-  ld32(taddr + 32, v + 32);
+  uint32_t r[64];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x64.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, "
+      "%32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, "
+      "%48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%64];\n"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
+        "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
+        "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]),
+        "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]),
+        "=r"(r[30]), "=r"(r[31]), "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]),
+        "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]), "=r"(r[40]), "=r"(r[41]),
+        "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47]),
+        "=r"(r[48]), "=r"(r[49]), "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]),
+        "=r"(r[54]), "=r"(r[55]), "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]),
+        "=r"(r[60]), "=r"(r[61]), "=r"(r[62]), "=r"(r[63])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 64; i++) v[i] = __uint_as_float(r[i]);
 }
 __device__ __forceinline__ void fence_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -254,122 +316,177 @@ __device__ __forceinline__ void fence_after() {
 }
 }  // namespace tc
 
-__global__ void __launch_bounds__(128, 4) mlp_infer_tc_kernel(const __nv_bfloat16 *x, uint32_t n,
-                                                              const float *params, float *score,
-                                                              uint32_t *ids, uint32_t *err) {
+// Two FP32 operations per instruction (sm_100's packed FP32 pipe).
+__device__ __forceinline__ u64 pk(float a, float b) {
+  return ((u64)__float_as_uint(b) << 32) | __float_as_uint(a);
+}
+__device__ __forceinline__ u64 add2(u64 a, u64 b) {
+  u64 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
+  u64 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ float lo32(u64 x) { return __uint_as_float((uint32_t)x); }
+__device__ __forceinline__ float hi32(u64 x) { return __uint_as_float((uint32_t)(x >> 32)); }
+// relu(a), relu(b) as packed BF16 hi parts, and what they leave as packed lo parts
+__device__ __forceinline__ void split_relu(float a, float b, uint32_t &hi, uint32_t &lo) {
+  a = fmaxf(a, 0.f);
+  b = fmaxf(b, 0.f);
+  hi = pack2(a, b);
+  const u64 h = pk(__uint_as_float(hi << 16), __uint_as_float(hi & 0xFFFF0000u));
+  const u64 rest = fma2(h, pk(-1.f, -1.f), pk(a, b));  // exact: h has a's leading bits
+  lo = pack2(lo32(rest), hi32(rest));
+}
+
+__global__ void __launch_bounds__(128 * tc::GROUPS, 1)
+    mlp_infer_tc_kernel(const __nv_bfloat16 *x, uint32_t n, const float *params, float *score,
+                        uint32_t *ids, uint32_t *err) {
   extern __shared__ __align__(1024) uint8_t sm_tc[];
-  const uint32_t tid = threadIdx.x, warp = tid >> 5;
+  const uint32_t tid = threadIdx.x & 127, group = threadIdx.x >> 7, warp = threadIdx.x >> 5;
   const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(sm_tc);
-  const uint32_t bar = sbase + tc::SM_BAR;
-  uint32_t *taddr_slot = reinterpret_cast<uint32_t *>(sm_tc + tc::SM_BAR + 8);
-  // the weights as the B operands (N = hidden unit, K = input), BF16; the
-  // padding columns 8..15 of layer 1 are zero; biases and W3 in registers
-  for (uint32_t i = tid; i < tc::N * 16; i += blockDim.x) {
-    const uint32_t nn = i / 16, k = i % 16;
-    const float wv = k < (uint32_t)F ? params[OFF_W1 + k * H + nn] : 0.f;
-    *reinterpret_cast<__nv_bfloat16 *>(sm_tc + tc::SM_B1 + tc::off(nn, k, 2)) = __float2bfloat16_rn(wv);
+  const uint32_t bar = sbase + tc::SM_BAR + 8 * group;
+  uint32_t *taddr_slot = reinterpret_cast<uint32_t *>(sm_tc + tc::SM_BAR + 8 * tc::GROUPS);
+  // the weights as the B operands (N = hidden unit, K = input), BF16; layer 1's
+  // row 8 is its bias, rows 9..15 are zero. All loads first: one latency.
+  {
+    constexpr uint32_t T = 128 * tc::GROUPS;
+    float w1[tc::N * 16 / T], w2[tc::N * H / T];
+#pragma unroll
+    for (uint32_t u = 0; u < tc::N * 16 / T; u++) {
+      const uint32_t i = u * T + threadIdx.x, k = i / tc::N, nn = i % tc::N;
+      w1[u] = k < (uint32_t)F ? params[OFF_W1 + k * H + nn]
+                              : k == (uint32_t)F ? params[OFF_B1 + nn] : 0.f;
+    }
+#pragma unroll
+    for (uint32_t u = 0; u < tc::N * H / T; u++) w2[u] = params[OFF_W2 + u * T + threadIdx.x];
+    float *bias = reinterpret_cast<float *>(sm_tc + tc::SM_BIAS);  // b2[64], W3[64]
+    if (threadIdx.x < 2 * H)
+      bias[threadIdx.x] = bf(params[(threadIdx.x < H ? OFF_B2 : OFF_W3 - H) + threadIdx.x]);
+#pragma unroll
+    for (uint32_t u = 0; u < tc::N * 16 / T; u++) {
+      const uint32_t i = u * T + threadIdx.x, k = i / tc::N, nn = i % tc::N;
+      *reinterpret_cast<__nv_bfloat16 *>(sm_tc + tc::SM_B1 + tc::off(nn, k, 2)) =
+          __float2bfloat16_rn(w1[u]);
+    }
+#pragma unroll
+    for (uint32_t u = 0; u < tc::N * H / T; u++) {
+      const uint32_t i = u * T + threadIdx.x, k = i / tc::N, nn = i % tc::N;
+      *reinterpret_cast<__nv_bfloat16 *>(sm_tc + tc::SM_B2 + tc::off(nn, k, 8)) =
+          __float2bfloat16_rn(w2[u]);
+    }
   }
-  for (uint32_t i = tid; i < tc::N * (uint32_t)H; i += blockDim.x) {
-    const uint32_t nn = i / H, k = i % H;
-    *reinterpret_cast<__nv_bfloat16 *>(sm_tc + tc::SM_B2 + tc::off(nn, k, 8)) =
-        __float2bfloat16_rn(params[OFF_W2 + k * H + nn]);
-  }
-  float *bias = reinterpret_cast<float *>(sm_tc + tc::SM_BIAS);  // b1[64], b2[64], W3[64]
-  for (uint32_t i = tid; i < 3 * (uint32_t)H; i += blockDim.x)
-    bias[i] = bf(params[(i < (uint32_t)H ? OFF_B1 : i < 2u * H ? OFF_B2 - H : OFF_W3 - 2 * H) + i]);
+  const float *bias = reinterpret_cast<const float *>(sm_tc + tc::SM_BIAS);
   if (tid == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 0) {  // 128 tensor-memory columns: layer 1 in 0..63, layer 2 in 64..127
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 128;" ::"r"(
-        sbase + tc::SM_BAR + 8));
+  if (warp == 0) {  // all 512 tensor-memory columns
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
+        sbase + tc::SM_BAR + 8 * tc::GROUPS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   tc::fence_async_smem();
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
-  const uint32_t tmem = *taddr_slot;
-  const uint32_t lane_base = (32 * warp) << 16;  // this warp's tensor-memory lanes
+  const uint32_t tmem_base = *taddr_slot;
+  const uint32_t tmem = tmem_base + tc::T_GROUP * group;
+  const uint32_t mine = tmem + ((32 * (warp & 3)) << 16);  // this warp's lanes
   const float b3 = bf(params[OFF_B3]);
   uint32_t phase = 0;
   bool ok = true;
-  const uint32_t tiles = (n + tc::M - 1) / tc::M;
-  for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-    const uint32_t row = tile * tc::M + tid;
-    // A1: this page's 8 BF16 features, zero padding to K = 16
-    {
-      uint4 f = make_uint4(0, 0, 0, 0);
-      if (row < n) f = __ldg(reinterpret_cast<const uint4 *>(x) + row);
-      *reinterpret_cast<uint4 *>(sm_tc + tc::SM_A1 + tc::off(tid, 0, 2)) = f;
-      *reinterpret_cast<uint4 *>(sm_tc + tc::SM_A1 + tc::off(tid, 8, 2)) = make_uint4(0, 0, 0, 0);
-    }
-    tc::fence_async_smem();
+  // the group's operand stores and accumulator reads done; true when no
+  // thread's wait ran out
+  const auto publish = [&]() {
+    uint32_t all;
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     tc::fence_before();
-    __syncthreads();
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %2, 0;\n\t"
+        "barrier.cta.red.and.pred q, %1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(all)
+        : "r"(group + 1), "r"((uint32_t)ok)
+        : "memory");
     tc::fence_after();
+    return all != 0;
+  };
+  const uint32_t tiles = (n + tc::M - 1) / tc::M, step = gridDim.x * tc::GROUPS;
+  uint32_t tile = group * gridDim.x + blockIdx.x;
+  const auto load = [&](uint32_t t) {  // this page's 8 BF16 features
+    const u64 row = (u64)t * tc::M + tid;
+    return row < n ? __ldg(reinterpret_cast<const uint4 *>(x) + row) : make_uint4(0, 0, 0, 0);
+  };
+  uint4 f = load(tile);
+  for (; tile < tiles; tile += step) {
+    const uint32_t row = tile * tc::M + tid;
+    {
+      const uint32_t a[8] = {f.x, f.y, f.z, f.w, 0x3F80u, 0, 0, 0};  // features, 1, 0, ..
+      tc::st8(mine + tc::T_A, a);
+    }
+    f = load(tile + step);
+    ok = publish();
+    if (!ok) break;
     if (tid == 0) {
-      tc::mma(tmem, tc::sdesc(sbase + tc::SM_A1, 256), tc::sdesc(sbase + tc::SM_B1, 256), 0);
+      tc::mma_ts(tmem, tmem + tc::T_A, tc::sdesc(sbase + tc::SM_B1, 256), 0);
       tc::commit(bar);
     }
     ok = tc::wait(bar, phase);
     phase ^= 1;
     tc::fence_after();
+    // layer-1 epilogue: ReLU, BF16 hi + lo parts as the A operands of layer 2
     float v[64];
-    tc::ld64(tmem + lane_base, v);
-    // layer-1 epilogue: bias, ReLU, BF16 hi + lo parts as the A operands of layer 2
+    tc::ld64(mine, v);
 #pragma unroll
-    for (int h = 0; h < H; h += 8) {
-      uint32_t hw[4], lw[4];
+    for (uint32_t c = 0; c < (uint32_t)H; c += 32) {
+      uint32_t hw[16], lw[16];
 #pragma unroll
-      for (int e = 0; e < 8; e += 2) {
-        const float a0 = fmaxf(v[h + e] + bias[h + e], 0.f);
-        const float a1 = fmaxf(v[h + e + 1] + bias[h + e + 1], 0.f);
-        const float h0 = bf(a0), h1 = bf(a1);
-        hw[e / 2] = pack2(h0, h1);
-        lw[e / 2] = pack2(a0 - h0, a1 - h1);
-      }
-      *reinterpret_cast<uint4 *>(sm_tc + tc::SM_A2H + tc::off(tid, h, 8)) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-      *reinterpret_cast<uint4 *>(sm_tc + tc::SM_A2L + tc::off(tid, h, 8)) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+      for (int e = 0; e < 16; e++) split_relu(v[c + 2 * e], v[c + 2 * e + 1], hw[e], lw[e]);
+      tc::st16(mine + tc::T_A + c / 2, hw);
+      tc::st16(mine + tc::T_A + tc::T_LO + c / 2, lw);
     }
-    tc::fence_async_smem();
-    tc::fence_before();
-    __syncthreads();
-    tc::fence_after();
-    if (tid == 0 && ok) {
+    ok = publish();
+    if (!ok) break;
+    if (tid == 0) {
 #pragma unroll
       for (uint32_t s = 0; s < (uint32_t)H / 16; s++) {
-        const uint32_t kb = s * 256;  // 16 K-elements = two core matrices along K
-        tc::mma(tmem + tc::N, tc::sdesc(sbase + tc::SM_A2H + kb, 1024),
-                tc::sdesc(sbase + tc::SM_B2 + kb, 1024), s > 0);
-        tc::mma(tmem + tc::N, tc::sdesc(sbase + tc::SM_A2L + kb, 1024),
-                tc::sdesc(sbase + tc::SM_B2 + kb, 1024), 1);
+        // 16 K-elements: 8 columns of A, two core matrices of B
+        const u64 b = tc::sdesc(sbase + tc::SM_B2 + s * 256, 1024);
+        tc::mma_ts(tmem, tmem + tc::T_A + 8 * s, b, s > 0);
+        tc::mma_ts(tmem, tmem + tc::T_A + tc::T_LO + 8 * s, b, 1);
       }
       tc::commit(bar);
     }
-    if (ok) ok = tc::wait(bar, phase);
+    ok = tc::wait(bar, phase);
     phase ^= 1;
     tc::fence_after();
-    tc::ld64(tmem + lane_base + tc::N, v);
-    float y = 0.f;
+    u64 y = 0;  // even and odd units' sums
+    tc::ld64(mine, v);
+    {
 #pragma unroll
-    for (int h = 0; h < H; h++)
-      y = fmaf(fmaxf(v[h] + bias[H + h], 0.f), bias[2 * H + h], y);
+      for (int h = 0; h < H; h += 4) {
+        const float4 b = *reinterpret_cast<const float4 *>(bias + h);
+        const float4 w = *reinterpret_cast<const float4 *>(bias + H + h);
+        const u64 p = add2(pk(v[h], v[h + 1]), pk(b.x, b.y));
+        const u64 q = add2(pk(v[h + 2], v[h + 3]), pk(b.z, b.w));
+        y = fma2(pk(fmaxf(lo32(p), 0.f), fmaxf(hi32(p), 0.f)), pk(w.x, w.y), y);
+        y = fma2(pk(fmaxf(lo32(q), 0.f), fmaxf(hi32(q), 0.f)), pk(w.z, w.w), y);
+      }
+    }
     if (row < n) {
-      score[row] = y + b3;
+      score[row] = lo32(y) + hi32(y) + b3;
       if (ids) ids[row] = row;
     }
-    tc::fence_before();
-    __syncthreads();  // every lane's reads of the accumulators are done before the next tile
-    tc::fence_after();
   }
-  if (!ok && err && tid == 0) atomicCAS(err, 0u, ERR_BARRIER);
+  if (!ok && err) atomicCAS(err, 0u, ERR_BARRIER);
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
   if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 128;" ::"r"(tmem));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_base));
 }
 
 // ---- training on the 5th-generation tensor cores ----------------------------------
@@ -467,18 +584,27 @@ __global__ void __launch_bounds__(128, 1)
   const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(sm);
   const uint32_t bar = sbase + tt::SM_BAR;
   uint32_t *taddr_slot = reinterpret_cast<uint32_t *>(sm + tt::SM_BAR + 8);
+  float w1[4], w2[32];
+#pragma unroll
+  for (uint32_t u = 0; u < 4; u++) w1[u] = params[OFF_W1 + u * 128 + t];
+#pragma unroll
+  for (uint32_t u = 0; u < 32; u++) w2[u] = params[OFF_W2 + u * 128 + t];
   // operands that do not change: zeros everywhere (padding rows and columns,
   // the lo parts of exact values), the weights, the two rows of ones
   for (uint32_t i = t * 16; i < tt::SM_BIAS; i += 128 * 16)
     *reinterpret_cast<uint4 *>(sm + i) = make_uint4(0, 0, 0, 0);
   __syncthreads();
-  for (uint32_t i = t; i < 64 * (uint32_t)F; i += 128) {
-    const uint32_t nn = i / F, k = i % F;
-    tt::put(sm, tt::SM_B1, nn, k, 2, __float2bfloat16_rn(params[OFF_W1 + k * H + nn]));
+  // (loaded ahead of the zeroing, all at once: a minibatch's launch is a tile or
+  // two per CTA, and its prologue's dependent loads cost as much as the tile)
+#pragma unroll
+  for (uint32_t u = 0; u < 4; u++) {
+    const uint32_t i = u * 128 + t, k = i / H, nn = i % H;
+    tt::put(sm, tt::SM_B1, nn, k, 2, __float2bfloat16_rn(w1[u]));
   }
-  for (uint32_t i = t; i < (uint32_t)(H * H); i += 128) {
-    const uint32_t a = i / H, b = i % H;  // W2[a][b]: input a, output b
-    const __nv_bfloat16 w = __float2bfloat16_rn(params[OFF_W2 + i]);
+#pragma unroll
+  for (uint32_t u = 0; u < 32; u++) {
+    const uint32_t i = u * 128 + t, a = i / H, b = i % H;  // W2[a][b]: input a, output b
+    const __nv_bfloat16 w = __float2bfloat16_rn(w2[u]);
     tt::put(sm, tt::SM_B2F, b, a, 8, w);
     tt::put(sm, tt::SM_B2B, a, b, 8, w);
   }
@@ -745,14 +871,15 @@ cudaError_t launch_log1p(const float *in, float *out, u64 n, cudaStream_t s) {
 cudaError_t launch_mlp_infer(const void *x, uint32_t n, const float *params, float *score,
                              uint32_t *ids, uint32_t *err, cudaStream_t s) {
   if (!n) return cudaSuccess;
+  // one CTA per SM; a small launch spreads its tiles over the SMs before a second
+  // warpgroup of any CTA gets one
   const uint32_t tiles = (n + tc::M - 1) / tc::M;
-  // up to 4 CTAs per SM (4 x 128 tensor-memory columns = all 512), so an SM
-  // overlaps the MMA and epilogue latencies of four tiles
-  const int grid = (int)std::min<uint32_t>(tiles, 148u * 4);
-  mlp_infer_tc_kernel<<<grid, 128, tc::SM_BYTES, s>>>((const __nv_bfloat16 *)x, n, params, score,
-                                                      ids, err);
+  const int grid = (int)std::min<uint32_t>(tiles, 148u);
+  mlp_infer_tc_kernel<<<grid, 128 * tc::GROUPS, tc::SM_BYTES, s>>>(
+      (const __nv_bfloat16 *)x, n, params, score, ids, err);
   return cudaGetLastError();
 }
+
 cudaError_t launch_mlp_grad(const void *x, const float *y, uint64_t total, uint32_t count,
                             uint64_t sample_seed, const float *params, float scale, float *grad,
                             float *loss, uint32_t *err, cudaStream_t s) {
