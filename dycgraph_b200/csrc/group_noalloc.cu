@@ -33,7 +33,7 @@ constexpr uint32_t kMax = DYCG_GROUP_NOALLOC_MAX_RECORDS;
 constexpr size_t kTemp = 4u << 20;  // CUB sort/scan temporary storage
 constexpr size_t kUp8 = ((size_t)kMax * 8 + 255) & ~(size_t)255;
 constexpr size_t kUp4 = ((size_t)kMax * 4 + 255) & ~(size_t)255;
-constexpr size_t kBytes = 256 + 2 * kUp8 + 3 * kUp4 + kTemp;
+constexpr size_t kBytes = 256 + 2 * kUp8 + 2 * kUp4 + kTemp;
 
 __device__ __align__(256) unsigned char g_group_scratch[kBytes];
 
