@@ -126,7 +126,7 @@ int dycg_insert_edges(dycg_engine *e, const dycg_edge *adds, size_t na, dycg_bat
 }
 
 int dycg_cache_maintenance(dycg_engine *e, dycg_batch_stats *stats) {
-  return guard(e, [&](Engine &g) { g.cache_maintenance(false, stats); });
+  return guard(e, [&](Engine &g) { g.maintain(stats); });
 }
 
 int dycg_reserve_batch(dycg_engine *e, size_t max_records) {

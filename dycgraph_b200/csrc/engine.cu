@@ -535,7 +535,9 @@ void Engine::init() {
   if (nq_) {
     init_queries(timeout);
     inited_ = true;
-    cache_maintenance(true, nullptr);
+    cache_maintenance(true);
+  sync_check("first cache load");
+  maintenance_stats(nullptr);
     return;
   }
   if (opt_.algo == DYCG_ALGO_PR) {
@@ -605,7 +607,9 @@ void Engine::init() {
     pr_count_ = h_ctl_->pad[1];
   }
   inited_ = true;
-  cache_maintenance(true, nullptr);
+  cache_maintenance(true);
+  sync_check("first cache load");
+  maintenance_stats(nullptr);
 }
 
 void Engine::reserve_batch(size_t max_records) {
@@ -869,6 +873,8 @@ void Engine::apply(const dycg_edge *dels, size_t nd, const dycg_edge *adds, size
       CK(cudaMemcpyAsync(h_qctl_, qctl_, (u64)nq_ * sizeof(Ctl), cudaMemcpyDeviceToHost, st_));
     CK(cudaMemcpyAsync(h_seq_, seq_, 8, cudaMemcpyDeviceToHost, st_));
   }
+  // the maintenance needs nothing of this from the host: one wait for both
+  if (maintenance) cache_maintenance(false);
   sync_check("batch");
   Ctl c = *h_ctl_;
   if (nq_ && qmode_ == DYCG_QUERIES_PER_QUERY) {
@@ -929,7 +935,7 @@ void Engine::apply(const dycg_edge *dels, size_t nd, const dycg_edge *adds, size
       stats->ms_repair -= pm;
     }
   }
-  if (maintenance) cache_maintenance(false, stats);
+  if (maintenance) maintenance_stats(stats);
   if (stats) {
     stats->kernel_launches = launches_ - l0;
     float tot = 0;
@@ -1808,7 +1814,9 @@ void Engine::sample_row_edges(const uint32_t *sources, uint64_t count, uint64_t 
   CK(e);
 }
 
-void Engine::cache_maintenance(bool initial, dycg_batch_stats *stats) {
+// Queues the cache maintenance of a snapshot (asynchronous); its counters are
+// read by maintenance_stats after a synchronisation.
+void Engine::cache_maintenance(bool initial) {
   check_loaded();
   if (feat_ && !initial) {
     // page-read history for the learned policy; this snapshot's reads go into
@@ -1835,23 +1843,10 @@ void Engine::cache_maintenance(bool initial, dycg_batch_stats *stats) {
   if (policy_ == DYCG_CACHE_LEARNED && !initial) {
     // admission ran before the repair (policy_prefetch); the call ends here
     CK(cudaEventRecord(ev_[5], st_));
-    if (prefetched_ && stats) {
+    if (prefetched_)
       CK(cudaMemcpyAsync(cwk_.h_plan, cwk_.plan, sizeof(CachePlan), cudaMemcpyDeviceToHost, st_));
-      sync_check("learned maintenance");
-      float ms = 0;
-      cudaEventElapsedTime(&ms, pev_[0], pev_[1]);
-      stats->ms_cache = ms;
-      const CachePlan &pl = *cwk_.h_plan;
-      stats->cache_pages_loaded = pl.admit;
-      stats->cache_pages_evicted = pl.evict;
-      const u64 page_bytes = (4ull << page_shift_) * out_.stride;
-      stats->link_bytes += (u64)pl.admit * page_bytes;
-      stats->hbm_adj_bytes += (u64)pl.admit * page_bytes;
-    }
-    prefetched_ = false;
     return;
   }
-  prefetched_ = false;
   if (!cache_slots_) {
     CK(cudaMemsetAsync(page_hits_, 0, (u64)npages_ * 4, st_));
     return;
@@ -1862,18 +1857,29 @@ void Engine::cache_maintenance(bool initial, dycg_batch_stats *stats) {
   hotness_round(initial, !initial);
   CK(cudaEventRecord(ev_[5], st_));
   CK(cudaMemcpyAsync(cwk_.h_plan, cwk_.plan, sizeof(CachePlan), cudaMemcpyDeviceToHost, st_));
-  sync_check("cache apply");
-  if (stats) {
-    float ms = 0;
-    cudaEventElapsedTime(&ms, ev_[4], ev_[5]);
-    const CachePlan &pl = *cwk_.h_plan;
-    stats->ms_cache = ms;
-    stats->cache_pages_loaded = pl.admit;
-    stats->cache_pages_evicted = pl.evict;
-    const u64 page_bytes = (4ull << page_shift_) * out_.stride;
-    stats->link_bytes += (u64)pl.admit * page_bytes;
-    stats->hbm_adj_bytes += (u64)pl.admit * page_bytes;
-  }
+  planned_ = true;
+}
+
+void Engine::maintain(dycg_batch_stats *stats) {
+  cache_maintenance(false);
+  sync_check("cache maintenance");
+  maintenance_stats(stats);
+}
+
+void Engine::maintenance_stats(dycg_batch_stats *stats) {
+  const bool learned = prefetched_, hot = planned_;
+  prefetched_ = planned_ = false;
+  if (!stats || !(hot || (learned && policy_ == DYCG_CACHE_LEARNED))) return;
+  float ms = 0;
+  if (hot) cudaEventElapsedTime(&ms, ev_[4], ev_[5]);
+  else cudaEventElapsedTime(&ms, pev_[0], pev_[1]);
+  const CachePlan &pl = *cwk_.h_plan;
+  stats->ms_cache = ms;
+  stats->cache_pages_loaded = pl.admit;
+  stats->cache_pages_evicted = pl.evict;
+  const u64 page_bytes = (4ull << page_shift_) * out_.stride;
+  stats->link_bytes += (u64)pl.admit * page_bytes;
+  stats->hbm_adj_bytes += (u64)pl.admit * page_bytes;
 }
 
 // One hotness round on the device: decayed page scores, top-K ranking, the

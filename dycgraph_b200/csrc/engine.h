@@ -58,7 +58,7 @@ class Engine {
   // mode: 0 fused batch, 1 deletions only, 2 insertions only
   void apply(const dycg_edge *dels, size_t nd, const dycg_edge *adds, size_t na, bool device_ptrs,
              int mode, bool maintenance, dycg_batch_stats *stats);
-  void cache_maintenance(bool initial, dycg_batch_stats *stats);
+  void maintain(dycg_batch_stats *stats);
   void reserve_batch(size_t max_records);
   void gather(uint32_t *values, uint32_t *parents);
   void gather_ranks(float *ranks, float *residuals);
@@ -116,6 +116,8 @@ class Engine {
   void hotness_round(bool initial, bool side = false);
   void join_staging();
   void maintenance_device();
+  void cache_maintenance(bool initial);
+  void maintenance_stats(dycg_batch_stats *stats);
   void init_queries(u64 timeout);
   void repair_queries(uint32_t phases, u64 timeout);
   MultiLaunch multi_launch(uint32_t phases, u64 timeout);
@@ -202,7 +204,7 @@ class Engine {
   void *tx_ = nullptr;
   float *ty_ = nullptr;
   uint32_t trace_cap_ = 0, trace_n_ = 0, trace_post_ = 0;
-  bool trace_pending_ = false, prefetched_ = false;
+  bool trace_pending_ = false, prefetched_ = false, planned_ = false;
   uint32_t learned_cap_div_ = 256;
   uint32_t *pperiod_ = nullptr;  // device {snapshot counter, refresh period} of the layout features
   cudaEvent_t pev_[2] = {};

@@ -245,6 +245,12 @@ __device__ void suffix_chunk(const MutParams &M, uint32_t c, Counts &C) {
   const Adj &A = M.adj[dir];
   const Rec *list = M.dels[dir];
   const uint32_t lane = lane_id();
+  // nothing left to look for: the records were found in the prefix (their
+  // remainders are in HBM, the suffix is across the link)
+  bool wanted = false;
+  for (uint32_t i = ch.x + lane; i < ch.y && !wanted; i += 32)
+    wanted = list[i].w && M.rem[dir][i];
+  if (!__any_sync(0xffffffffu, wanted)) return;
   const uint32_t row = list[ch.x].x;
   const u64 off = A.off[row];
   const uint32_t srt = A.srt[row], len = A.len[row];
