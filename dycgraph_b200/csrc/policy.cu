@@ -746,33 +746,34 @@ __global__ void __launch_bounds__(128, 1)
     phase ^= 1;
     tc::fence_after();
   }
-  // G's rows to the gradient: warps 0-1 hold dW2, warp 2 dW1, the biases, dW3
-  if (ok && done) {
-    float g[32];
-    if (warp < 2) {
+  // G's rows to the gradient: warps 0-1 hold dW2, warp 2 dW1, the biases, dW3.
+  // Per 32 columns a lane has one destination or none (a test per element and
+  // a fully unrolled walk over all columns took half of a one-tile launch, most
+  // of it in instruction fetches)
+  if (ok && done && warp < 3) {
+    const bool wide = (reinterpret_cast<uintptr_t>(grad) & 15) == 0;
+#pragma unroll 1
+    for (uint32_t c = 0; c < (warp < 2 ? 64u : 224u); c += 32) {
+      float g[32];
+      tc::ld32(tmem + lane_base + tt::T_G + c, g);  // (columns 208.. unused)
+      float *to = nullptr;
+      if (warp < 2) to = grad + OFF_W2 + t * H + c;
+      else if (c < tt::B_DH1) to = t == tt::A_ONE ? grad + OFF_B2 + c : nullptr;
+      else if (c < tt::B_H2)
+        to = t >= tt::A_X && t < tt::A_X + F ? grad + OFF_W1 + (t - tt::A_X) * H + c - tt::B_DH1
+             : t == tt::A_ONE                ? grad + OFF_B1 + c - tt::B_DH1
+                                             : nullptr;
+      else if (c < tt::B_ONE) to = t == tt::A_DY ? grad + OFF_W3 + c - tt::B_H2 : nullptr;
+      if (c == tt::B_ONE) {
+        if (t == tt::A_DY) atomicAdd(grad + OFF_B3, g[0]);
+      } else if (to && wide) {  // every parameter block starts at a multiple of four
 #pragma unroll
-      for (uint32_t c = 0; c < 64; c += 32) {
-        tc::ld32(tmem + lane_base + tt::T_G + tt::B_DH2 + c, g);
+        for (int j = 0; j < 32; j += 4)
+          atomicAdd(reinterpret_cast<float4 *>(to + j),
+                    make_float4(g[j], g[j + 1], g[j + 2], g[j + 3]));
+      } else if (to) {
 #pragma unroll
-        for (int j = 0; j < 32; j++) atomicAdd(grad + OFF_W2 + t * H + c + j, g[j]);
-      }
-    } else if (warp == 2) {
-      for (uint32_t c = 0; c < 224; c += 32) {  // G columns 0..223 (208.. unused)
-        tc::ld32(tmem + lane_base + tt::T_G + c, g);
-#pragma unroll
-        for (int j = 0; j < 32; j++) {
-          const uint32_t col = c + j;
-          if (t >= tt::A_X && t < tt::A_X + F && col >= tt::B_DH1 && col < tt::B_DH1 + H)
-            atomicAdd(grad + OFF_W1 + (t - tt::A_X) * H + (col - tt::B_DH1), g[j]);
-          else if (t == tt::A_ONE && col < tt::B_DH1)
-            atomicAdd(grad + OFF_B2 + col, g[j]);
-          else if (t == tt::A_ONE && col < tt::B_H2)
-            atomicAdd(grad + OFF_B1 + (col - tt::B_DH1), g[j]);
-          else if (t == tt::A_DY && col >= tt::B_H2 && col < tt::B_ONE)
-            atomicAdd(grad + OFF_W3 + (col - tt::B_H2), g[j]);
-          else if (t == tt::A_DY && col == tt::B_ONE)
-            atomicAdd(grad + OFF_B3, g[j]);
-        }
+        for (int j = 0; j < 32; j++) atomicAdd(to + j, g[j]);
       }
     }
   }
