@@ -25,8 +25,8 @@
 // edge-lane tile is staged once in shared memory and the CTA's warps split
 // its (chunk, query group) pairs; a query-lane tile's warps split its chunks.
 // Per query the phases are the single-query repair's (repair.cu): deletion
-// seeds (parent == u), invalidation waves over out-rows, reset, pull over
-// in-rows, frontier + insertion seeds, push closure. The batched form has no
+// seeds (parent == u), invalidation waves over out-rows (resetting as they
+// mark), pull over in-rows with the insertion seeds, push closure. The batched form has no
 // counterpart in the reference engine, which repairs one source per engine
 // (include/framework/framework.cuh:1803 InitGraph(src)).
 #include "frontier.cuh"
@@ -506,10 +506,14 @@ struct InvalidatePh {
   uint32_t *inew_next;
   uint32_t qpar;  // parity of the next wave's queue
   uint32_t tag, epoch;
+  // (whoever marks a (y, q) resets its key at once: its old parent is not needed
+  // any more, and no pass over the affected vertices is spent on it)
   __device__ void mark(uint32_t y, uint32_t k, uint32_t bits) {
     const uint32_t old = atomicOr(P->affm + (u64)y * NB + k, bits);
     const uint32_t fresh = bits & ~old;
     if (fresh) {
+      for (uint32_t f = fresh; f; f &= f - 1)
+        P->key[((u64)y * NB + k) * 32 + __ffs(f) - 1] = KEY_INF;
       atomicOr(inew_next + (u64)y * NB + k, fresh);
       note_affected(*P, y, epoch);
       enqueue_once(*P, qpar, y, tag);
@@ -530,14 +534,16 @@ struct InvalidatePh {
     }
     // lane 0 takes every block's children; their affected-mask atomics are
     // independent and issued together, the fresh bits handled after
-    uint32_t bits[NB], old[NB];
+    uint32_t bits[NB], old[NB], any = 0;
 #pragma unroll
     for (int k = 0; k < NB; k++) {
       bits[k] = 0;
       if (!m[k]) continue;
       const bool child = ((m[k] >> lane) & 1u) && key_parent1(cur[k]) == x + 1u;
       bits[k] = __ballot_sync(0xffffffffu, child);
+      any |= bits[k];
     }
+    if (!any) return;
     if (lane == 0) {
 #pragma unroll
       for (int k = 0; k < NB; k++)
@@ -545,9 +551,9 @@ struct InvalidatePh {
       bool fresh_any = false;
 #pragma unroll
       for (int k = 0; k < NB; k++) {
-        const uint32_t fresh = bits[k] & ~old[k];
-        if (fresh) {
-          atomicOr(inew_next + (u64)y * NB + k, fresh);
+        bits[k] &= ~old[k];
+        if (bits[k]) {
+          atomicOr(inew_next + (u64)y * NB + k, bits[k]);
           fresh_any = true;
         }
       }
@@ -555,6 +561,13 @@ struct InvalidatePh {
         note_affected(*P, y, epoch);
         enqueue_once(*P, qpar, y, tag);
       }
+    }
+    // the fresh ones' keys, a lane each
+#pragma unroll
+    for (int k = 0; k < NB; k++) {
+      if (!m[k]) continue;
+      const uint32_t fresh = __shfl_sync(0xffffffffu, bits[k], 0);
+      if ((fresh >> lane) & 1u) P->key[((u64)y * NB + k) * 32 + lane] = KEY_INF;
     }
   }
   __device__ void endQ(uint32_t, int, uint32_t, u64 &) {}
@@ -590,10 +603,24 @@ struct InvalidatePh {
   __device__ void endE(uint32_t, int, uint32_t, u64 *) {}
 };
 
-// Affected (v, q) takes the best (value(x) + w, parent x) over live in-edges.
+// Affected (v, q) takes the best (value(x) + w, parent x) over live in-edges and
+// enters the closure's first frontier when there is one. A (v, q) that an
+// insertion seed of the same phase lowers enters it through that seed.
 template <uint32_t ALGO, bool STORED, int NB>
 struct PullPh {
   const MultiParams *P;
+  uint32_t tag;
+  // the lanes' results for block k of v (warp-collective)
+  __device__ void settle(uint32_t v, int k, bool mine, u64 best) {
+    const uint32_t lane = lane_id();
+    const bool fin = mine && best != KEY_INF;
+    if (fin) lower_key<STRICT>(P->key + ((u64)v * NB + k) * 32 + lane, best);
+    const unsigned bits = __ballot_sync(0xffffffffu, fin);
+    if (bits && lane == 0) {
+      atomicOr(P->nmask[0] + (u64)v * NB + k, bits);
+      enqueue_once(*P, 0, v, tag);
+    }
+  }
   static constexpr bool STRICT = Strict<ALGO, STORED>::value;
   __device__ u64 cand(uint32_t v, uint32_t x, uint32_t w, u64 kx) const {
     const uint32_t vx = key_value(kx);
@@ -621,9 +648,7 @@ struct PullPh {
     }
   }
   __device__ void endQ(uint32_t v, int k, uint32_t mk, u64 &best) {
-    const uint32_t lane = lane_id();
-    if (((mk >> lane) & 1u) && best != KEY_INF)
-      lower_key<STRICT>(P->key + ((u64)v * NB + k) * 32 + lane, best);
+    settle(v, k, (mk >> lane_id()) & 1u, best);
   }
   __device__ void beginE(uint32_t, int k, uint32_t mk, u64 *s) {
     const uint32_t lane = lane_id();
@@ -655,11 +680,8 @@ struct PullPh {
     }
   }
   __device__ void endE(uint32_t v, int k, uint32_t mk, u64 *s) {
-    const uint32_t lane = lane_id();
-    if ((mk >> lane) & 1u) {
-      const u64 best = s[k * 32 + lane];
-      if (best != KEY_INF) lower_key<STRICT>(P->key + ((u64)v * NB + k) * 32 + lane, best);
-    }
+    const bool mine = (mk >> lane_id()) & 1u;
+    settle(v, k, mine, mine ? s[k * 32 + lane_id()] : KEY_INF);
   }
 };
 
@@ -984,13 +1006,17 @@ __global__ void __launch_bounds__(BLOCK, NB >= 8 ? DYCG_MULTI_MIN_BLOCKS : 3)
       for (int k = 0; k < NB; k++) {
         const u64 kv = ld_key(P.key + (u64)e.y * Q + k * 32 + lane);
         const unsigned bits = __ballot_sync(0xffffffffu, key_parent1(kv) == e.x + 1u);
-        if (bits && lane == 0) {
-          const uint32_t old = atomicOr(P.affm + (u64)e.y * NB + k, bits);
-          if (bits & ~old) {
-            atomicOr(P.inew[0] + (u64)e.y * NB + k, bits & ~old);
+        if (!bits) continue;  // warp-uniform
+        uint32_t fresh = 0;
+        if (lane == 0) {
+          fresh = bits & ~atomicOr(P.affm + (u64)e.y * NB + k, bits);
+          if (fresh) {
+            atomicOr(P.inew[0] + (u64)e.y * NB + k, fresh);
             any = true;
           }
         }
+        fresh = __shfl_sync(0xffffffffu, fresh, 0);
+        if ((fresh >> lane) & 1u) P.key[(u64)e.y * Q + k * 32 + lane] = KEY_INF;
       }
       if (lane == 0 && any) {
         note_affected(P, e.y, epoch);
@@ -1029,50 +1055,14 @@ __global__ void __launch_bounds__(BLOCK, NB >= 8 ? DYCG_MULTI_MIN_BLOCKS : 3)
       }
     }
     if (gtid == 0) ctl->tphase[0] = globaltimer_ns();  // seeds + invalidation done
-    // 3. reset the affected (v, q)
-    {
-      // (complete: the invalidation's last barrier is behind)
-      na = *(volatile uint32_t *)&ctl->n_aff;
-      for (uint32_t i = gw; i < na; i += nw) {
-        const uint32_t v = P.aff[i];
-#pragma unroll
-        for (int k = 0; k < NB; k++) {
-          const uint32_t mk = P.affm[(u64)v * NB + k];
-          if ((mk >> lane) & 1u) P.key[(u64)v * Q + k * 32 + lane] = KEY_INF;
-        }
-      }
-      if (!grid_sync(ctl, gen, 0, SEL_AFF, P.timeout_ns).ok) goto done;
-      // 4. pull over in-rows
-      PullPh<ALGO, STORED, NB> ph{&P};
-      auto prep = [&](uint32_t v, uint32_t (&m)[NB]) { return take_masks<NB>(P.affm, v, false, m); };
-      if (!multi_expand<NB, STORED>(P, P.in, P.aff, na, prep, ph, s, s_stage, acc, gen, NO_QUEUE,
-                                    SEL_AFF, 0, P.pull_qratio)
-               .ok)
-        goto done;
-      if (gtid == 0) ctl->tphase[1] = globaltimer_ns();  // reset + pull done
-    }
+    // (complete: the invalidation's last barrier is behind)
+    na = *(volatile uint32_t *)&ctl->n_aff;
   }
   {
-    // 5. frontier: affected (v, q) with a finite value, then insertion seeds
+    // 3. insertion seeds and the pull over the affected (v, q)'s in-rows, one
+    // phase: whatever either reads is an upper bound of a live path, and every
+    // (v, q) either lowers enters the first frontier
     const uint32_t ftag = tag++;
-    if (P.phases & PH_DELETE) {
-      for (uint32_t i = gw; i < na; i += nw) {
-        const uint32_t v = P.aff[i];
-        bool any = false;
-#pragma unroll
-        for (int k = 0; k < NB; k++) {
-          const uint32_t mk = P.affm[(u64)v * NB + k];
-          const bool fin = ((mk >> lane) & 1u) &&
-                           key_value(ld_key(P.key + (u64)v * Q + k * 32 + lane)) != INF32;
-          const unsigned bits = __ballot_sync(0xffffffffu, fin);
-          if (bits && lane == 0) {
-            atomicOr(P.nmask[0] + (u64)v * NB + k, bits);
-            any = true;
-          }
-        }
-        if (lane == 0 && any) enqueue_once(P, 0, v, ftag);
-      }
-    }
     if (P.phases & PH_INSERT) {
       const uint32_t n_add = P.hdr->na;
       for (uint32_t i = gw; i < n_add; i += nw) {
@@ -1098,11 +1088,19 @@ __global__ void __launch_bounds__(BLOCK, NB >= 8 ? DYCG_MULTI_MIN_BLOCKS : 3)
         if (lane == 0 && any) enqueue_once(P, 0, e.y, ftag);
       }
     }
+    if (na) {
+      PullPh<ALGO, STORED, NB> ph{&P, ftag};
+      auto prep = [&](uint32_t v, uint32_t (&m)[NB]) { return take_masks<NB>(P.affm, v, false, m); };
+      sn = multi_expand<NB, STORED>(P, P.in, P.aff, na, prep, ph, s, s_stage, acc, gen, NO_QUEUE,
+                                    SEL_Q0, 0, P.pull_qratio);
+    } else {
+      sn = grid_sync(ctl, gen, 0, SEL_Q0, P.timeout_ns);
+    }
   }
-  sn = grid_sync(ctl, gen, 0, SEL_Q0, P.timeout_ns);
   if (!sn.ok) goto done;
-  if (gtid == 0) ctl->tphase[2] = globaltimer_ns();  // frontier + insertion seeds done
-  // 6. closure waves (or one asynchronous phase)
+  // (the two stages share one phase: its time is reported as the pull's)
+  if (gtid == 0) ctl->tphase[1] = ctl->tphase[2] = globaltimer_ns();
+  // 4. closure waves (or one asynchronous phase)
   if ((P.phases & PH_CLOSE) && P.async) {
     const uint32_t cnt = sn.cnt;
     RelaxPh<ALGO, STORED, NB> ph{&P, P.nmask[0], QPAR_ASYNC, tag++};
@@ -1132,7 +1130,7 @@ __global__ void __launch_bounds__(BLOCK, NB >= 8 ? DYCG_MULTI_MIN_BLOCKS : 3)
     }
   }
   if (gtid == 0) ctl->tphase[3] = globaltimer_ns();  // closure done
-  // 7. clear the snapshot's affected masks
+  // 5. clear the snapshot's affected masks
   if (P.phases & PH_DELETE) {
     for (uint32_t i = gw; i < na; i += nw)
       if (lane < (uint32_t)NB) P.affm[(u64)P.aff[i] * NB + lane] = 0;
