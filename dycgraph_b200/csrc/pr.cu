@@ -79,6 +79,26 @@ __device__ __forceinline__ void push_batch(const PrParams *P, uint32_t *outq, ui
   append_batch(outq, outc, P->n, want, y, &P->ctl->err);
 }
 
+// The same without looking at the results (no value comes back from L2): a
+// dense round finds its frontier by a scan afterwards.
+__device__ __forceinline__ void push_only(const PrParams *P, const uint32_t (&y)[UNROLL],
+                                          const bool (&valid)[UNROLL], float c, Acc &acc) {
+#pragma unroll
+  for (int u = 0; u < UNROLL; u++)
+    if (valid[u]) {
+      atomicAdd(P->r + y[u], c);
+      acc.improved++;
+    }
+}
+
+// A round is dense when at least 1 in DENSE vertices is in its frontier: its rows
+// then hold several times n occurrences, and reading every residual once costs
+// less than a returned value, a crossing test and a queue append per push. A
+// frontier is the vertices with |r| > eps either way (outside the frontier none
+// is above it when a round begins, and a vertex that crossed and came back is
+// dropped when it is consumed), so the rounds push the same values.
+constexpr uint32_t DENSE = 16;
+
 __device__ __forceinline__ uint32_t old_degree(const PrParams *P, uint32_t u) {
   return __float_as_uint(P->delta[u]);
 }
@@ -117,6 +137,7 @@ struct ScatterOp {
   const PrParams *P;
   uint32_t *outq;
   uint32_t *outc;
+  bool dense;
   struct Row {
     float c;
   };
@@ -133,7 +154,8 @@ struct ScatterOp {
   }
   __device__ void edges(uint32_t, const uint32_t (&y)[UNROLL], const uint32_t (&)[UNROLL],
                         const bool (&valid)[UNROLL], Row &row, Acc &acc) {
-    push_batch(P, outq, outc, y, valid, row.c, acc);
+    if (dense) push_only(P, y, valid, row.c, acc);
+    else push_batch(P, outq, outc, y, valid, row.c, acc);
   }
   template <int G>
   __device__ void end(uint32_t, bool, Row &) {}
@@ -170,6 +192,31 @@ __device__ void amend_records(const PrParams &P, uint32_t cur, Acc &acc) {
       }
       append_batch(q, qc, P.n, want, v, &P.ctl->err);
     }
+  }
+}
+
+// Frontier of a dense round: the vertices above epsilon, in vertex order (so
+// that the next round's rows are read in arena order), four per lane and append.
+__device__ void collect(const PrParams &P, uint32_t next) {
+  const uint32_t lane = lane_id();
+  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  for (u64 v0 = (u64)gw * 32 * UNROLL; v0 < P.n; v0 += (u64)warps * 32 * UNROLL) {
+    float rv[UNROLL];
+    uint32_t v[UNROLL];
+    bool want[UNROLL];
+#pragma unroll
+    for (int u = 0; u < UNROLL; u++) {
+      v[u] = (uint32_t)v0 + u * 32 + lane;
+      rv[u] = v[u] < P.n ? __ldcg(P.r + v[u]) : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < UNROLL; u++) {
+      if (!isfinite(rv[u])) atomicCAS(&P.ctl->err, 0u, ERR_NONFINITE);
+      want[u] = fabsf(rv[u]) > P.eps;
+      if (want[u]) P.queued[v[u]] = 1;
+    }
+    append_batch(P.q[next], &P.ctl->q_count[next], P.n, want, v, &P.ctl->err);
   }
 }
 
@@ -211,11 +258,17 @@ __global__ void __launch_bounds__(BLOCK) pr_kernel(const __grid_constant__ PrPar
                      P.timeout_ns);
       if (!sn.ok) goto done;
       // Scatter
-      ScatterOp op{&P, P.q[cur ^ 1], &ctl->q_count[cur ^ 1]};
+      const bool dense = (u64)cnt * DENSE >= P.n;
+      ScatterOp op{&P, P.q[cur ^ 1], &ctl->q_count[cur ^ 1], dense};
       sn = expand_rows<false>(P.out, P.q[cur], cnt, op, acc, P.tiles, ctl, gen,
                               cur ? SEL_Q0 : SEL_Q1, cur ? SYNC_RESET_Q1 : SYNC_RESET_Q0,
                               P.timeout_ns);
       if (!sn.ok) goto done;
+      if (dense) {
+        collect(P, cur ^ 1);
+        sn = grid_sync(ctl, gen, 0, cur ? SEL_Q0 : SEL_Q1, P.timeout_ns);
+        if (!sn.ok) goto done;
+      }
       cur ^= 1;
       if (gtid == 0) ctl->waves = round + 1;
     }

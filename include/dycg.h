@@ -446,8 +446,8 @@ int dycg_tune_query_mapping(dycg_engine *e, const dycg_edge *dels, size_t nd,
  * snapshot, or NULL. In the batched many-query form each snapshot is one
  * replay of a CUDA graph (ingest, mutation, learned admission when that
  * policy is set, repair, cache maintenance) captured once per batch size
- * class (powers of two >= 1024; records are padded with out-of-range entries
- * that ingest drops), with no host synchronisation between snapshots; the
+ * class (powers of two >= 1024; the graph reads the snapshot's own counts and
+ * record addresses), with no host synchronisation between snapshots; the
  * admission plan is computed on the device. Per-stage times are then not
  * split (ms_total per snapshot, ms_repair from the repair kernel's own
  * stamps). Other forms, and an engine still recording policy traces, apply
