@@ -65,9 +65,6 @@ Engine::Engine(const dycg_options &opt) : opt_(opt) {
   if (opt_.cache_policy > DYCG_CACHE_LEARNED) throw Error(DYCG_EINVAL, "unknown cache policy");
   if (opt_.frontier_queue > DYCG_QUEUE_CLAIMED)
     throw Error(DYCG_EINVAL, "unknown frontier-queue scheme");
-  // one CTA per SM: 2.64 ms of mutation per 100K-update R-MAT 26 snapshot,
-  // against 2.85 ms with one warp per record (same box and snapshots)
-  mut_ctas_ = opt_.mutation_ctas ? opt_.mutation_ctas : (uint32_t)num_sms_;
   policy_ = opt_.cache_policy;
   stored_ = opt_.algo == DYCG_ALGO_SSSP && opt_.weight_mode == DYCG_WEIGHT_STORED;
   has_in_ = !opt_.symmetric && opt_.algo != DYCG_ALGO_PR;
@@ -236,6 +233,16 @@ void Engine::build_from_sorted_keys(u64 *keys, uint32_t *wv, u64 m, bool weight_
 void Engine::finish_load() {
   const uint32_t n = n_;
   npages_ = out_.pages + (has_in_ ? in_.pages : 0);
+  // Most CTAs (of 16 warps) of the mutation kernel. Random host transactions cost
+  // four times as much over tens of GB as within one, unless those in flight fall
+  // into a narrow window: a CTA on a quarter of the SMs takes 2.41 ms of a
+  // 100K-update R-MAT 26 snapshot (30 GB), one on half of them 2.71, one on each
+  // 2.98. At 1.6 GB (R-MAT 21) the three take 0.94-0.96 ms, and below it the
+  // suffix scans want all the warps (CC on 500K vertices: 3.66 against 3.40 ms a pass).
+  const u64 arena_bytes = (out_.slots + (has_in_ ? in_.slots : 0)) * 4 * out_.stride;
+  mut_ctas_ = opt_.mutation_ctas          ? opt_.mutation_ctas
+              : arena_bytes > (4ull << 30) ? (uint32_t)std::max(1, num_sms_ / 4)
+                                           : (uint32_t)num_sms_;
   page_slot_ = (uint32_t *)dmalloc((u64)npages_ * 4);
   page_hits_ = (uint32_t *)dmalloc((u64)npages_ * 4);
   CK(cudaMemsetAsync(page_slot_, 0xFF, (u64)npages_ * 4, st_));
