@@ -1850,7 +1850,7 @@ void Engine::cache_maintenance(bool initial) {
   if (policy_ == DYCG_CACHE_LEARNED && !initial) {
     // admission ran before the repair (policy_prefetch); the call ends here
     CK(cudaEventRecord(ev_[5], st_));
-    if (prefetched_)
+    if (prefetched_ && cache_slots_)  // (without cache slots nothing was planned)
       CK(cudaMemcpyAsync(cwk_.h_plan, cwk_.plan, sizeof(CachePlan), cudaMemcpyDeviceToHost, st_));
     return;
   }
@@ -1876,7 +1876,7 @@ void Engine::maintain(dycg_batch_stats *stats) {
 void Engine::maintenance_stats(dycg_batch_stats *stats) {
   const bool learned = prefetched_, hot = planned_;
   prefetched_ = planned_ = false;
-  if (!stats || !(hot || (learned && policy_ == DYCG_CACHE_LEARNED))) return;
+  if (!stats || !cache_slots_ || !(hot || (learned && policy_ == DYCG_CACHE_LEARNED))) return;
   float ms = 0;
   if (hot) cudaEventElapsedTime(&ms, ev_[4], ev_[5]);
   else cudaEventElapsedTime(&ms, pev_[0], pev_[1]);
