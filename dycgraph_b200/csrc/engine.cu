@@ -30,9 +30,11 @@ namespace dycg {
 #define CK(x)                                                                              \
   do {                                                                                     \
     cudaError_t _e = (x);                                                                  \
-    if (_e != cudaSuccess)                                                                 \
+    if (_e != cudaSuccess) {                                                               \
+      cudaGetLastError(); /* reported here, not once more by the next launch's check */    \
       throw Error(_e == cudaErrorMemoryAllocation ? DYCG_ENOMEM : DYCG_ECUDA,              \
                   std::string(#x) + ": " + cudaGetErrorString(_e));                        \
+    }                                                                                      \
   } while (0)
 
 static u64 round_up(u64 x, u64 m) { return (x + m - 1) / m * m; }
@@ -40,6 +42,17 @@ static void fill_phases(dycg_batch_stats *s, const Ctl &c);
 constexpr u64 FETCH_CHUNK = 1u << 20;  // bytes of one pinned chunk of the result ring
 constexpr u64 FETCH_THREADS = 6u << 20;  // results from which helper threads store them
 constexpr size_t CTL_CLEAR = 2 * sizeof(Ctl) + 64;  // control blocks and batch counters
+
+// Around the steps that change graph and results: an exception among them leaves
+// a snapshot half applied and its wave tags and frontier not taken over, so the
+// engine counts as failed unless the steps reach their end.
+struct Committing {
+  bool &failed;
+  bool done = false;
+  ~Committing() {
+    if (!done) failed = true;
+  }
+};
 
 Engine::Engine(const dycg_options &opt) : opt_(opt) {
   if (opt_.algo > DYCG_ALGO_PR) throw Error(DYCG_EINVAL, "unknown algorithm");
@@ -873,6 +886,7 @@ void Engine::apply(const dycg_edge *dels, size_t nd, const dycg_edge *adds, size
     bytes += (nd + na) * sizeof(dycg_edge);
   }
   CK(cudaMemcpyAsync(d_hdr_, h_hdr_, bytes, cudaMemcpyHostToDevice, st_));
+  Committing snapshot{failed};
   enqueue_snapshot(nd, na, false);
   CK(cudaMemcpyAsync(h_ctl_, ctl_, sizeof(Ctl), cudaMemcpyDeviceToHost, st_));
   if (nq_) {
@@ -903,7 +917,6 @@ void Engine::apply(const dycg_edge *dels, size_t nd, const dycg_edge *adds, size
     sync_check("tag reset");
   }
   if (c.err) {
-    failed = true;
     const int code = (c.err == ERR_WAVES || c.err == ERR_BARRIER) ? DYCG_ELIMIT : DYCG_ECAPACITY;
     throw Error(code, "batch failed on the device (error code " + std::to_string(c.err) + ")");
   }
@@ -912,6 +925,7 @@ void Engine::apply(const dycg_edge *dels, size_t nd, const dycg_edge *adds, size
     pr_cur_ = c.pad[0];
     pr_count_ = c.pad[1];
   }
+  snapshot.done = true;
   float ms[4] = {0, 0, 0, 0};
   cudaEventElapsedTime(&ms[0], ev_[0], ev_[1]);
   cudaEventElapsedTime(&ms[1], ev_[1], ev_[2]);
@@ -1535,9 +1549,13 @@ void Engine::apply_batches(const dycg_edge *dels, const uint64_t *nd, const dycg
     bev_.push_back(e);
   }
   std::vector<uint32_t> cls(count);
-  u64 od = 0, oa = 0;
-  for (uint32_t i = 0; i < count; i++) {
+  for (uint32_t i = 0; i < count; i++) {  // captures that fail, fail before anything is applied
     cls[i] = cls_of(std::max<u64>(std::max(nd[i], na[i]), 1));
+    graph_for(cls[i]);
+  }
+  u64 od = 0, oa = 0;
+  Committing snapshots{failed};
+  for (uint32_t i = 0; i < count; i++) {
     const SnapshotGraph &g = graph_for(cls[i]);
     // the class's graph reads the batch where it lies and takes its own counts
     h_bhdr_[i] = BatchHdr{d_dels + od, d_adds + oa, (uint32_t)nd[i], (uint32_t)na[i], {0, 0}};
@@ -1554,7 +1572,6 @@ void Engine::apply_batches(const dycg_edge *dels, const uint64_t *nd, const dycg
   sync_check("batches");
   for (uint32_t i = 0; i < count; i++)
     if (h_bctl_[i].err) {
-      failed = true;
       const uint32_t er = h_bctl_[i].err;
       throw Error(er == ERR_WAVES || er == ERR_BARRIER ? DYCG_ELIMIT : DYCG_ECAPACITY,
                   "snapshot " + std::to_string(i) + " failed on the device (error code " +
@@ -1566,6 +1583,7 @@ void Engine::apply_batches(const dycg_edge *dels, const uint64_t *nd, const dycg
     CK(cudaMemcpyAsync(seq_ + 1, h_seq_ + 1, 4, cudaMemcpyHostToDevice, st_));
     sync_check("tag reset");
   }
+  snapshots.done = true;
   if (stats) {
     for (uint32_t i = 0; i < count; i++) {
       const Ctl &c = h_bctl_[i];
