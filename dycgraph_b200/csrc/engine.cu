@@ -655,6 +655,7 @@ void Engine::ensure_batch(size_t cnt) {
   batch_allocs_.clear();
   size_t c = std::max<size_t>(cnt, 1024);
   c = std::max(c, bcap_ * 2);
+  bcap_ = 0;  // nothing is held until all of it is: an allocation below may fail
   auto al = [&](size_t bytes) {
     void *p = nullptr;
     CK(cudaMalloc(&p, std::max<size_t>(bytes, 16)));

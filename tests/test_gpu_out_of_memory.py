@@ -58,3 +58,28 @@ def test_snapshot_that_runs_out_of_memory_under_way_fails_the_engine():
     e.apply_batch(d, a)
     orc.apply_batch(d, a)
     assert np.array_equal(e.gather()[0], orc.values()[0])
+
+
+def test_batch_buffers_that_do_not_fit_leave_the_engine_usable():
+    n, off, dst, w = graph()
+    e = dg.Engine("sssp", weight_mode="stored")
+    e.load_csr(n, off, dst, w)
+    e.start()
+    orc = oracle.Oracle(oracle.SSSP, n, off, dst, w, weight_mode=oracle.WEIGHT_STORED)
+    orc.init()
+    for step in range(3):
+        o, dd, ww = orc.csr()
+        d, a = cases.random_batch(n, o, dd, ww, 300, 300, step)
+        e.apply_batch(d, a)
+        orc.apply_batch(d, a)
+        assert np.array_equal(e.gather()[0], orc.values()[0]), step
+        with Held():
+            # (the first list alone, 16 bytes a record, is twice what is left)
+            with pytest.raises(dg.DycgError) as err:
+                e.reserve_batch(8 << 20)
+            assert err.value.code == ENOMEM
+    e.reserve_batch(2000)
+    d, a = cases.random_batch(n, *orc.csr(), 2000, 2000, 9)
+    e.apply_batch(d, a)
+    orc.apply_batch(d, a)
+    assert np.array_equal(e.gather()[0], orc.values()[0])
