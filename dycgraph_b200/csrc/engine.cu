@@ -2042,7 +2042,8 @@ void Engine::info(dycg_graph_info *out) {
   for (uint32_t x : l) m += x;
   out->live_edges = m;
   out->arena_slots = out_.slots + (has_in_ ? in_.slots : 0);
-  out->arena_used = top_out + top_in;
+  // (requests that met the arena's end may have left the top past it)
+  out->arena_used = std::min(top_out, out_.slots) + (has_in_ ? std::min(top_in, in_.slots) : 0);
   out->pages = npages_;
   out->cache_slots = cache_slots_;
   out->cached_pages = cache_slots_ ? cache_slots_ - cwk_.h_plan->free_count : 0;

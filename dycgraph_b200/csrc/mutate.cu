@@ -376,15 +376,37 @@ __device__ void append_slots(const MutParams &M, uint32_t dir, uint32_t pos, uin
   }
 }
 
+// A block of `slots` slots at the arena tail, or NO_BLOCK when the rest of the arena
+// does not hold it. Small blocks are many (a thousand rows may outgrow theirs in one
+// launch) and take one addition; a large one that does not fit must leave the rest
+// to smaller ones, so it takes a compare-and-swap, and there are few of them.
+constexpr u64 NO_BLOCK = ~0ull;
+constexpr uint32_t SMALL_BLOCK = 1u << 16;
+__device__ __forceinline__ u64 reserve_block(const Adj &A, uint32_t slots) {
+  u64 top = *(volatile u64 *)A.top;
+  if (slots <= SMALL_BLOCK) {
+    if (top + slots > A.arena) return NO_BLOCK;
+    top = atomicAdd(A.top, (u64)slots);
+    return top + slots <= A.arena ? top : NO_BLOCK;
+  }
+  while (top + slots <= A.arena) {
+    const u64 seen = atomicCAS(A.top, top, top + slots);
+    if (seen == top) return top;
+    top = seen;
+  }
+  return NO_BLOCK;
+}
+
 // Then, the deletions done, the descriptors. A row that does not fit drops its
 // deleted slots on its way to a new power-of-two block (with headroom) at the
 // arena tail, or in its own block: when they are half of it (the copy then pays
-// for itself), and, once half of the arena's headroom is used, whenever the live
-// occurrences and a reserve fit. While there is headroom a row with few deleted
-// slots gets the block its slots ask for. So a stream of balanced updates cannot
-// eat the arena (2,000-update snapshots on R-MAT 16 used to after some 5,000 of
-// them) and no repair reads a slot deleted long ago for ever. Rows that change
-// their slots are left to the relocation phase.
+// for itself), once the block that its slots ask for would reach into the second half
+// of the arena's headroom, whenever the live occurrences and a reserve fit, and
+// whenever they fit at all if the arena has no such block left. So a row takes
+// space for good only when its live occurrences outgrow its block (2,000-update
+// snapshots on R-MAT 16 used to eat the arena in some 5,000 of them), no row asks
+// in vain for a larger block than it needs, and no repair reads a slot deleted
+// long ago for ever. Rows that change their slots are left to the relocation phase.
 __device__ void append_rows(const MutParams &M, uint32_t dir, uint32_t pos, uint32_t na,
                             Counts &C) {
   const Adj &A = M.adj[dir];
@@ -402,24 +424,36 @@ __device__ void append_rows(const MutParams &M, uint32_t dir, uint32_t pos, uint
   }
   const auto block = [](u64 slots) { return next_pow2_u32((uint32_t)(slots + slots / 8 + 1)); };
   const u64 need = (u64)live + count, off = A.off[row];
-  const bool scarce = *(volatile u64 *)A.top > M.scarce[dir];
-  const uint32_t tight = block(need);
-  if (tight > cap || !(scarce || need <= cap / 2)) {
-    const uint32_t ncap = scarce ? tight : block((u64)len + count);
-    const u64 noff = atomicAdd(A.top, (u64)ncap);
-    const uint32_t nchunk = (len + RELOC_CHUNK - 1) / RELOC_CHUNK;
-    const uint32_t cb = atomicAdd(&M.mctl->tile_count, nchunk);
-    const uint32_t k = atomicAdd(&M.mctl->q_count[1], 1u);
-    if (noff + ncap > A.arena || k >= M.reloc.cap || cb + nchunk > M.reloc.chunk_cap) {
-      atomicCAS(&M.ctl->err, 0u, ERR_ARENA);
+  const uint32_t tight = block(need), roomy = block((u64)len + count);
+  const bool scarce = *(volatile u64 *)A.top + roomy > M.scarce[dir];
+  bool stays = tight <= cap && (scarce || need <= cap / 2);
+  if (!stays) {
+    uint32_t ncap = scarce ? tight : roomy;
+    u64 noff = reserve_block(A, ncap);
+    if (noff == NO_BLOCK && need > cap && tight < ncap) {
+      ncap = tight;
+      noff = reserve_block(A, ncap);
+    }
+    stays = noff == NO_BLOCK && need <= cap;
+    if (!stays) {
+      if (noff == NO_BLOCK) {
+        atomicCAS(&M.ctl->err, 0u, ERR_ARENA);
+        return;
+      }
+      const uint32_t nchunk = (len + RELOC_CHUNK - 1) / RELOC_CHUNK;
+      const uint32_t cb = atomicAdd(&M.mctl->tile_count, nchunk);
+      const uint32_t k = atomicAdd(&M.mctl->q_count[1], 1u);
+      if (k >= M.reloc.cap || cb + nchunk > M.reloc.chunk_cap) {
+        atomicCAS(&M.ctl->err, 0u, ERR_ARENA);
+        return;
+      }
+      M.reloc.rec[k] = RelocRec{row, pos, len, dir, off, noff};
+      for (uint32_t c = 0; c < nchunk; c++) M.reloc.chunks[cb + c] = make_uint2(k, c);
+      A.off[row] = noff;
+      A.cap[row] = ncap;
+      C.moved++;
       return;
     }
-    M.reloc.rec[k] = RelocRec{row, pos, len, dir, off, noff};
-    for (uint32_t c = 0; c < nchunk; c++) M.reloc.chunks[cb + c] = make_uint2(k, c);
-    A.off[row] = noff;
-    A.cap[row] = ncap;
-    C.moved++;
-    return;
   }
   const uint32_t k = atomicAdd(&M.mctl->q_count[1], 1u);
   if (k >= M.reloc.cap) {
