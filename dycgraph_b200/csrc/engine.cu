@@ -681,6 +681,7 @@ void Engine::ensure_batch(size_t cnt) {
   const u64 slots = out_.slots + (has_in_ ? in_.slots : 0);
   reloc_.rec = (RelocRec *)al(dirs * c * sizeof(RelocRec));
   reloc_.wide = (uint32_t *)al(dirs * c * 4);
+  reloc_.longs = (uint2 *)al(dirs * c * sizeof(uint2));
   reloc_.cap = (uint32_t)(dirs * c);
   const u64 cc = std::min<u64>(slots / RELOC_CHUNK + dirs * c + 1024, 0x7FFFFFFFull);
   reloc_.chunks = (uint2 *)al(cc * sizeof(uint2));

@@ -170,7 +170,8 @@ struct RelocRec {
 struct Reloc {
   RelocRec *rec;
   uint2 *chunks;      // of rows that move
-  uint32_t *wide;     // long rows that stay
+  uint32_t *wide;     // rows that stay and take a CTA
+  uint2 *longs;       // rows that the whole grid copies
   uint32_t cap, chunk_cap;
 };
 struct MutParams {

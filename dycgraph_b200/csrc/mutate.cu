@@ -34,6 +34,13 @@ namespace {
 
 constexpr int MUT_BLOCK = 512;
 constexpr uint32_t COMPACT_WARP = 1024;  // longest row that one warp compacts
+// Rows above this many slots are copied by the whole grid (copy_long), wherever they
+// go. In place, one CTA takes 2048 slots per host round trip; on the way to a new
+// block, a chunk's place needs the deletion bits of all slots before it. Mutation of
+// a snapshot of 100 records that fills one row, by those forms -> by the grid: 2^13
+// slots moved 0.066 -> 0.041 ms, 2^14 in place 0.076 -> 0.040, 2^16 0.25 -> 0.045,
+// 2^20 3.9 -> 0.21, 2^23 in place 32 -> 1.5, moved 8.2 -> 0.98. At 2^12 they are level.
+constexpr uint32_t LONG_ROW = 1u << 12;
 
 struct Counts {
   uint32_t link = 0, hbm = 0, missing = 0, moved = 0;
@@ -376,6 +383,32 @@ __device__ void append_slots(const MutParams &M, uint32_t dir, uint32_t pos, uin
   }
 }
 
+// Long rows of this launch in two lists (0: those that stay in their block, 1: those
+// that move, from the end of the same array), each row with the number of its first
+// chunk: one addition gives both places, so the numbers ascend along a list. The
+// chunks' counts live in the suffix phase's list, which is over: 4 bytes per 512
+// slots of long rows, where that list has 16 per 256 slots of the arena.
+constexpr uint32_t LONG_CHUNK = 512;
+struct LongRows {
+  uint2 *first;      // (relocation record, first chunk) of row 0, row 1 at first[step]
+  int step;
+  uint32_t *count;   // per chunk: its live slots, then those before it
+  uint32_t rows, chunks;
+  __device__ uint2 &row(uint32_t i) const { return first[(int)i * step]; }
+};
+__device__ __forceinline__ LongRows long_rows(const MutParams &M, uint32_t list) {
+  const u64 n = *(volatile u64 *)(list ? &M.mctl->a_tail : &M.mctl->a_head);
+  return {list ? M.reloc.longs + M.reloc.cap - 1 : M.reloc.longs, list ? -1 : 1,
+          reinterpret_cast<uint32_t *>(M.suffix) + (u64)list * M.suffix_cap * 2,
+          (uint32_t)(n >> 32), (uint32_t)n};
+}
+__device__ __forceinline__ void list_long(const MutParams &M, uint32_t list, uint32_t k,
+                                          uint32_t len) {
+  const u64 at = atomicAdd(list ? &M.mctl->a_tail : &M.mctl->a_head,
+                           (1ull << 32) | ((len + LONG_CHUNK - 1) / LONG_CHUNK));
+  long_rows(M, list).row(at >> 32) = make_uint2(k, (uint32_t)at);
+}
+
 // A block of `slots` slots at the arena tail, or NO_BLOCK when the rest of the arena
 // does not hold it. Small blocks are many (a thousand rows may outgrow theirs in one
 // launch) and take one addition; a large one that does not fit must leave the rest
@@ -440,8 +473,8 @@ __device__ void append_rows(const MutParams &M, uint32_t dir, uint32_t pos, uint
         atomicCAS(&M.ctl->err, 0u, ERR_ARENA);
         return;
       }
-      const uint32_t nchunk = (len + RELOC_CHUNK - 1) / RELOC_CHUNK;
-      const uint32_t cb = atomicAdd(&M.mctl->tile_count, nchunk);
+      const uint32_t nchunk = len > LONG_ROW ? 0 : (len + RELOC_CHUNK - 1) / RELOC_CHUNK;
+      const uint32_t cb = nchunk ? atomicAdd(&M.mctl->tile_count, nchunk) : 0;
       const uint32_t k = atomicAdd(&M.mctl->q_count[1], 1u);
       if (k >= M.reloc.cap || cb + nchunk > M.reloc.chunk_cap) {
         atomicCAS(&M.ctl->err, 0u, ERR_ARENA);
@@ -449,6 +482,7 @@ __device__ void append_rows(const MutParams &M, uint32_t dir, uint32_t pos, uint
       }
       M.reloc.rec[k] = RelocRec{row, pos, len, dir, off, noff};
       for (uint32_t c = 0; c < nchunk; c++) M.reloc.chunks[cb + c] = make_uint2(k, c);
+      if (len > LONG_ROW) list_long(M, 1, k, len);
       A.off[row] = noff;
       A.cap[row] = ncap;
       C.moved++;
@@ -461,8 +495,9 @@ __device__ void append_rows(const MutParams &M, uint32_t dir, uint32_t pos, uint
     return;
   }
   M.reloc.rec[k] = RelocRec{row, pos, len, dir, off, off};
-  // a long row takes a whole CTA
-  if (len > COMPACT_WARP) M.reloc.wide[atomicAdd(&M.mctl->q_count[2], 1u)] = k;
+  // a wide row takes a whole CTA, a long one the whole grid
+  if (len > LONG_ROW) list_long(M, 0, k, len);
+  else if (len > COMPACT_WARP) M.reloc.wide[atomicAdd(&M.mctl->q_count[2], 1u)] = k;
 }
 
 // Deleted slots among the first `count` of the row at off (warp-collective).
@@ -595,12 +630,179 @@ __device__ void finish_row(const MutParams &M, const RelocRec &rec, uint32_t sor
 __device__ void finish_warp(const MutParams &M, const RelocRec &rec, Counts &C) {
   const Adj &A = M.adj[rec.dir];
   const bool stays = rec.new_off == rec.old_off;
-  if (stays && rec.len > COMPACT_WARP) return;  // a CTA's
+  if (rec.len > (stays ? COMPACT_WARP : LONG_ROW)) return;  // a CTA's or the grid's
   const uint32_t srt = A.srt[rec.row];
   const uint32_t sorted = srt - dead_slots(A, rec.old_off, srt);
   __syncwarp();
   if (stays) compact_row<32>(M, rec, nullptr, C);
   finish_row(M, rec, sorted, lane_id(), 32);
+}
+
+// Chunk g of a list: its row's relocation record (x) and its number in the row (y).
+__device__ __forceinline__ uint2 long_chunk(const LongRows &L, uint32_t g) {
+  uint32_t lo = 0, hi = L.rows;
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) / 2;
+    if (L.row(mid).y <= g) lo = mid; else hi = mid;
+  }
+  const uint2 r = L.row(lo);
+  return make_uint2(r.x, g - r.y);
+}
+
+// A warp's chunk in registers: its slots, which of them live, and where those go.
+constexpr uint32_t LONG_PER = LONG_CHUNK / 32;
+struct LongPiece {
+  uint2 v[LONG_PER];
+  unsigned live[LONG_PER];
+  u64 to;
+  uint32_t dir;
+};
+__device__ __forceinline__ void read_long(const MutParams &M, const LongRows &L, uint32_t g,
+                                          LongPiece &x, Counts &C) {
+  const uint32_t lane = lane_id();
+  const uint2 ch = long_chunk(L, g);
+  const RelocRec rec = M.reloc.rec[ch.x];
+  const Adj &A = M.adj[rec.dir];
+  x.dir = rec.dir;
+  x.to = rec.new_off + L.count[g];
+  const uint32_t b = ch.y * LONG_CHUNK, cnt = min(rec.len - b, LONG_CHUNK);
+  const u64 p = rec.old_off + b;
+  // the chunk's deletion bits, a word per lane
+  const uint32_t sh = (uint32_t)p & 31;
+  const uint32_t bits =
+      lane * 32 < sh + cnt ? *(volatile uint32_t *)(A.tbits + (p >> 5) + lane) : ~0u;
+#pragma unroll
+  for (uint32_t t = 0; t < LONG_PER; t++)
+    if (t * 32 + lane < cnt) {
+      x.v[t] = read_pair_rw(A, p + t * 32 + lane);
+      C.link += 4u * A.stride;
+    }
+#pragma unroll
+  for (uint32_t t = 0; t < LONG_PER; t++) {
+    const uint32_t lo = __shfl_sync(0xffffffffu, bits, t);
+    const uint32_t hi = __shfl_sync(0xffffffffu, bits, t + 1);
+    const uint32_t left = cnt > t * 32 ? cnt - t * 32 : 0u;  // slots from here on
+    x.live[t] = ~__funnelshift_r(lo, hi, sh) & (left >= 32 ? ~0u : (1u << left) - 1);
+  }
+}
+// Half a chunk at a time goes through shared memory (`half`: the warp's part), so that
+// the stores cover whole 128-byte lines however the live slots were scattered: a store
+// per 32 slots read left the link with 50-byte writes.
+constexpr uint32_t LONG_HALF = LONG_CHUNK / 2;
+__device__ __forceinline__ void write_long(const MutParams &M, const LongPiece &x, uint2 *half,
+                                           Counts &C) {
+  const Adj &A = M.adj[x.dir];
+  const uint32_t lane = lane_id();
+  u64 to = x.to;
+#pragma unroll
+  for (uint32_t h = 0; h < 2; h++) {
+    uint32_t n = 0;
+#pragma unroll
+    for (uint32_t t = h * (LONG_PER / 2); t < (h + 1) * (LONG_PER / 2); t++) {
+      if ((x.live[t] >> lane) & 1u) half[n + __popc(x.live[t] & ((1u << lane) - 1))] = x.v[t];
+      n += __popc(x.live[t]);
+    }
+    __syncwarp();
+    for (u64 p = (to & ~31ull) + lane; p < to + n; p += 32) {
+      if (p < to) continue;
+      const bool c = write_slot(A, p, half[p - to].x, half[p - to].y);
+      C.link += 4u * A.stride;
+      if (c) C.hbm += 4u * A.stride;
+    }
+    __syncwarp();
+    to += n;
+  }
+}
+
+// Long rows by the whole grid: the live slots of every chunk are counted, a CTA per
+// row turns the counts into places, and the chunks are copied, a warp each. Rows
+// that move are copied as the warps come; rows that stay in steps of as many
+// chunks as there are warps, all read before any is written: a live slot's place is
+// never past its own, and chunks are taken in order, so what a step overwrites
+// has been read, and no copy elsewhere is needed. What bounds it is the host link
+// (2^20 slots are 4 MB in and up to 4 out).
+__device__ Snap copy_long(const MutParams &M, uint32_t &gen, Counts &C) {
+  constexpr uint32_t W = MUT_BLOCK / 32;
+  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+  const uint32_t gw = warp * gridDim.x + blockIdx.x, nw = gridDim.x * W;
+  const LongRows lists[2] = {long_rows(M, 0), long_rows(M, 1)};
+  for (const LongRows &L : lists)
+    for (uint32_t g = gw; g < L.chunks; g += nw) {
+      const uint2 ch = long_chunk(L, g);
+      const RelocRec rec = M.reloc.rec[ch.x];
+      const uint32_t b = ch.y * LONG_CHUNK, cnt = min(rec.len - b, LONG_CHUNK);
+      const uint32_t dead = dead_slots(M.adj[rec.dir], rec.old_off + b, cnt);
+      if (lane == 0) L.count[g] = cnt - dead;
+    }
+  Snap sn = grid_sync(M.mctl, gen, 0, SEL_Q1, M.timeout_ns);
+  if (!sn.ok) return sn;
+  __shared__ uint32_t s_sum[W];
+  for (const LongRows &L : lists)
+    for (uint32_t i = blockIdx.x; i < L.rows; i += gridDim.x) {
+      const uint2 lr = L.row(i);
+      const uint32_t nch = (M.reloc.rec[lr.x].len + LONG_CHUNK - 1) / LONG_CHUNK;
+      uint32_t before = 0;
+      for (uint32_t c0 = 0; c0 < nch; c0 += MUT_BLOCK) {
+        const uint32_t c = c0 + threadIdx.x, x = c < nch ? L.count[lr.y + c] : 0u;
+        uint32_t sum = x;  // inclusive over the warp, then over the CTA
+#pragma unroll
+        for (int o = 1; o < 32; o *= 2) {
+          const uint32_t y = __shfl_up_sync(0xffffffffu, sum, o);
+          if (lane >= (uint32_t)o) sum += y;
+        }
+        __syncthreads();  // (s_sum is free again)
+        if (lane == 31) s_sum[warp] = sum;
+        __syncthreads();
+        uint32_t all = 0;
+        for (uint32_t w = 0; w < W; w++) {
+          if (w == warp) sum += all;
+          all += s_sum[w];
+        }
+        if (c < nch) L.count[lr.y + c] = before + sum - x;
+        before += all;
+      }
+    }
+  sn = grid_sync(M.mctl, gen, 0, SEL_Q1, M.timeout_ns);
+  if (!sn.ok) return sn;
+  __shared__ uint2 s_half[W][LONG_HALF];
+  LongPiece x;
+  for (uint32_t g = gw; g < lists[1].chunks; g += nw) {
+    read_long(M, lists[1], g, x, C);
+    write_long(M, x, s_half[warp], C);
+  }
+  for (uint32_t g0 = 0; g0 < lists[0].chunks; g0 += nw) {
+    const bool mine = g0 + gw < lists[0].chunks;
+    if (mine) read_long(M, lists[0], g0 + gw, x, C);
+    sn = grid_sync(M.mctl, gen, 0, SEL_Q1, M.timeout_ns);
+    if (!sn.ok) return sn;
+    if (mine) write_long(M, x, s_half[warp], C);
+  }
+  // (every deletion bit and every slot that an insertion takes has been read)
+  sn = grid_sync(M.mctl, gen, 0, SEL_Q1, M.timeout_ns);
+  if (!sn.ok) return sn;
+  for (const LongRows &L : lists)
+    for (uint32_t i = blockIdx.x; i < L.rows; i += gridDim.x) {
+      const uint2 lr = L.row(i);
+      const RelocRec rec = M.reloc.rec[lr.x];
+      const Adj &A = M.adj[rec.dir];
+      // live slots of the sorted prefix: those of its whole chunks and the rest's
+      const uint32_t srt = A.srt[rec.row], c = srt / LONG_CHUNK, part = srt % LONG_CHUNK;
+      uint32_t sorted = c * LONG_CHUNK < rec.len ? L.count[lr.y + c] : A.live[rec.row];
+      sorted += part - dead_slots(A, rec.old_off + srt - part, part);
+      __syncthreads();  // (before any thread clears bits)
+      if (rec.new_off == rec.old_off) {
+        const u64 w0 = rec.old_off >> 5, w1 = (rec.old_off + rec.len - 1) >> 5;
+        for (u64 w = w0 + threadIdx.x; w <= w1; w += MUT_BLOCK) {
+          uint32_t b = ~0u;  // the row's bits of this word
+          if (w == w0) b &= ~0u << (rec.old_off & 31);
+          if (w == w1) b &= ~0u >> (31 - ((rec.old_off + rec.len - 1) & 31));
+          if (b == ~0u) A.tbits[w] = 0;
+          else atomicAnd(A.tbits + w, ~b);
+        }
+      }
+      finish_row(M, rec, sorted, threadIdx.x, MUT_BLOCK);
+    }
+  return sn;
 }
 
 }  // namespace
@@ -666,6 +868,8 @@ __global__ void __launch_bounds__(MUT_BLOCK, 1)
         compact_row<MUT_BLOCK>(M, rec, sm, C);
         finish_row(M, rec, sorted, threadIdx.x, MUT_BLOCK);
       }
+      if (*(volatile u64 *)&M.mctl->a_head | *(volatile u64 *)&M.mctl->a_tail)
+        sn = copy_long(M, gen, C);
     }
   }
   if (!sn.ok && threadIdx.x == 0) atomicCAS(&M.ctl->err, 0u, ERR_BARRIER);
@@ -686,7 +890,10 @@ cudaError_t launch_mutate(const MutParams &M, uint32_t records, uint32_t ctas, c
   // capping the CTAs narrows that window of the host arena, and the host link
   // serves transactions in a narrow window several times faster than ones
   // spread over a multi-GB arena. A small batch needs no more CTAs than it has
-  // warps' work for, and its barriers are cheaper with fewer.
+  // warps' work for, and its barriers are cheaper with fewer; but one record can fill
+  // a row of any length, so there are eight: three records that fill a 2^20-slot row
+  // take 1.0 ms with one CTA, 0.20 with eight and 0.17 with sixteen, a batch of 32
+  // records 19 us of mutation with four or eight CTAs and 20.5 with sixteen.
   int dev = 0, sms = 0, per_sm = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -695,7 +902,8 @@ cudaError_t launch_mutate(const MutParams &M, uint32_t records, uint32_t ctas, c
   if (e != cudaSuccess) return e;
   const u64 warps = ((u64)records * M.dirs + 3) / 4;
   const u64 grid = std::max<u64>(
-      1, std::min<u64>({(warps + 1) / 2, (u64)ctas, (u64)std::max(per_sm, 1) * (u64)sms}));
+      1, std::min<u64>({std::max<u64>((warps + 1) / 2, 8), (u64)ctas,
+                        (u64)std::max(per_sm, 1) * (u64)sms}));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(MUT_BLOCK);
