@@ -982,7 +982,7 @@ void Engine::apply(const dycg_edge *dels, size_t nd, const dycg_edge *adds, size
 // or batched; phases a launch skipped have no stamp and count zero).
 static void fill_phases(dycg_batch_stats *s, const Ctl &c) {
   const u64 t[4] = {c.tphase[0], c.tphase[1], c.tphase[2], c.tphase[3]};
-  double *out[4] = {&s->ms_phase_invalidate, &s->ms_phase_pull, &s->ms_phase_seed,
+  double *out[4] = {&s->ms_phase_invalidate, &s->ms_phase_seed, &s->ms_phase_pull,
                     &s->ms_phase_closure};
   u64 prev = c.stat[ST_T_START];
   for (int i = 0; i < 4; i++) {

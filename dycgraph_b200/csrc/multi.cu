@@ -1087,6 +1087,9 @@ __global__ void __launch_bounds__(BLOCK, NB >= 8 ? DYCG_MULTI_MIN_BLOCKS : 3)
         }
         if (lane == 0 && any) enqueue_once(P, 0, e.y, ftag);
       }
+      // the seeds' share of the phase: until the first warp, which has as many as any,
+      // is through with its own
+      if (gtid == 0) ctl->tphase[1] = globaltimer_ns();
     }
     if (na) {
       PullPh<ALGO, STORED, NB> ph{&P, ftag};
@@ -1098,8 +1101,7 @@ __global__ void __launch_bounds__(BLOCK, NB >= 8 ? DYCG_MULTI_MIN_BLOCKS : 3)
     }
   }
   if (!sn.ok) goto done;
-  // (the two stages share one phase: its time is reported as the pull's)
-  if (gtid == 0) ctl->tphase[1] = ctl->tphase[2] = globaltimer_ns();
+  if (gtid == 0) ctl->tphase[2] = globaltimer_ns();  // pull done
   // 4. closure waves (or one asynchronous phase)
   if ((P.phases & PH_CLOSE) && P.async) {
     const uint32_t cnt = sn.cnt;

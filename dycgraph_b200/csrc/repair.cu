@@ -306,6 +306,9 @@ __global__ void __launch_bounds__(REPAIR_BLOCK, 1) repair_kernel(const __grid_co
       if (P.delta) note_min(ctl, imp);
       append_batch(P.q[0], &ctl->q_count[0], P.n, want, v, &ctl->err);
     }
+    // the seeds' share of the phase: until the first warp, which has as many as any,
+    // is through with its own
+    if (gtid == 0) ctl->tphase[1] = globaltimer_ns();
   }
   if (!(P.phases & (PH_DELETE | PH_INSERT)) && P.delta) {
     // static solve: the minimum of the frontier it was given
@@ -321,8 +324,7 @@ __global__ void __launch_bounds__(REPAIR_BLOCK, 1) repair_kernel(const __grid_co
     sn = grid_sync(ctl, gen, SYNC_RESET_VMIN, SEL_Q0, P.timeout_ns);
   }
   if (!sn.ok) goto done;
-  // (the two stages share one phase: its time is reported as the pull's)
-  if (gtid == 0) ctl->tphase[1] = ctl->tphase[2] = globaltimer_ns();
+  if (gtid == 0) ctl->tphase[2] = globaltimer_ns();  // pull done
   // 4. closure waves. Ordered (P.delta, for high-diameter graphs, the B200 form
   // of the reference's ordered insertion schedule, framework.cuh:537-556): each
   // wave expands only the frontier vertices whose value is below the wave's

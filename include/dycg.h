@@ -143,8 +143,8 @@ typedef struct dycg_batch_stats {
   /* time inside the repair kernel per phase (SSSP/BFS/CC: one source, or
      the batched many-query form; zero for PageRank and per-query repairs) */
   double ms_phase_invalidate;  /* deletion seeds + invalidation waves        */
-  double ms_phase_pull;        /* reset + pull over in-rows                  */
-  double ms_phase_seed;        /* frontier + insertion seeds                 */
+  double ms_phase_pull;        /* pull over in-rows, after the seeds         */
+  double ms_phase_seed;        /* insertion seeds                            */
   double ms_phase_closure;     /* push closure waves                         */
   uint64_t reserved[2];
 } dycg_batch_stats;
