@@ -24,6 +24,7 @@
 #include <unistd.h>
 
 #include "engine.h"
+#include "mutation_grid.h"
 
 namespace dycg {
 
@@ -246,16 +247,8 @@ void Engine::build_from_sorted_keys(u64 *keys, uint32_t *wv, u64 m, bool weight_
 void Engine::finish_load() {
   const uint32_t n = n_;
   npages_ = out_.pages + (has_in_ ? in_.pages : 0);
-  // Most CTAs (of 16 warps) of the mutation kernel. Random host transactions cost
-  // four times as much over tens of GB as within one, unless those in flight fall
-  // into a narrow window: a CTA on a quarter of the SMs takes 2.41 ms of a
-  // 100K-update R-MAT 26 snapshot (30 GB), one on half of them 2.71, one on each
-  // 2.98. At 1.6 GB (R-MAT 21) the three take 0.94-0.96 ms, and below it the
-  // suffix scans want all the warps (CC on 500K vertices: 3.66 against 3.40 ms a pass).
-  const u64 arena_bytes = (out_.slots + (has_in_ ? in_.slots : 0)) * 4 * out_.stride;
-  mut_ctas_ = opt_.mutation_ctas          ? opt_.mutation_ctas
-              : arena_bytes > (4ull << 30) ? (uint32_t)std::max(1, num_sms_ / 4)
-                                           : (uint32_t)num_sms_;
+  mut_ctas_ = mutation_ctas(opt_.mutation_ctas, (uint32_t)num_sms_,
+                            (out_.slots + (has_in_ ? in_.slots : 0)) * 4 * out_.stride);
   page_slot_ = (uint32_t *)dmalloc((u64)npages_ * 4);
   page_hits_ = (uint32_t *)dmalloc((u64)npages_ * 4);
   CK(cudaMemsetAsync(page_slot_, 0xFF, (u64)npages_ * 4, st_));

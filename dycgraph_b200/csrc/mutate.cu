@@ -27,12 +27,12 @@
 // 1.14.
 #include "frontier.cuh"
 #include "internal.h"
+#include "mutation_grid.h"
 
 namespace dycg {
 
 namespace {
 
-constexpr int MUT_BLOCK = 512;
 constexpr uint32_t COMPACT_WARP = 1024;  // longest row that one warp compacts
 // Rows above this many slots are copied by the whole grid (copy_long), wherever they
 // go. In place, one CTA takes 2048 slots per host round trip; on the way to a new
@@ -885,27 +885,16 @@ __global__ void __launch_bounds__(MUT_BLOCK, 1)
 
 cudaError_t launch_mutate(const MutParams &M, uint32_t records, uint32_t ctas, cudaStream_t s) {
   if (!records) return cudaSuccess;
-  // The records are in row order (sorted by ingest) and the rows in arena
-  // order, so the warps in flight work on a window of consecutive records;
-  // capping the CTAs narrows that window of the host arena, and the host link
-  // serves transactions in a narrow window several times faster than ones
-  // spread over a multi-GB arena. A small batch needs no more CTAs than it has
-  // warps' work for, and its barriers are cheaper with fewer; but one record can fill
-  // a row of any length, so there are eight: three records that fill a 2^20-slot row
-  // take 1.0 ms with one CTA, 0.20 with eight and 0.17 with sixteen, a batch of 32
-  // records 19 us of mutation with four or eight CTAs and 20.5 with sixteen.
   int dev = 0, sms = 0, per_sm = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e == cudaSuccess)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mutate_kernel, MUT_BLOCK, 0);
   if (e != cudaSuccess) return e;
-  const u64 warps = ((u64)records * M.dirs + 3) / 4;
-  const u64 grid = std::max<u64>(
-      1, std::min<u64>({std::max<u64>((warps + 1) / 2, 8), (u64)ctas,
-                        (u64)std::max(per_sm, 1) * (u64)sms}));
+  const uint32_t grid =
+      mutation_grid(records, M.dirs, ctas, (u64)std::max(per_sm, 1) * (u64)sms);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
+  cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(MUT_BLOCK);
   cfg.stream = s;
   cudaLaunchAttribute attr[1];

@@ -103,8 +103,10 @@ typedef struct dycg_options {
                           /* DYCG_QUEUE_CLAIMED, how warps share a wave's rows */
                           /* (the batched form's scheme is tuned, see          */
                           /* dycg_tune_query_mapping)                          */
-  uint32_t mutation_ctas; /* most CTAs of the mutation kernel (0: one per SM, */
-                          /* on a quarter of the SMs for arenas above 4 GB).  */
+  uint32_t mutation_ctas; /* most CTAs of the mutation kernel, counted in CTAs */
+                          /* of eight warps and rounded up to an even number  */
+                          /* (0: two per SM, on a quarter of the SMs for      */
+                          /* arenas above 4 GB).                              */
                           /* They take a snapshot's records in row order, so  */
                           /* fewer CTAs in flight keep their host transactions*/
                           /* in a narrower window of the arena, which the host*/
