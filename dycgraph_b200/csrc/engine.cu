@@ -8,14 +8,11 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <fstream>
 #include <sstream>
-#include <system_error>
-#include <thread>
 #include <unordered_set>
 
 #include <fcntl.h>
@@ -25,6 +22,7 @@
 
 #include "engine.h"
 #include "mutation_grid.h"
+#include "ring.h"
 
 namespace dycg {
 
@@ -1261,11 +1259,9 @@ void Engine::fetch_keys(const u64 *key, uint32_t Q, uint32_t q, uint32_t *values
 // Two device arrays of `bytes` each into ordinary host memory (a null
 // destination is skipped), through a ring of pinned chunks: the copies run at
 // the link's rate (a copy to pageable memory goes through one driver thread's
-// staging), and helper threads empty the ring, since one thread's stores into
-// fresh pages reach a fraction of that rate. This thread alone talks to the
-// device: it announces a chunk when its copy has arrived and sends the next one
-// into a slot once the slot's last chunk has been stored. Below FETCH_THREADS
-// bytes the helpers' start costs more than they save.
+// staging), and helper threads empty the ring (ring.h), since one thread's stores
+// into fresh pages reach a fraction of that rate. Below FETCH_THREADS bytes the
+// helpers' start costs more than they save.
 void Engine::fetch(const void *d0, void *h0, const void *d1, void *h1, u64 bytes) {
   const u64 all = (h0 ? bytes : 0) + (h1 ? bytes : 0);
   if (all < FETCH_THREADS) {
@@ -1286,51 +1282,19 @@ void Engine::fetch(const void *d0, void *h0, const void *d1, void *h1, u64 bytes
     for (u64 o = 0; h && o < bytes; o += FETCH_CHUNK)
       parts.push_back({d + o, h + o, (size_t)std::min<u64>(FETCH_CHUNK, bytes - o)});
   }
-  const uint32_t slots = fetch_slots_, total = (uint32_t)parts.size();
-  std::atomic<uint32_t> arrived{0}, taken{0};
-  std::vector<std::atomic<uint8_t>> stored(total);
-  for (auto &s : stored) s.store(0, std::memory_order_relaxed);
-  auto store_one = [&]() {  // the next chunk that nobody has taken; false: none left
-    const uint32_t i = taken.fetch_add(1);
-    if (i >= total) return false;
-    while (arrived.load(std::memory_order_acquire) <= i) std::this_thread::yield();
-    if (arrived.load(std::memory_order_acquire) <= total)  // (above: the copies failed)
-      std::memcpy(parts[i].h, h_fetch_ + (u64)(i % slots) * FETCH_CHUNK, parts[i].n);
-    stored[i].store(1, std::memory_order_release);
-    return true;
-  };
-  auto send = [&](uint32_t i) {
-    cudaError_t x = cudaMemcpyAsync(h_fetch_ + (u64)(i % slots) * FETCH_CHUNK, parts[i].d,
-                                    parts[i].n, cudaMemcpyDeviceToHost, st_);
-    return x != cudaSuccess ? x : cudaEventRecord(fetch_ev_[i % slots], st_);
-  };
-  cudaError_t x = cudaSuccess;
-  for (uint32_t i = 0; i < std::min(slots, total) && x == cudaSuccess; i++) x = send(i);
-  std::vector<std::thread> crew;
-  try {
-    for (int t = 0; t < 3 && x == cudaSuccess; t++)
-      crew.emplace_back([&]() {
-        while (store_one()) {
-        }
-      });
-  } catch (const std::system_error &) {
-    // fewer helpers, or none: this thread stores what is left
-  }
-  for (uint32_t i = 0; i < total && x == cudaSuccess; i++) {
-    x = cudaEventSynchronize(fetch_ev_[i % slots]);
-    if (x != cudaSuccess) break;
-    arrived.store(i + 1, std::memory_order_release);
-    if (crew.empty()) store_one();
-    // slots freed meanwhile (in order) take the chunks that follow
-    if (i + slots < total) {
-      while (!stored[i].load(std::memory_order_acquire)) std::this_thread::yield();
-      x = send(i + slots);
-    }
-  }
-  if (x != cudaSuccess) arrived.store(total + 1, std::memory_order_release);
-  for (std::thread &t : crew) t.join();
+  const uint32_t slots = fetch_slots_;
+  const auto slot = [&](uint32_t i) { return h_fetch_ + (u64)(i % slots) * FETCH_CHUNK; };
+  const int x = run_ring(
+      (uint32_t)parts.size(), slots,
+      [&](uint32_t i) {
+        const cudaError_t e =
+            cudaMemcpyAsync(slot(i), parts[i].d, parts[i].n, cudaMemcpyDeviceToHost, st_);
+        return (int)(e != cudaSuccess ? e : cudaEventRecord(fetch_ev_[i % slots], st_));
+      },
+      [&](uint32_t i) { return (int)cudaEventSynchronize(fetch_ev_[i % slots]); },
+      [&](uint32_t i) { std::memcpy(parts[i].h, slot(i), parts[i].n); });
   cudaStreamSynchronize(st_);
-  CK(x);
+  CK((cudaError_t)x);
 }
 
 // ---- mapping autotuner and multi-snapshot replay ------------------------------
