@@ -114,15 +114,16 @@ void Engine::join_staging() {
 
 void *Engine::dmalloc(size_t bytes) {
   void *p = nullptr;
-  CK(cudaMalloc(&p, std::max<size_t>(bytes, 16)));
-  dallocs_.push_back(p);
+  bytes = std::max<size_t>(bytes, 16);
+  CK(cudaMalloc(&p, bytes));
+  dallocs_.push_back({p, bytes});
   return p;
 }
 
 void Engine::dfree_all() {
-  for (void *p : dallocs_) cudaFree(p);
+  for (const Alloc &a : dallocs_) cudaFree(a.p);
   dallocs_.clear();
-  for (void *p : batch_allocs_) cudaFree(p);
+  for (const Alloc &a : batch_allocs_) cudaFree(a.p);
   batch_allocs_.clear();
 }
 
@@ -210,7 +211,8 @@ void Engine::build_direction(Arena &A, const u64 *keys, const uint32_t *wv, u64 
   sync_check("scatter");
   // free the temporaries (they are the last allocations made)
   for (void *p : {temp, (void *)rowstart, (void *)cap64, (void *)deg}) {
-    auto it = std::find(dallocs_.begin(), dallocs_.end(), p);
+    auto it = std::find_if(dallocs_.begin(), dallocs_.end(),
+                           [&](const Alloc &a) { return a.p == p; });
     if (it != dallocs_.end()) dallocs_.erase(it);
     cudaFree(p);
   }
@@ -642,15 +644,16 @@ void Engine::reserve_batch(size_t max_records) {
 void Engine::ensure_batch(size_t cnt) {
   if (cnt <= bcap_) return;
   drop_graphs();  // captured graphs hold the old buffers
-  for (void *p : batch_allocs_) cudaFree(p);
+  for (const Alloc &a : batch_allocs_) cudaFree(a.p);
   batch_allocs_.clear();
   size_t c = std::max<size_t>(cnt, 1024);
   c = std::max(c, bcap_ * 2);
   bcap_ = 0;  // nothing is held until all of it is: an allocation below may fail
   auto al = [&](size_t bytes) {
     void *p = nullptr;
-    CK(cudaMalloc(&p, std::max<size_t>(bytes, 16)));
-    batch_allocs_.push_back(p);
+    bytes = std::max<size_t>(bytes, 16);
+    CK(cudaMalloc(&p, bytes));
+    batch_allocs_.push_back({p, bytes});
     return p;
   };
   const size_t dirs = has_in_ ? 2 : 1;
@@ -1030,8 +1033,6 @@ void Engine::set_queries(const uint32_t *sources, uint32_t count, uint32_t mode)
     apool_cap_ = 65535;
     apool_ = (uint32_t *)dmalloc((u64)apool_cap_ * nb * 4);
     qnb_ = nb;
-    qbytes_ = (u64)Q * 4 + n * Q * 8 + 6 * n * nb * 4 + (u64)mtile_cap_ * sizeof(uint4) +
-              (u64)aring_cap_ * 8 + n * 4 + (u64)apool_cap_ * nb * 4;
   } else {
     d_sources_ = (uint32_t *)dmalloc((u64)count * 4);
     CK(cudaMemcpyAsync(d_sources_, sources, (u64)count * 4, cudaMemcpyHostToDevice, st_));
@@ -1041,7 +1042,6 @@ void Engine::set_queries(const uint32_t *sources, uint32_t count, uint32_t mode)
     CK(cudaHostAlloc(&hq, (u64)count * sizeof(Ctl), cudaHostAllocDefault));
     hallocs_.push_back(hq);
     h_qctl_ = (Ctl *)hq;
-    qbytes_ = (u64)count * 4 + n * count * 8 + (u64)count * sizeof(Ctl);
   }
   seq_ = (uint32_t *)dmalloc(8);
   void *hs = nullptr;
@@ -1626,7 +1626,6 @@ void Engine::policy_alloc() {
   CK(cudaEventCreate(&pev_[0]));
   CK(cudaEventCreate(&pev_[1]));
   sync_check("policy alloc");
-  policy_bytes_ = np * (POLICY_F * 2 + 16 + 1 + 12) + 4ull * POLICY_PARAMS * 4;
 }
 
 void Engine::set_cache_policy(uint32_t policy) {
@@ -2006,9 +2005,11 @@ void Engine::info(dycg_graph_info *out) {
   out->cache_slots = cache_slots_;
   out->cached_pages = cache_slots_ ? cache_slots_ - cwk_.h_plan->free_count : 0;
   out->host_bytes = out->arena_slots * 4 * out_.stride;
-  out->device_bytes = (u64)n_ * (8 + 4 * 6) + (u64)n_ * (has_in_ ? 48 : 24) +
-                      ((u64)cache_slots_ << page_shift_) * 4 * out_.stride + index_bytes_ +
-                      qbytes_ + policy_bytes_;
+  // every buffer: state, descriptors, cache and index, queues, batch lists, traces
+  u64 held = hrec_bytes_ + (u64)trace_cap_ * npages_ * (POLICY_F * 2 + 4);
+  for (const std::vector<Alloc> *v : {&dallocs_, &batch_allocs_})
+    for (const Alloc &a : *v) held += a.bytes;
+  out->device_bytes = held;
   out->reserved[0] = index_bytes_;  // fence index + deletion bitmap (part of the budget)
   out->page_shift = page_shift_;
   out->has_incoming = has_in_ ? 1 : 0;

@@ -140,7 +140,11 @@ class Engine {
   uint32_t n_ = 0;
   bool loaded_ = false, inited_ = false, has_in_ = false, stored_ = false;
   Arena out_, in_;
-  std::vector<void *> dallocs_;
+  struct Alloc {
+    void *p;
+    size_t bytes;
+  };
+  std::vector<Alloc> dallocs_;
   std::vector<void *> hallocs_;
 
   // cache
@@ -180,7 +184,6 @@ class Engine {
   uint32_t aring_cap_ = 0, apool_cap_ = 0;
   uint32_t *ainq_ = nullptr, *apool_ = nullptr;
   uint32_t qratio_ = 4, heavy_ = 64, tile_ = 4096, pull_qratio_ = 4, sched_ = 0;
-  u64 qbytes_ = 0;
   bool tune_ = false;
   std::vector<dycg_query_mapping> tried_;
   // multi-snapshot replay: one graph per padded batch-size class
@@ -208,7 +211,6 @@ class Engine {
   uint32_t learned_cap_div_ = 256;
   uint32_t *pperiod_ = nullptr;  // device {snapshot counter, refresh period} of the layout features
   cudaEvent_t pev_[2] = {};
-  u64 policy_bytes_ = 0;
 
   // batch buffers
   size_t bcap_ = 0;
@@ -224,7 +226,7 @@ class Engine {
   uint32_t *rem_[2] = {}, *matches_[2] = {};
   BatchHdr *d_hdr_ = nullptr, *h_hdr_ = nullptr;  // header, records behind it
   dycg_edge_dev *d_edges_ = nullptr;
-  std::vector<void *> batch_allocs_;
+  std::vector<Alloc> batch_allocs_;
   uint64_t launches_ = 0;
 };
 
