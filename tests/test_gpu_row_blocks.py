@@ -72,3 +72,38 @@ def test_hub_larger_than_the_headroom(incoming, stored):
         assert h.apply(gone, spare)["insertions"] == step
         spare = gone
     h.check()
+
+
+def test_rows_past_half_of_the_headroom_stay_when_they_fit():
+    # 60,000 rows alike, so one row is the model of all of them. Their first growth, to
+    # blocks of 16, takes 960,000 of the 2^20 spare slots; from then on a full row whose
+    # live occurrences and a reserve fit stays, more than half full or not
+    rows, n = 60_000, 60_040
+    row = list(range(rows, rows + 7))
+    off = np.minimum(np.arange(n + 1), rows).astype(np.uint64) * 7
+    e = dg.Engine("pr", epsilon=1.0)  # (no incoming rows, nothing to repair)
+    e.load_csr(n, off, np.tile(np.array(row, np.uint32), rows))
+    e.start()
+    first = e.info()
+
+    def records(targets):
+        u = np.repeat(np.arange(rows), len(targets))
+        return np.stack([u, np.tile(targets, rows), np.ones(len(u))], 1).astype(np.uint32)
+
+    def step(gone, new):
+        st = e.apply_batch(records(gone), records(new))
+        assert st["missing_deletes"] == 0
+        for v in gone:
+            row.remove(v)
+        row.extend(sorted(new))
+        o, dst, _ = e.csr()
+        assert (np.diff(o.astype(np.int64))[:rows] == len(row)).all()
+        assert (dst.reshape(rows, -1) == np.array(row, np.uint32)).all()
+        return st["relocated_rows"], e.info()["arena_used"] - first["arena_used"]
+
+    assert step([], [rows + 30, rows + 9]) == (rows, 16 * rows)
+    gone = row[1:8:2]
+    assert step(gone, [rows + 20 + i for i in range(6)]) == (0, 16 * rows)  # 9 + 6 slots
+    for _ in range(6):  # 11 of 16 slots live, three deleted and three inserted each time
+        moved = step(row[::3][:3], [v for v in range(rows, rows + 40) if v not in row][:3])
+        assert moved == (0, 16 * rows)
