@@ -1,5 +1,7 @@
 """dycg_graph_info.device_bytes counts every device buffer the engine holds, the row and
 chunk lists of a batch included, as the device's own figure of free memory shows."""
+import gc
+
 import numpy as np
 import pytest
 import torch
@@ -27,6 +29,7 @@ def test_device_bytes_is_what_the_device_gave(queries):
         return e
 
     build().close()  # (code, and what the runtime keeps for itself)
+    gc.collect()     # (engines that earlier tests left open)
     free0, _ = torch.cuda.mem_get_info()
     e = build()
     free1, _ = torch.cuda.mem_get_info()

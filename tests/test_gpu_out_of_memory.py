@@ -1,6 +1,8 @@
 """Device memory that runs out inside a call, made by holding nearly all of it in
 another allocation: the call returns its error, and what follows is either refused
 (the snapshot was under way) or right (it was not)."""
+import gc
+
 import numpy as np
 import pytest
 import torch
@@ -18,6 +20,7 @@ class Held:
     """All device memory but LEFT bytes."""
 
     def __enter__(self):
+        gc.collect()
         torch.cuda.empty_cache()
         free, _ = torch.cuda.mem_get_info()
         self.block = torch.empty(free - LEFT, dtype=torch.uint8, device="cuda")
