@@ -4,7 +4,7 @@
 // (include/framework/framework.cuh:780-6112) for one path: load a graph into
 // the paged pinned store, solve once, then per snapshot ingest + mutate +
 // repair + cache maintenance, all on one CUDA stream with one host
-// synchronisation at the end of a batch (two when the cache refreshes).
+// synchronisation at the end of a batch.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -549,8 +549,8 @@ void Engine::init() {
     init_queries(timeout);
     inited_ = true;
     cache_maintenance(true);
-  sync_check("first cache load");
-  maintenance_stats(nullptr);
+    sync_check("first cache load");
+    maintenance_stats(nullptr);
     return;
   }
   if (opt_.algo == DYCG_ALGO_PR) {
@@ -629,7 +629,7 @@ void Engine::reserve_batch(size_t max_records) {
   check_loaded();
   if (max_records > 0x3FFFFFFFull) throw Error(DYCG_EINVAL, "batch too large");
   if (inited_ && nq_ && qmode_ == DYCG_QUERIES_BATCHED) {
-    // multi-snapshot replay: buffers for the largest padding class, and the
+    // multi-snapshot replay: buffers for the largest size class, and the
     // graph of every class up to it captured now rather than on first use
     uint32_t top = 1024;
     while (top < max_records) top *= 2;

@@ -186,7 +186,7 @@ class Engine {
   uint32_t qratio_ = 4, heavy_ = 64, tile_ = 4096, pull_qratio_ = 4, sched_ = 0;
   bool tune_ = false;
   std::vector<dycg_query_mapping> tried_;
-  // multi-snapshot replay: one graph per padded batch-size class
+  // multi-snapshot replay: one graph per batch-size class
   std::map<uint32_t, SnapshotGraph> graphs_;
   std::vector<cudaEvent_t> bev_;
   Ctl *h_bctl_ = nullptr;

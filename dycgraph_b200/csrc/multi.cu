@@ -26,9 +26,9 @@
 // its (chunk, query group) pairs; a query-lane tile's warps split its chunks.
 // Per query the phases are the single-query repair's (repair.cu): deletion
 // seeds (parent == u), invalidation waves over out-rows (resetting as they
-// mark), pull over in-rows with the insertion seeds, push closure. The batched form has no
-// counterpart in the reference engine, which repairs one source per engine
-// (include/framework/framework.cuh:1803 InitGraph(src)).
+// mark), pull over in-rows with the insertion seeds, push closure. The batched
+// form has no counterpart in the reference engine, which repairs one source per
+// engine (include/framework/framework.cuh:1803 InitGraph(src)).
 #include "frontier.cuh"
 #include "internal.h"
 
@@ -135,7 +135,7 @@ __device__ __forceinline__ void note_affected(const MultiParams &P, uint32_t y, 
 // Slots [b, e) of the row at `off`, `stride` apart per lane: each lane loads
 // its slot UNROLL chunks ahead of use, then the converged warp calls
 // visit(id, weight, valid). Charges traffic and per-page hotness like
-// warp_slots (frontier.cuh).
+// group_slots (frontier.cuh).
 template <bool WITH_W, class Visit>
 __device__ __forceinline__ void walk(const Adj &A, u64 off, uint32_t b, uint32_t e,
                                      uint32_t stride, Visit &visit, Acc &acc) {
@@ -969,8 +969,9 @@ __device__ bool async_phase(const MultiParams &P, const Adj &A, const uint32_t *
 }
 
 // CTAs per SM the register allocation is sized for at 8 blocks of queries:
-// 3 (85 registers, ~140 bytes of spills per thread) measured ~3% faster on
-// the R-MAT 24 / 256-query workload than 2 (104 registers, no spills)
+// 3 (80 registers, 136 bytes of spills per thread with stored weights, 344 with
+// the rule's) measured ~3% faster on the R-MAT 24 / 256-query workload than 2
+// (104 registers, no spills)
 #ifndef DYCG_MULTI_MIN_BLOCKS
 #define DYCG_MULTI_MIN_BLOCKS 3
 #endif

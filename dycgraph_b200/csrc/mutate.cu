@@ -6,25 +6,27 @@
 // BuildDeletionPlan :685-739): a deletion requested r times removes r live
 // occurrences (fewer if fewer exist: the rest are counted missing), additions
 // append occurrences, and a row whose block is full drops its deleted slots and,
-// if it outgrew the block, moves to a new power-of-two block at the arena tail. Rows stay sorted in their prefix, so
-// a deletion finds its target through the HBM fence index and one 128-byte
-// read of the row instead of the reference's linear row scan. A deletion sets
-// a bit of the HBM deletion bitmap (no host-link write).
+// if it outgrew the block, moves to a new power-of-two block at the arena tail.
+// Rows stay sorted in their prefix, so a deletion finds its target through the
+// HBM fence index and one 128-byte read of the row instead of the reference's
+// linear row scan. A deletion sets a bit of the HBM deletion bitmap (no host-link
+// write).
 //
 // One cooperative launch mutates both directions: deletions and the inserted
 // slots, a barrier, [long suffixes: two passes with a barrier each], the
-// insertions' descriptors, a barrier, [relocated rows]. Bracketed phases run only when the batch needs them, which
-// the barriers' published counters decide, so a snapshot needs no host
+// insertions' descriptors, a barrier, [full rows; long ones by the whole grid, with
+// barriers of their own]. Bracketed phases run only when the batch needs them,
+// which the barriers' published counters decide, so a snapshot needs no host
 // synchronisation and a captured one takes the same path. What bounds it is the
 // host link's random transactions, one per deletion and one per insertion and
 // direction (3.4 ns each over a 1 GB arena: 0.68 ms of the 0.77 ms that phase 1
 // takes for 100K updates at R-MAT 21), and the chain of dependent accesses (~6
 // us) for small batches: so an 8-lane group serves a deletion (a 128-byte line
-// per step), a lane an insertion row, and a small batch spreads over all SMs.
+// per step), a lane an insertion row, and a small batch spreads over the SMs.
 // Mutation per snapshot, before (a warp per record, a launch per step and
-// direction, two host synchronisations) -> now: 32 updates 0.115 -> 0.022 ms,
-// R-MAT 16 2K 0.140 -> 0.063, R-MAT 20 BFS 10K 0.20 -> 0.12, R-MAT 21 100K 1.62 ->
-// 1.14.
+// direction, two host synchronisations) -> now: 32 updates 0.115 -> 0.019 ms,
+// R-MAT 16 2K 0.140 -> 0.063 (0.10 after some hundred snapshots, when most rows
+// are suffix), R-MAT 20 BFS 10K 0.20 -> 0.12, R-MAT 21 100K 1.62 -> 1.14.
 #include "frontier.cuh"
 #include "internal.h"
 #include "mutation_grid.h"
@@ -432,10 +434,11 @@ __device__ __forceinline__ u64 reserve_block(const Adj &A, uint32_t slots) {
 
 // Then, the deletions done, the descriptors. A row that does not fit drops its
 // deleted slots on its way to a new power-of-two block (with headroom) at the
-// arena tail, or in its own block: when they are half of it (the copy then pays
-// for itself), once the block that its slots ask for would reach into the second half
-// of the arena's headroom, whenever the live occurrences and a reserve fit, and
-// whenever they fit at all if the arena has no such block left. So a row takes
+// arena tail, or in its own block: when they are half of it (the copy of a block is
+// then paid for by half as many appends before the next one; 5/8 and 3/4 took the
+// same time in every stream), once the block that its slots ask for would reach into
+// the second half of the arena's headroom, whenever the live occurrences and a reserve
+// fit, and whenever they fit at all if the arena has no such block left. So a row takes
 // space for good only when its live occurrences outgrow its block (2,000-update
 // snapshots on R-MAT 16 used to eat the arena in some 5,000 of them), no row asks
 // in vain for a larger block than it needs, and no repair reads a slot deleted

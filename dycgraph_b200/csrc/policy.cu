@@ -173,6 +173,7 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 // other's load, MMA and barrier latencies. 1.85M pages: 104 us with scalar
 // epilogues and A in shared memory, 77 now (half the issue slots; the rest is the
 // chain load - MMA - epilogue - MMA - epilogue of the four groups in flight).
+// 512 threads leave 128 registers each, which spills 60 bytes a thread.
 // The weights sit in shared memory in the no-swizzle K-major layout of 8-row x
 // 16-byte core matrices:
 // element (row, k) of an operand with KC chunks of 8 along K lives at

@@ -96,7 +96,8 @@ __device__ __forceinline__ void push_only(const PrParams *P, const uint32_t (&y)
 // less than a returned value, a crossing test and a queue append per push. A
 // frontier is the vertices with |r| > eps either way (outside the frontier none
 // is above it when a round begins, and a vertex that crossed and came back is
-// dropped when it is consumed), so the rounds push the same values.
+// dropped when it is consumed), so the rounds push the same values. It is worth
+// little: 1.67 against 1.71 ms of an R-MAT 18 snapshot's kernel without the rule.
 constexpr uint32_t DENSE = 16;
 
 __device__ __forceinline__ uint32_t old_degree(const PrParams *P, uint32_t u) {

@@ -235,7 +235,8 @@ struct RelaxOp {
 // merged phases and the batched accesses, kernel time per snapshot before ->
 // now: R-MAT 16 SSSP 2K updates 0.24 -> 0.14 ms, R-MAT 20 BFS 10K 0.24 -> 0.12
 // ms, R-MAT 21 SSSP 100K 0.73 -> 0.36 ms, 1024^2 grid SSSP 1K (1,580 ordered
-// waves) 39.4 -> 20.2 ms.
+// waves) 39.4 -> 20.2 ms. 1024 threads leave 64 registers each: CC and
+// stored-weight SSSP spill 164 and 172 bytes a thread, BFS and rule-weight SSSP 56.
 template <uint32_t ALGO, bool STORED>
 __global__ void __launch_bounds__(REPAIR_BLOCK, 1) repair_kernel(const __grid_constant__ RepairParams P) {
   Ctl *ctl = P.ctl;
