@@ -271,7 +271,11 @@ constexpr uint32_t GROUP_ROW = 64;
 // Static: warp k of every block before warp k + 1 of any, so that a short wave
 // spreads over all SMs; one item per warp while the wave fits (its latency is
 // one row's), up to four per warp above (short rows leave most of 32 lanes
-// idle).
+// idle). Where admit can say no (Op::SIFTS) and there are 32 items per warp, a lane
+// asks for each: most of a long ordered queue is only carried to the next wave. CC
+// on the 4096^2 grid, some ten million items in ~800 waves: asked four at a time 3.0
+// ms a wave (2,422-3,219 ms of repair a snapshot), 32 at a time 0.50 (539), from
+// 128 items per warp on 0.67. Its SSSP, whose waves are short: 338 ms either way.
 template <bool WITH_W, class Op>
 __device__ Snap expand_rows(const Adj &A, const uint32_t *items, uint32_t cnt, Op &op, Acc &acc,
                             Tiles T, Ctl *ctl, uint32_t &gen, uint32_t sel, uint32_t reset_flags,
@@ -281,23 +285,8 @@ __device__ Snap expand_rows(const Adj &A, const uint32_t *items, uint32_t cnt, O
   const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
   const uint32_t per = claimed || cnt <= nw ? 1u : cnt <= 2 * nw ? 2u : 4u;
   const uint32_t grp = lane >> 3;
-  uint32_t i = gw * per;
-  if (claimed) {
-    if (lane == 0) i = atomicAdd(&ctl->grab, 1u);
-    i = __shfl_sync(0xffffffffu, i, 0);
-  }
-  while (i < cnt) {
-    const bool have = grp < per && i + grp < cnt;
-    const uint32_t v = have ? __ldcg(items + i + grp) : 0u;
-    if (claimed) {
-      if (lane == 0) i = atomicAdd(&ctl->grab, 1u);
-      i = __shfl_sync(0xffffffffu, i, 0);
-    } else {
-      i += nw * per;
-    }
-    const uint32_t len = have ? A.len[v] : 0u;
-    const u64 off = have ? A.off[v] : 0ull;
-    const bool on = op.admit(v, have);
+  // the rows of up to four items, one per 8-lane group
+  const auto expand = [&](uint32_t v, uint32_t len, u64 off, bool on) {
     const bool small = per > 1 && len <= GROUP_ROW;
     if (__any_sync(0xffffffffu, on && small))
       group_slots<8, WITH_W>(A, v, on && small, off, 0, len, 8, op, acc);
@@ -324,6 +313,44 @@ __device__ Snap expand_rows(const Adj &A, const uint32_t *items, uint32_t cnt, O
       }
       group_slots<32, WITH_W>(A, bv, true, bo, 0, bl, 32, op, acc);
     }
+  };
+  uint32_t i = gw * per;
+  if (claimed) {
+    if (lane == 0) i = atomicAdd(&ctl->grab, 1u);
+    i = __shfl_sync(0xffffffffu, i, 0);
+  }
+  if constexpr (Op::SIFTS) {
+    if (!claimed && cnt / 32 >= nw) {
+      // eight of the rounds below at once: lane l has item l % 4 of round l / 4
+      for (; i < cnt; i += nw * 32) {
+        const uint32_t at = i + (lane >> 2) * (nw * 4) + (lane & 3);
+        const uint32_t iv = at < cnt ? __ldcg(items + at) : 0u;
+        unsigned left = __ballot_sync(0xffffffffu, op.template admit<1>(iv, at < cnt));
+        while (left) {
+          int src = -1;
+#pragma unroll
+          for (uint32_t g = 0; g < 4; g++) {
+            if (g == grp) src = __ffs(left) - 1;
+            left &= left - 1;
+          }
+          const uint32_t v = __shfl_sync(0xffffffffu, iv, src & 31);
+          expand(v, src >= 0 ? A.len[v] : 0u, src >= 0 ? A.off[v] : 0ull, src >= 0);
+        }
+      }
+    }
+  }
+  while (i < cnt) {
+    const bool have = grp < per && i + grp < cnt;
+    const uint32_t v = have ? __ldcg(items + i + grp) : 0u;
+    if (claimed) {
+      if (lane == 0) i = atomicAdd(&ctl->grab, 1u);
+      i = __shfl_sync(0xffffffffu, i, 0);
+    } else {
+      i += nw * per;
+    }
+    const uint32_t len = have ? A.len[v] : 0u;
+    const u64 off = have ? A.off[v] : 0ull;
+    expand(v, len, off, op.template admit<8>(v, have));
   }
   // The items have been consumed: the queue resets can apply here. When no row
   // was heavy this barrier's snapshot already holds every append of the

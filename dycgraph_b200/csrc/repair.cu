@@ -68,6 +68,8 @@ template <uint32_t ALGO>
 struct InvalidateOp {
   const RepairParams *P;
   struct Row {};
+  static constexpr bool SIFTS = false;
+  template <int G>
   __device__ bool admit(uint32_t, bool on) { return on; }
   template <int G>
   __device__ bool begin(uint32_t, bool on, Row &) { return on; }
@@ -105,13 +107,15 @@ __device__ __forceinline__ void note_min(Ctl *ctl, uint32_t value) {
 // closure's first frontier when it has a value (a CC vertex always has its own
 // id). A vertex lowered later, by an insertion seed of the same phase, enters
 // it through that seed.
-template <uint32_t ALGO, bool STORED>
+template <uint32_t ALGO, bool STORED, bool ORDERED>
 struct PullOp {
   const RepairParams *P;
   uint32_t tag;
   struct Row {
     u64 best;
   };
+  static constexpr bool SIFTS = false;
+  template <int G>
   __device__ bool admit(uint32_t, bool on) { return on; }
   template <int G>
   __device__ bool begin(uint32_t, bool on, Row &r) {
@@ -151,17 +155,17 @@ struct PullOp {
       if (m != KEY_INF) lower_from<Strict<ALGO, STORED>::value>(P->key + v, m, ld_key(P->key + v));
       want[0] = atomicExch(P->wtag + v, tag) != tag;
     }
-    if (P->delta)
+    if (ORDERED)
       note_min(P->ctl, want[0] ? min(key_value(m), ALGO == ALGO_CC ? v : INF32) : INF32);
     append_batch(P->q[0], &P->ctl->q_count[0], P->n, want, val, &P->ctl->err);
   }
 };
 
 // Push relaxation of the out-edges of a frontier vertex. In the ordered
-// closure (P->delta) only vertices below thr are expanded: the others are
+// closure only vertices below thr are expanded: the others are
 // carried to the next queue, and every carried value and improvement lowers
 // the next wave's minimum.
-template <uint32_t ALGO, bool STORED>
+template <uint32_t ALGO, bool STORED, bool ORDERED>
 struct RelaxOp {
   const RepairParams *P;
   uint32_t *outq;
@@ -172,12 +176,15 @@ struct RelaxOp {
   struct Row {
     uint32_t dv, imp;  // the vertex's value; the lowest value this lane pushed
   };
+  static constexpr bool SIFTS = ORDERED;
+  // groups of G lanes hold the same item
+  template <int G>
   __device__ bool admit(uint32_t v, bool on) {
-    if (!P->delta) return on;
-    const bool lead = (lane_id() & 7) == 0;  // a group's lanes hold the same item
+    if (!ORDERED) return on;
+    const bool lead = (lane_id() & (G - 1)) == 0;
     const uint32_t d = on ? key_value(ld_key(P->key + v)) : INF32;
     // one read decides for the whole group
-    const uint32_t dv = __shfl_sync(0xffffffffu, d, 0, 8);
+    const uint32_t dv = G == 1 ? d : __shfl_sync(0xffffffffu, d, 0, G);
     const bool later = on && dv != INF32 && dv >= thr;
     if (__any_sync(0xffffffffu, later)) {
       const uint32_t val[1] = {v};
@@ -225,7 +232,7 @@ struct RelaxOp {
   }
   template <int G>
   __device__ void end(uint32_t, bool, Row &r) {
-    if (P->delta) note_min(P->ctl, r.imp);
+    if (ORDERED) note_min(P->ctl, r.imp);
   }
 };
 
@@ -236,9 +243,11 @@ struct RelaxOp {
 // now: R-MAT 16 SSSP 2K updates 0.24 -> 0.14 ms, R-MAT 20 BFS 10K 0.24 -> 0.12
 // ms, R-MAT 21 SSSP 100K 0.73 -> 0.36 ms, 1024^2 grid SSSP 1K (1,580 ordered
 // waves) 39.4 -> 20.2 ms. 1024 threads leave 64 registers each: CC and
-// stored-weight SSSP spill 164 and 172 bytes a thread, BFS and rule-weight SSSP 56.
-template <uint32_t ALGO, bool STORED>
-__global__ void __launch_bounds__(REPAIR_BLOCK, 1) repair_kernel(const __grid_constant__ RepairParams P) {
+// stored-weight SSSP spill 172 and 164 bytes a thread, BFS and rule-weight SSSP 48
+// and 44 (ordered: 284 and 300, 136).
+template <uint32_t ALGO, bool STORED, bool ORDERED>
+__global__ void __launch_bounds__(REPAIR_BLOCK, 1)
+    repair_kernel(const __grid_constant__ RepairParams P) {
   Ctl *ctl = P.ctl;
   Acc acc = {0, 0, 0, 0, 0};
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -304,21 +313,21 @@ __global__ void __launch_bounds__(REPAIR_BLOCK, 1) repair_kernel(const __grid_co
           }
         }
       }
-      if (P.delta) note_min(ctl, imp);
+      if (ORDERED) note_min(ctl, imp);
       append_batch(P.q[0], &ctl->q_count[0], P.n, want, v, &ctl->err);
     }
     // the seeds' share of the phase: until the first warp, which has as many as any,
     // is through with its own
     if (gtid == 0) ctl->tphase[1] = globaltimer_ns();
   }
-  if (!(P.phases & (PH_DELETE | PH_INSERT)) && P.delta) {
+  if (ORDERED && !(P.phases & (PH_DELETE | PH_INSERT))) {
     // static solve: the minimum of the frontier it was given
     const uint32_t cnt = *(volatile uint32_t *)&ctl->q_count[0];
     for (uint32_t i0 = first; i0 < cnt; i0 += gstride)
       note_min(ctl, i0 + lane < cnt ? key_value(ld_key(P.key + P.q[0][i0 + lane])) : INF32);
   }
   if (na) {
-    PullOp<ALGO, STORED> op{&P, tag_base};
+    PullOp<ALGO, STORED, ORDERED> op{&P, tag_base};
     sn = expand_rows<STORED>(P.in, P.aff, na, op, acc, P.tiles, ctl, gen, SEL_Q0, SYNC_RESET_VMIN,
                              P.timeout_ns, P.claimed);
   } else {
@@ -326,7 +335,7 @@ __global__ void __launch_bounds__(REPAIR_BLOCK, 1) repair_kernel(const __grid_co
   }
   if (!sn.ok) goto done;
   if (gtid == 0) ctl->tphase[2] = globaltimer_ns();  // pull done
-  // 4. closure waves. Ordered (P.delta, for high-diameter graphs, the B200 form
+  // 4. closure waves. Ordered (P.delta > 0, for high-diameter graphs, the B200 form
   // of the reference's ordered insertion schedule, framework.cuh:537-556): each
   // wave expands only the frontier vertices whose value is below the wave's
   // minimum + delta and carries the rest to the next wave, so a vertex is
@@ -342,7 +351,8 @@ __global__ void __launch_bounds__(REPAIR_BLOCK, 1) repair_kernel(const __grid_co
         break;
       }
       const uint32_t thr = sn.vmin > INF32 - P.delta ? INF32 : sn.vmin + P.delta;
-      RelaxOp<ALGO, STORED> op{&P, P.q[cur ^ 1], &ctl->q_count[cur ^ 1], tag_base + 1 + wave, thr};
+      RelaxOp<ALGO, STORED, ORDERED> op{&P, P.q[cur ^ 1], &ctl->q_count[cur ^ 1],
+                                        tag_base + 1 + wave, thr};
       sn = expand_rows<STORED>(P.out, P.q[cur], sn.cnt, op, acc, P.tiles, ctl, gen,
                                cur ? SEL_Q0 : SEL_Q1,
                                (cur ? SYNC_RESET_Q1 : SYNC_RESET_Q0) | SYNC_RESET_VMIN,
@@ -385,7 +395,7 @@ __global__ void init_state_kernel(u64 *key, uint32_t n, uint32_t source, uint32_
   }
 }
 
-template <uint32_t ALGO, bool STORED>
+template <uint32_t ALGO, bool STORED, bool ORDERED>
 static cudaError_t launch_one(const RepairLaunch &L, cudaStream_t s) {
   RepairParams P;
   P.out = L.out;
@@ -415,23 +425,31 @@ static cudaError_t launch_one(const RepairLaunch &L, cudaStream_t s) {
   static int blocks_per_sm = -1;
   if (blocks_per_sm < 0) {
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &blocks_per_sm, repair_kernel<ALGO, STORED>, REPAIR_BLOCK, 0);
+        &blocks_per_sm, repair_kernel<ALGO, STORED, ORDERED>, REPAIR_BLOCK, 0);
     if (e != cudaSuccess) return e;
   }
   const int grid = blocks_per_sm * L.num_sms;
   void *args[] = {&P};
-  return cudaLaunchCooperativeKernel((const void *)repair_kernel<ALGO, STORED>, grid,
+  return cudaLaunchCooperativeKernel((const void *)repair_kernel<ALGO, STORED, ORDERED>, grid,
                                      REPAIR_BLOCK, args, 0, s);
+}
+
+// Kernels of their own for the two closures: what only the ordered one needs costs the
+// other no registers.
+template <uint32_t ALGO, bool STORED>
+static cudaError_t launch_closure(const RepairLaunch &L, cudaStream_t s) {
+  return L.delta ? launch_one<ALGO, STORED, true>(L, s) : launch_one<ALGO, STORED, false>(L, s);
 }
 
 cudaError_t launch_repair(const RepairLaunch &L, cudaStream_t s) {
   switch (L.algo) {
     case ALGO_SSSP:
-      return L.stored ? launch_one<ALGO_SSSP, true>(L, s) : launch_one<ALGO_SSSP, false>(L, s);
+      return L.stored ? launch_closure<ALGO_SSSP, true>(L, s)
+                      : launch_closure<ALGO_SSSP, false>(L, s);
     case ALGO_BFS:
-      return launch_one<ALGO_BFS, false>(L, s);
+      return launch_closure<ALGO_BFS, false>(L, s);
     case ALGO_CC:
-      return launch_one<ALGO_CC, false>(L, s);
+      return launch_closure<ALGO_CC, false>(L, s);
     default:
       return cudaErrorInvalidValue;
   }

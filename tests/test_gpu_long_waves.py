@@ -1,0 +1,81 @@
+"""Ordered closures whose wave queues are long: at the line from which a lane asks for
+each item of the queue (32 per warp of the launch), against the fixed point, and the
+time of a wave that carries millions of items."""
+import numpy as np
+import pytest
+
+import dycgraph_b200 as dg
+from tests import cases
+
+pytestmark = pytest.mark.gpu
+LINE = 148 * 32 * 32  # items: SMs x warps x 32
+
+
+def fan(width):
+    """0 -> 1..width (weights 1..64), each of which points at two of the next 30,000
+    vertices (some of these have hundreds of in-edges) and those at one another."""
+    rng = np.random.default_rng(width)
+    n = width + 30_001
+    mid = np.arange(1, width + 1)
+    u = np.concatenate([np.zeros(width, np.int64), np.repeat(mid, 2), np.arange(width + 1, n)])
+    v = np.concatenate([mid, width + 1 + (rng.random(2 * width) ** 3 * 30_000).astype(np.int64),
+                        rng.integers(width + 1, n, 30_000)])
+    key = np.unique(u * n + v)
+    u, v = key // n, key % n
+    off = np.concatenate([[0], np.bincount(u, minlength=n).cumsum()]).astype(np.uint64)
+    return n, off, v.astype(np.uint32), cases.hw(u, v)
+
+
+def solve(algo, n, u, v, w):
+    """Distances from 0, levels from 0, or least labels, by relaxing every edge until
+    nothing changes (a few rounds on these graphs)."""
+    inf = 0xFFFFFFFF
+    x = np.arange(n, dtype=np.int64) if algo == "cc" else np.full(n, inf, np.int64)
+    x[0] = 0
+    step = {"sssp": w.astype(np.int64), "bfs": 1, "cc": 0}[algo]
+    while True:
+        y = x.copy()
+        np.minimum.at(y, v, np.where(x[u] < inf, x[u] + step, inf))
+        if np.array_equal(x, y):
+            return x
+        x = y
+
+
+@pytest.mark.parametrize("algo,delta", [("sssp", 5), ("bfs", 1), ("cc", 1)])
+@pytest.mark.parametrize("width", [LINE - 1, LINE, LINE + 1, LINE * 5 // 2 + 3])
+def test_waves_at_the_line(width, algo, delta):
+    n, off, dst, w = fan(width)
+    stored = algo == "sssp"
+    e = dg.Engine(algo, weight_mode="stored" if stored else "hash128", ordered_delta=delta)
+    e.load_csr(n, off, dst, w if stored else None)
+    e.start()
+    u, v = np.repeat(np.arange(n), np.diff(off.astype(np.int64))), dst.astype(np.int64)
+    assert np.array_equal(e.gather()[0], solve(algo, n, u, v, w))
+    k = int(off[1]) - 7
+    d = np.stack([u[:k], v[:k], w[:k]], 1).astype(np.uint32)
+    w2 = w.copy()
+    w2[:k] = w[:k] % 64 + 1
+    a = np.stack([u[:k], v[:k], w2[:k]], 1).astype(np.uint32)
+    e.apply_batch(d, [])
+    assert np.array_equal(e.gather()[0], solve(algo, n, u[k:], v[k:], w[k:]))
+    e.apply_batch([], a)
+    assert np.array_equal(e.gather()[0], solve(algo, n, u, v, w2))
+
+
+def test_carried_items_cost_a_wave_little():
+    # labels of the grid of 4096^2 vertices one value at a time: a wave expands a few
+    # of some ten million queued vertices and carries the rest (asked four at a time, 3 ms)
+    side = 4096
+    e = dg.Engine("cc", ordered_delta=1)
+    e.load_grid(side, 10, 8, 5, 1, 1000)
+    e.start()
+    rng = np.random.default_rng(1)
+    best = float("inf")
+    for seed in range(3):
+        d = e.sample_edges(5000, seed + 1)
+        u = rng.integers(0, side * side, 5000)
+        a = np.stack([u, (u + 1) % (side * side), np.ones(5000)], 1).astype(np.uint32)
+        st = e.apply_batch(d, a)
+        assert st["waves"] > 50 and st["affected"] > 1_000_000
+        best = min(best, st["ms_phase_closure"] / st["waves"])
+    assert best < 1.5, best
