@@ -684,6 +684,8 @@ void Engine::ensure_batch(size_t cnt) {
   suffix_cap_ = (uint32_t)std::min<u64>(slots / SUFFIX_CHUNK + dirs * c + 16, 0x7FFFFFFFull);
   suffix_ = (uint4 *)al((u64)suffix_cap_ * sizeof(uint4));
   suffix_ids_ = (uint32_t *)al((u64)std::min(suffix_cap_, SUFFIX_KEEP) * SUFFIX_CHUNK * 4);
+  over_window_ = (uint32_t)std::min<size_t>(dirs * c, OVER_WINDOW);
+  over_hist_ = (uint32_t *)al((size_t)over_window_ * OVER_SEGS * 4);
   for (size_t d = 0; d < dirs; d++) {
     rem_[d] = (uint32_t *)al(c * 4);
     matches_[d] = (uint32_t *)al(c * 4);
@@ -797,6 +799,8 @@ void Engine::enqueue_snapshot(size_t nd, size_t na, bool capture) {
     M.suffix = suffix_;
     M.suffix_cap = suffix_cap_;
     M.suffix_ids = suffix_ids_;
+    M.over_hist = over_hist_;
+    M.over_window = over_window_;
     M.reloc = reloc_;
     M.scarce[0] = out_.scarce;
     M.scarce[1] = in_.scarce;

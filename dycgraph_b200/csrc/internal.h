@@ -161,6 +161,9 @@ cudaError_t launch_ingest(const IngestLaunch &L, uint32_t *launches, cudaStream_
 // R-MAT 21 snapshot's mutation, this rule 1.14.
 constexpr uint32_t DEFER_SUFFIX = 1024, DEFER_SHORT = 64, DEFER_RECORDS = 3;
 constexpr uint32_t SUFFIX_CHUNK = 256, SUFFIX_KEEP = 16384;  // 16 MB of ids
+// Records that want fewer occurrences than match in a suffix: segments of the suffix
+// that their matches are counted by, and records counted at a time (8 MB of counts).
+constexpr uint32_t OVER_SEGS = 32, OVER_WINDOW = 65536;
 // Bookkeeping of rows whose block is full: new_off == old_off, compacted in place.
 constexpr uint32_t RELOC_CHUNK = 1024;
 struct RelocRec {
@@ -185,6 +188,8 @@ struct MutParams {
   uint4 *suffix;             // chunks: first record, end record, chunk, direction | chunks << 1
   uint32_t suffix_cap;
   uint32_t *suffix_ids;      // the first SUFFIX_KEEP chunks' slots, between the passes
+  uint32_t *over_hist;       // matches per segment of over_window records at a time
+  uint32_t over_window;
   Reloc reloc;
   u64 scarce[2];             // arena top from which full rows stay in their blocks if they can
   Ctl *ctl, *mctl;           // snapshot counters; this launch's barrier and queues
