@@ -683,7 +683,9 @@ void Engine::ensure_batch(size_t cnt) {
   // whole chunks of the deferred suffixes, and one part chunk per row
   suffix_cap_ = (uint32_t)std::min<u64>(slots / SUFFIX_CHUNK + dirs * c + 16, 0x7FFFFFFFull);
   suffix_ = (uint4 *)al((u64)suffix_cap_ * sizeof(uint4));
-  suffix_ids_ = (uint32_t *)al((u64)std::min(suffix_cap_, SUFFIX_KEEP) * SUFFIX_CHUNK * 4);
+  suffix_keep_ = (uint32_t)std::min<u64>(
+      suffix_cap_, std::min<u64>(std::max<u64>(slots / 1024, SUFFIX_KEEP_LEAST), SUFFIX_KEEP_MOST));
+  suffix_ids_ = (uint32_t *)al((u64)suffix_keep_ * SUFFIX_CHUNK * 4);
   over_window_ = (uint32_t)std::min<size_t>(dirs * c, OVER_WINDOW);
   over_hist_ = (uint32_t *)al((size_t)over_window_ * OVER_SEGS * 4);
   for (size_t d = 0; d < dirs; d++) {
@@ -799,6 +801,7 @@ void Engine::enqueue_snapshot(size_t nd, size_t na, bool capture) {
     M.suffix = suffix_;
     M.suffix_cap = suffix_cap_;
     M.suffix_ids = suffix_ids_;
+    M.suffix_keep = suffix_keep_;
     M.over_hist = over_hist_;
     M.over_window = over_window_;
     M.reloc = reloc_;

@@ -222,7 +222,7 @@ class Engine {
   uint32_t *found_ = nullptr, *touched_ = nullptr, *counts_ = nullptr;
   Reloc reloc_{};
   uint4 *suffix_ = nullptr;  // long-suffix deletions (mutate.cu)
-  uint32_t suffix_cap_ = 0, *suffix_ids_ = nullptr;
+  uint32_t suffix_cap_ = 0, suffix_keep_ = 0, *suffix_ids_ = nullptr;
   uint32_t over_window_ = 0, *over_hist_ = nullptr;
   uint32_t *rem_[2] = {}, *matches_[2] = {};
   BatchHdr *d_hdr_ = nullptr, *h_hdr_ = nullptr;  // header, records behind it

@@ -160,7 +160,12 @@ cudaError_t launch_ingest(const IngestLaunch &L, uint32_t *launches, cudaStream_
 // Scanning rows up to 1024 slots per record instead took 1.90 ms of a 100K-update
 // R-MAT 21 snapshot's mutation, this rule 1.14.
 constexpr uint32_t DEFER_SUFFIX = 1024, DEFER_SHORT = 64, DEFER_RECORDS = 3;
-constexpr uint32_t SUFFIX_CHUNK = 256, SUFFIX_KEEP = 16384;  // 16 MB of ids
+constexpr uint32_t SUFFIX_CHUNK = 256;
+// Chunks whose slots' records stay in HBM between the passes: one per 1024 arena
+// slots, within these (16 to 64 MB). A 1M-update Zipf snapshot on R-MAT 27 has some
+// 45,000 without a cache: its suffixes take 8.0 ms with 16,384 of them kept, 2.9 with
+// all.
+constexpr uint32_t SUFFIX_KEEP_LEAST = 16384, SUFFIX_KEEP_MOST = 65536;
 // Records that want fewer occurrences than match in a suffix: segments of the suffix
 // that their matches are counted by, and records counted at a time (8 MB of counts).
 constexpr uint32_t OVER_SEGS = 32, OVER_WINDOW = 65536;
@@ -187,7 +192,8 @@ struct MutParams {
   uint32_t *rem[2], *matches[2];  // long suffixes: wanted and matching occurrences
   uint4 *suffix;             // chunks: first record, end record, chunk, direction | chunks << 1
   uint32_t suffix_cap;
-  uint32_t *suffix_ids;      // the first SUFFIX_KEEP chunks' slots, between the passes
+  uint32_t *suffix_ids;      // the first suffix_keep chunks' slots, between the passes
+  uint32_t suffix_keep;
   uint32_t *over_hist;       // matches per segment of over_window records at a time
   uint32_t over_window;
   Reloc reloc;

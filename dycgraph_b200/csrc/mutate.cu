@@ -243,7 +243,7 @@ __device__ void delete_records(const MutParams &M, uint32_t dir, uint32_t p0, ui
 //   COUNT  every live slot is looked up among the row's records (sorted by
 //          neighbour): a lane's eight slots are read together and bisected
 //          together. Each record's matches are counted, and the slots' records
-//          stay in HBM (chunks past SUFFIX_KEEP are read from the host again).
+//          stay in HBM (chunks past suffix_keep are read from the host again).
 //   MARK   the matches of the records that want all of theirs are deleted.
 // A record that wants fewer than there are (two hubs joined by many occurrences) gets
 // the earliest ones. Its suffix is cut into OVER_SEGS segments:
@@ -291,7 +291,7 @@ __device__ void suffix_chunk(const MutParams &M, uint32_t c, uint32_t window, Co
   const uint32_t b = srt + ch.z * SUFFIX_CHUNK, e = min(len, b + SUFFIX_CHUNK);
   uint32_t *keep = M.suffix_ids + (u64)c * SUFFIX_CHUNK;
   uint32_t lo[U];  // the slots' records, INF32: none that wants any
-  if (PASS != COUNT && c < SUFFIX_KEEP) {
+  if (PASS != COUNT && c < M.suffix_keep) {
 #pragma unroll
     for (int u = 0; u < U; u++) lo[u] = keep[u * 32 + lane];
   } else {
@@ -329,7 +329,7 @@ __device__ void suffix_chunk(const MutParams &M, uint32_t c, uint32_t window, Co
     for (int u = 0; u < U; u++)
       if (d[u] == INF32 || lo[u] >= ch.y || list[lo[u]].y != d[u] || !M.rem[dir][lo[u]])
         lo[u] = INF32;
-    if (PASS == COUNT && c < SUFFIX_KEEP) {
+    if (PASS == COUNT && c < M.suffix_keep) {
 #pragma unroll
       for (int u = 0; u < U; u++) keep[u * 32 + lane] = lo[u];
     }
@@ -412,7 +412,7 @@ __device__ void over_cut(const MutParams &M, uint32_t id, uint32_t window, Count
 #pragma unroll
     for (int u = 0; u < U; u++) {
       const uint32_t s = b + u * 32 + lane;
-      if (c < SUFFIX_KEEP) {
+      if (c < M.suffix_keep) {
         hit[u] = M.suffix_ids[(u64)c * SUFFIX_CHUNK + u * 32 + lane] == o.x;
       } else {
         hit[u] = s < len && read_dst_rw(A, off + s) == rec.y && !slot_deleted_rw(A, off + s);
