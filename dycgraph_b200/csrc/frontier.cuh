@@ -17,6 +17,7 @@ namespace dycg {
 constexpr uint32_t SYNC_RESET_TILES = 1;
 constexpr uint32_t SYNC_RESET_Q0 = 2;
 constexpr uint32_t SYNC_RESET_Q1 = 4;
+constexpr uint32_t SYNC_RESET_Q2 = 8;
 constexpr uint32_t SYNC_RESET_VMIN = 16;
 constexpr uint32_t SYNC_RESET_GRAB = 32;
 constexpr uint32_t SYNC_RESET_ASYNC = 64;
@@ -25,7 +26,7 @@ constexpr uint32_t SYNC_RESET_RANGES = 128;  // with Q0 / Q1: that queue's range
 // What a barrier publishes to every block: one of the queue counters (SEL_*),
 // the tile count and the ordered closure's minimum, as they stood when the last
 // block arrived.
-constexpr uint32_t SEL_Q0 = 0, SEL_Q1 = 1, SEL_AFF = 3;
+constexpr uint32_t SEL_Q0 = 0, SEL_Q1 = 1, SEL_Q2 = 2, SEL_AFF = 3;
 struct Snap {
   bool ok;         // false: the launch has failed, leave
   uint32_t cnt, tiles, vmin;
@@ -74,7 +75,7 @@ __device__ __forceinline__ Snap grid_sync(Ctl *c, uint32_t &gen, uint32_t flags,
       const uint4 q = __ldcg(reinterpret_cast<const uint4 *>(c->q_count));
       const uint4 t = __ldcg(reinterpret_cast<const uint4 *>(&c->tile_count));
       p.x = gen | (t.z ? FAILED : 0u);
-      p.y = sel == SEL_Q0 ? q.x : sel == SEL_Q1 ? q.y : q.w;
+      p.y = sel == SEL_Q0 ? q.x : sel == SEL_Q1 ? q.y : sel == SEL_Q2 ? q.z : q.w;
       p.z = t.x;
       p.w = ~t.y;
       // (counters that a flag resets are published as they were; a queue that
@@ -82,6 +83,7 @@ __device__ __forceinline__ Snap grid_sync(Ctl *c, uint32_t &gen, uint32_t flags,
       if (flags & SYNC_RESET_TILES) c->tile_count = 0;
       if (flags & SYNC_RESET_Q0) c->q_count[0] = 0;
       if (flags & SYNC_RESET_Q1) c->q_count[1] = 0;
+      if (flags & SYNC_RESET_Q2) c->q_count[2] = 0;
       if (flags & SYNC_RESET_RANGES) {
         const uint32_t par = (flags & SYNC_RESET_Q1) ? 1 : 0;
         for (int b = 0; b < 64; b++) c->qrange[par][b] = 0;
@@ -271,11 +273,7 @@ constexpr uint32_t GROUP_ROW = 64;
 // Static: warp k of every block before warp k + 1 of any, so that a short wave
 // spreads over all SMs; one item per warp while the wave fits (its latency is
 // one row's), up to four per warp above (short rows leave most of 32 lanes
-// idle). Where admit can say no (Op::SIFTS) and there are 32 items per warp, a lane
-// asks for each: most of a long ordered queue is only carried to the next wave. CC
-// on the 4096^2 grid, some ten million items in ~800 waves: asked four at a time 3.0
-// ms a wave (2,422-3,219 ms of repair a snapshot), 32 at a time 0.50 (539), from
-// 128 items per warp on 0.67. Its SSSP, whose waves are short: 338 ms either way.
+// idle).
 template <bool WITH_W, class Op>
 __device__ Snap expand_rows(const Adj &A, const uint32_t *items, uint32_t cnt, Op &op, Acc &acc,
                             Tiles T, Ctl *ctl, uint32_t &gen, uint32_t sel, uint32_t reset_flags,
@@ -285,8 +283,23 @@ __device__ Snap expand_rows(const Adj &A, const uint32_t *items, uint32_t cnt, O
   const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
   const uint32_t per = claimed || cnt <= nw ? 1u : cnt <= 2 * nw ? 2u : 4u;
   const uint32_t grp = lane >> 3;
-  // the rows of up to four items, one per 8-lane group
-  const auto expand = [&](uint32_t v, uint32_t len, u64 off, bool on) {
+  uint32_t i = gw * per;
+  if (claimed) {
+    if (lane == 0) i = atomicAdd(&ctl->grab, 1u);
+    i = __shfl_sync(0xffffffffu, i, 0);
+  }
+  while (i < cnt) {
+    const bool have = grp < per && i + grp < cnt;
+    const uint32_t v = have ? __ldcg(items + i + grp) : 0u;
+    if (claimed) {
+      if (lane == 0) i = atomicAdd(&ctl->grab, 1u);
+      i = __shfl_sync(0xffffffffu, i, 0);
+    } else {
+      i += nw * per;
+    }
+    const uint32_t len = have ? A.len[v] : 0u;
+    const u64 off = have ? A.off[v] : 0ull;
+    const bool on = op.admit(v, have);
     const bool small = per > 1 && len <= GROUP_ROW;
     if (__any_sync(0xffffffffu, on && small))
       group_slots<8, WITH_W>(A, v, on && small, off, 0, len, 8, op, acc);
@@ -313,44 +326,6 @@ __device__ Snap expand_rows(const Adj &A, const uint32_t *items, uint32_t cnt, O
       }
       group_slots<32, WITH_W>(A, bv, true, bo, 0, bl, 32, op, acc);
     }
-  };
-  uint32_t i = gw * per;
-  if (claimed) {
-    if (lane == 0) i = atomicAdd(&ctl->grab, 1u);
-    i = __shfl_sync(0xffffffffu, i, 0);
-  }
-  if constexpr (Op::SIFTS) {
-    if (!claimed && cnt / 32 >= nw) {
-      // eight of the rounds below at once: lane l has item l % 4 of round l / 4
-      for (; i < cnt; i += nw * 32) {
-        const uint32_t at = i + (lane >> 2) * (nw * 4) + (lane & 3);
-        const uint32_t iv = at < cnt ? __ldcg(items + at) : 0u;
-        unsigned left = __ballot_sync(0xffffffffu, op.template admit<1>(iv, at < cnt));
-        while (left) {
-          int src = -1;
-#pragma unroll
-          for (uint32_t g = 0; g < 4; g++) {
-            if (g == grp) src = __ffs(left) - 1;
-            left &= left - 1;
-          }
-          const uint32_t v = __shfl_sync(0xffffffffu, iv, src & 31);
-          expand(v, src >= 0 ? A.len[v] : 0u, src >= 0 ? A.off[v] : 0ull, src >= 0);
-        }
-      }
-    }
-  }
-  while (i < cnt) {
-    const bool have = grp < per && i + grp < cnt;
-    const uint32_t v = have ? __ldcg(items + i + grp) : 0u;
-    if (claimed) {
-      if (lane == 0) i = atomicAdd(&ctl->grab, 1u);
-      i = __shfl_sync(0xffffffffu, i, 0);
-    } else {
-      i += nw * per;
-    }
-    const uint32_t len = have ? A.len[v] : 0u;
-    const u64 off = have ? A.off[v] : 0ull;
-    expand(v, len, off, op.template admit<8>(v, have));
   }
   // The items have been consumed: the queue resets can apply here. When no row
   // was heavy this barrier's snapshot already holds every append of the

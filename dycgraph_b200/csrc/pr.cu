@@ -112,8 +112,6 @@ struct AmendOp {
   struct Row {
     float c;
   };
-  static constexpr bool SIFTS = false;
-  template <int G>
   __device__ bool admit(uint32_t, bool on) { return on; }
   template <int G>
   __device__ bool begin(uint32_t u, bool on, Row &row) {
@@ -144,8 +142,6 @@ struct ScatterOp {
   struct Row {
     float c;
   };
-  static constexpr bool SIFTS = false;
-  template <int G>
   __device__ bool admit(uint32_t, bool on) { return on; }
   template <int G>
   __device__ bool begin(uint32_t v, bool on, Row &row) {

@@ -68,8 +68,6 @@ template <uint32_t ALGO>
 struct InvalidateOp {
   const RepairParams *P;
   struct Row {};
-  static constexpr bool SIFTS = false;
-  template <int G>
   __device__ bool admit(uint32_t, bool on) { return on; }
   template <int G>
   __device__ bool begin(uint32_t, bool on, Row &) { return on; }
@@ -114,8 +112,6 @@ struct PullOp {
   struct Row {
     u64 best;
   };
-  static constexpr bool SIFTS = false;
-  template <int G>
   __device__ bool admit(uint32_t, bool on) { return on; }
   template <int G>
   __device__ bool begin(uint32_t, bool on, Row &r) {
@@ -176,11 +172,10 @@ struct RelaxOp {
   struct Row {
     uint32_t dv, imp;  // the vertex's value; the lowest value this lane pushed
   };
-  static constexpr bool SIFTS = ORDERED;
+  __device__ bool admit(uint32_t v, bool on) { return ORDERED ? below<8>(v, on) : on; }
   // groups of G lanes hold the same item
   template <int G>
-  __device__ bool admit(uint32_t v, bool on) {
-    if (!ORDERED) return on;
+  __device__ bool below(uint32_t v, bool on) {
     const bool lead = (lane_id() & (G - 1)) == 0;
     const uint32_t d = on ? key_value(ld_key(P->key + v)) : INF32;
     // one read decides for the whole group
@@ -244,7 +239,7 @@ struct RelaxOp {
 // ms, R-MAT 21 SSSP 100K 0.73 -> 0.36 ms, 1024^2 grid SSSP 1K (1,580 ordered
 // waves) 39.4 -> 20.2 ms. 1024 threads leave 64 registers each: CC and
 // stored-weight SSSP spill 172 and 164 bytes a thread, BFS and rule-weight SSSP 48
-// and 44 (ordered: 284 and 300, 136).
+// and 44 (ordered: 188 and 196, 80).
 template <uint32_t ALGO, bool STORED, bool ORDERED>
 __global__ void __launch_bounds__(REPAIR_BLOCK, 1)
     repair_kernel(const __grid_constant__ RepairParams P) {
@@ -343,7 +338,11 @@ __global__ void __launch_bounds__(REPAIR_BLOCK, 1)
   // barrier per wave: the expanding warps themselves carry what is above the
   // threshold, an item per warp (or group), so that the wave's rows spread over
   // all warps whatever their place in the queue, and the next wave's minimum is
-  // kept on the fly and published by the closing barrier.
+  // kept on the fly and published by the closing barrier. From an item per thread on
+  // the carrying is a pass and a barrier of its own: CC on the 4096^2 grid, some ten
+  // million items in ~800 waves, took 3.0 ms a wave when asked four at a time per warp
+  // (2,422-3,219 ms of repair a snapshot), and takes 0.5 so (the label order, and with
+  // it the number of waves, varies from run to run). SSSP there: 338 ms, 331 so.
   if (P.phases & PH_CLOSE) {
     for (uint32_t wave = 0; sn.cnt; wave++) {
       if (wave >= P.max_waves) {
@@ -353,9 +352,26 @@ __global__ void __launch_bounds__(REPAIR_BLOCK, 1)
       const uint32_t thr = sn.vmin > INF32 - P.delta ? INF32 : sn.vmin + P.delta;
       RelaxOp<ALGO, STORED, ORDERED> op{&P, P.q[cur ^ 1], &ctl->q_count[cur ^ 1],
                                         tag_base + 1 + wave, thr};
-      sn = expand_rows<STORED>(P.out, P.q[cur], sn.cnt, op, acc, P.tiles, ctl, gen,
+      const uint32_t *items = P.q[cur];
+      uint32_t cnt = sn.cnt;
+      if (ORDERED && cnt >= gstride) {
+        // a long queue, of which most is only carried: a lane asks for each item, and
+        // what is left (in the affected list, which the pull has read) is expanded
+        for (uint32_t i0 = first; i0 < cnt; i0 += gstride) {
+          const uint32_t i = i0 + lane;
+          const uint32_t v[1] = {i < cnt ? __ldcg(items + i) : 0u};
+          const bool want[1] = {op.template below<1>(v[0], i < cnt)};
+          append_batch(P.aff, &ctl->q_count[2], P.n, want, v, &ctl->err);
+        }
+        sn = grid_sync(ctl, gen, 0, SEL_Q2, P.timeout_ns);
+        if (!sn.ok) goto done;
+        items = P.aff;
+        cnt = sn.cnt;
+      }
+      sn = expand_rows<STORED>(P.out, items, cnt, op, acc, P.tiles, ctl, gen,
                                cur ? SEL_Q0 : SEL_Q1,
-                               (cur ? SYNC_RESET_Q1 : SYNC_RESET_Q0) | SYNC_RESET_VMIN,
+                               (cur ? SYNC_RESET_Q1 : SYNC_RESET_Q0) | SYNC_RESET_VMIN |
+                                   (ORDERED ? SYNC_RESET_Q2 : 0u),
                                P.timeout_ns, P.claimed);
       if (!sn.ok) goto done;
       if (gtid == 0) ctl->waves = wave + 1;
