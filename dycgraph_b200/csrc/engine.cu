@@ -21,7 +21,6 @@
 #include <unistd.h>
 
 #include "engine.h"
-#include "mutation_grid.h"
 #include "ring.h"
 
 namespace dycg {
@@ -247,8 +246,6 @@ void Engine::build_from_sorted_keys(u64 *keys, uint32_t *wv, u64 m, bool weight_
 void Engine::finish_load() {
   const uint32_t n = n_;
   npages_ = out_.pages + (has_in_ ? in_.pages : 0);
-  mut_ctas_ = mutation_ctas(opt_.mutation_ctas, (uint32_t)num_sms_,
-                            (out_.slots + (has_in_ ? in_.slots : 0)) * 4 * out_.stride);
   page_slot_ = (uint32_t *)dmalloc((u64)npages_ * 4);
   page_hits_ = (uint32_t *)dmalloc((u64)npages_ * 4);
   CK(cudaMemsetAsync(page_slot_, 0xFF, (u64)npages_ * 4, st_));
@@ -810,7 +807,8 @@ void Engine::enqueue_snapshot(size_t nd, size_t na, bool capture) {
     M.ctl = ctl_;
     M.mctl = mctl_;
     M.timeout_ns = timeout;
-    CK(launch_mutate(M, (uint32_t)std::max(nd, na), mut_ctas_, st_));
+    CK(launch_mutate(M, (uint32_t)std::max(nd, na), opt_.mutation_ctas,
+                     (out_.slots + (has_in_ ? in_.slots : 0)) * 4 * out_.stride, st_));
     launches_++;
   }
   if (!capture) CK(cudaEventRecord(ev_[2], st_));

@@ -128,7 +128,6 @@ class Engine {
 
   dycg_options opt_;
   int dev_ = 0, num_sms_ = 148;
-  uint32_t mut_ctas_ = 148;  // most CTAs of the mutation kernel
   cudaStream_t st_ = nullptr;
   cudaEvent_t ev_[6] = {};
   // side stream of the hotness path's page staging (eviction, admission list,

@@ -201,9 +201,10 @@ struct MutParams {
   Ctl *ctl, *mctl;           // snapshot counters; this launch's barrier and queues
   u64 timeout_ns;
 };
-// records: the longer of the two kinds (or the class's capacity); ctas: most
-// CTAs to launch
-cudaError_t launch_mutate(const MutParams &M, uint32_t records, uint32_t ctas, cudaStream_t s);
+// records: the longer of the two kinds (or the class's capacity); ctas: the caller's
+// limit (0: none); arena_bytes: of both directions
+cudaError_t launch_mutate(const MutParams &M, uint32_t records, uint32_t ctas, u64 arena_bytes,
+                          cudaStream_t s);
 
 // cache
 // Device-resident admission state: the free-slot count and the plan of the

@@ -992,7 +992,8 @@ __global__ void __launch_bounds__(MUT_BLOCK, 1)
   }
 }
 
-cudaError_t launch_mutate(const MutParams &M, uint32_t records, uint32_t ctas, cudaStream_t s) {
+cudaError_t launch_mutate(const MutParams &M, uint32_t records, uint32_t ctas, u64 arena_bytes,
+                          cudaStream_t s) {
   if (!records) return cudaSuccess;
   int dev = 0, sms = 0, per_sm = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -1001,7 +1002,8 @@ cudaError_t launch_mutate(const MutParams &M, uint32_t records, uint32_t ctas, c
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mutate_kernel, MUT_BLOCK, 0);
   if (e != cudaSuccess) return e;
   const uint32_t grid =
-      mutation_grid(records, M.dirs, ctas, (u64)std::max(per_sm, 1) * (u64)sms);
+      mutation_grid(records, M.dirs, ctas, (uint32_t)sms, arena_bytes,
+                    (u64)std::max(per_sm, 1) * (u64)sms);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(MUT_BLOCK);

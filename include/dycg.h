@@ -105,8 +105,8 @@ typedef struct dycg_options {
                           /* dycg_tune_query_mapping)                          */
   uint32_t mutation_ctas; /* most CTAs of the mutation kernel, counted in CTAs */
                           /* of eight warps and rounded up to an even number  */
-                          /* (0: two per SM, on a quarter of the SMs for      */
-                          /* arenas above 4 GB).                              */
+                          /* (0: two per SM; for arenas above 4 GB as many as */
+                          /* the batch is dense in them, a quarter at least). */
                           /* They take a snapshot's records in row order, so  */
                           /* fewer CTAs in flight keep their host transactions*/
                           /* in a narrower window of the arena, which the host*/
