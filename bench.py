@@ -79,7 +79,8 @@ def parse():
                          "and 1 for BFS/CC)")
     ap.add_argument("--json-out", default=None)
     ap.add_argument("--mutation-ctas", type=int, default=0,
-                    help="CTAs of the deletion/append kernels (0: the library default)")
+                    help="most CTAs of the mutation kernel, in CTAs of eight warps (0: the "
+                         "library default)")
     ap.add_argument("--frontier-queue", default="static", choices=["static", "claimed"],
                     help="single-source repair: how warps share a wave's rows")
     ap.add_argument("--page-shift", type=int, default=12,
@@ -189,7 +190,7 @@ class Clocks:
 # capture); the line's `traffic` scales it by the run's own algorithmic bytes.
 # None where no capture was taken.
 # batched repair kernel, R-MAT 20 / 256 queries, the two timed launches of
-# profiles/ncu_multi_repair_rmat20_q256.md: 2,728 MB DRAM / 589.2 MB algorithmic
+# profiles/ncu_multi_repair_rmat20_q256.md: 2,593 MB DRAM / 561.8 MB algorithmic
 NCU_TRAFFIC_RATIO = {("batched", "sssp"): 4.6}
 
 # Random host-link transactions cost about the same whatever their size up to
